@@ -123,9 +123,8 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g);
  *                until stt_destroy; where the device's texture limits do not
  *                admit the array, the load-based variant of the same shape runs);
  *   slab_variant the box the slab-staged projector stages with TMA;
- *   bp_variant   the column length of the voxel backprojection (solver), and
- *                whether each column's voxels are first prefetched into L2
- *                (for volumes larger than L2);
+ *   bp_variant   the column length of the voxel backprojection (0: by the
+ *                geometry's magnification) and the blocks per SM;
  *   staged_bins  bit b set: views whose central ray is 5b to 5b+5 degrees off
  *                the nearest of the x and z axes (bit 8: 40 to 45) are
  *                projected by the slab-staged kernel, the others by the gather
@@ -212,12 +211,7 @@ stt_status stt_fp_vjp(stt_ctx *ctx, const float *proj_bar, float *vol_bar, int v
 /* ---- backprojectors ------------------------------------------------------
  * Voxel-driven (ST_Tomography.cpp:690-730): vol = clamp(vol + alpha *
  * bicubic(corr at the voxel's projection), 0, gmax); voxels projecting
- * outside [2, W-2) x [2, H-2) are left unchanged.  Deterministic.  From
- * 2^23 voxels on, corr is first copied (on `stream`) into a texture the
- * context owns, which the column walk of the tuned bp_variant gathers from
- * (stt_sart_sweep writes it from the projector directly, at every size);
- * calls of one context that overlap on different streams race on that copy.
- * The result is the same either way. */
+ * outside [2, W-2) x [2, H-2) are left unchanged.  Deterministic. */
 stt_status stt_bp_voxel(stt_ctx *ctx, const float *corr, float *vol, double alpha, float gmax,
                         int view, void *stream);
 /* stt_bp_voxel on a volume stored as `dtype` (STT_DTYPE_BF16: each voxel is

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_fp_corr_slab(const GeomDev g, co
                                                       const T *__restrict__ vol, const T *__restrict__ vol_t,
                                                       const ViewSel sel, const B *__restrict__ b_stack,
                                                       float *__restrict__ raylen_state, float *__restrict__ corr,
-                                                      unsigned long long corr_surf, int *status) {
+                                                      int *status) {
     __shared__ alignas(128) T buf[2 * BX::N];
     __shared__ uint64_t bar[2];
     __shared__ int red[2][2 * WARPS];
@@ -293,9 +293,7 @@ __global__ void __launch_bounds__(32 * WARPS) k_fp_corr_slab(const GeomDev g, co
     } else {
         L = raylen_state ? raylen_state[pix] : 0.0f;
     }
-    const float c = __fdiv_rn(__fsub_rn(ld_voxel(b + pix), acc.s), __fadd_rn(L, 1.0f));
-    corr[pix] = c;
-    if (corr_surf) surf2DLayeredwrite(c, corr_surf, i * (int)sizeof(float), j, 0, cudaBoundaryModeZero);
+    corr[pix] = __fdiv_rn(__fsub_rn(ld_voxel(b + pix), acc.s), __fadd_rn(L, 1.0f));
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -356,7 +354,7 @@ void box_dims(cuuint32_t box[3]) {
 template <class BX, bool PK, typename T, typename B>
 cudaError_t launch_slab(const GeomDev &g, const ViewRec *views, const FpSlabMaps &m, const T *vol,
                         const T *vol_t, const ViewSel &sel, const B *b_stack, float *raylen_state, float *corr,
-                        cudaStream_t s, unsigned long long corr_surf, int *status) {
+                        cudaStream_t s, int *status) {
     static const bool carve = [] {
         cudaFuncSetAttribute(k_fp_corr_slab<BX, PK, T, B>, cudaFuncAttributePreferredSharedMemoryCarveout,
                              cudaSharedmemCarveoutMaxShared);
@@ -365,7 +363,7 @@ cudaError_t launch_slab(const GeomDev &g, const ViewRec *views, const FpSlabMaps
     }();
     (void)carve;
     k_fp_corr_slab<BX, PK, T, B><<<dim3((g.W + 31) / 32, (g.H + WARPS - 1) / WARPS, 1), 32 * WARPS, 0, s>>>(
-        g, views, m.x, m.z, vol, vol_t, sel, b_stack, raylen_state, corr, corr_surf, status);
+        g, views, m.x, m.z, vol, vol_t, sel, b_stack, raylen_state, corr, status);
     return cudaGetLastError();
 }
 
@@ -410,12 +408,11 @@ bool make_fp_slab_maps(const GeomDev &g, const unsigned short *vol, const unsign
 
 cudaError_t launch_fp_corr_slab(const GeomDev &g, const ViewRec *views, const FpSlabMaps &m, const unsigned short *vol,
                                 const unsigned short *vol_t, const ViewSel &sel, const unsigned short *b_stack,
-                                float *raylen_state, float *corr, cudaStream_t s, unsigned long long corr_surf,
-                                int *status) {
+                                float *raylen_state, float *corr, cudaStream_t s, int *status) {
     if (!m.ok || m.esize != 2 || (vol_t && !m.has_z)) return cudaErrorInvalidValue;
     typedef unsigned short U;
 #define STT_SLAB16(BOX) \
-    launch_slab<BOX, false, U, U>(g, views, m, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, status)
+    launch_slab<BOX, false, U, U>(g, views, m, vol, vol_t, sel, b_stack, raylen_state, corr, s, status)
     switch (m.variant & 3) {
     case 1: return STT_SLAB16(Box1);
     case 2: return STT_SLAB16(Box2);
@@ -427,10 +424,10 @@ cudaError_t launch_fp_corr_slab(const GeomDev &g, const ViewRec *views, const Fp
 
 cudaError_t launch_fp_corr_slab(const GeomDev &g, const ViewRec *views, const FpSlabMaps &m, const float *vol,
                                 const float *vol_t, const ViewSel &sel, const float *b_stack, float *raylen_state,
-                                float *corr, cudaStream_t s, unsigned long long corr_surf, int *status) {
+                                float *corr, cudaStream_t s, int *status) {
     if (!m.ok || m.esize != 4 || (vol_t && !m.has_z)) return cudaErrorInvalidValue;
 #define STT_SLAB(B, P) launch_slab<B, P, float, float>(g, views, m, vol, vol_t, sel, b_stack, raylen_state, corr, s, \
-                                                      corr_surf, status)
+                                                      status)
     switch (m.variant) {
     case 1: return STT_SLAB(Box1, false);
     case 2: return STT_SLAB(Box2, false);

@@ -203,7 +203,7 @@ __device__ __forceinline__ bool run_job(const SweepJob &J, int rank, T (*tile)[3
             dynamic_tiles(J.bar + 2, tickets, cx * cy * g.nz, [&](int t) {
                 const int x = (t % cx) * SWEEP_THREADS + threadIdx.x, y0 = ((t / cx) % cy) * SWEEP_COL;
                 const int z = t / (cx * cy);
-                if (x < g.nx) bp_column<SWEEP_COL, false>(g, vr, rows, vol, x, y0, z, J.alpha, J.gmax);
+                if (x < g.nx) bp_column<SWEEP_COL>(g, vr, rows, vol, x, y0, z, J.alpha, J.gmax);
             });
             tickets += (unsigned)(cx * cy * g.nz + nb);
         }

@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(32 * NW) k_fp_corr(const GeomDev g, const View
                                                      const T *__restrict__ vol, const T *__restrict__ vol_t,
                                                      const ViewSel sel, const B *__restrict__ b_stack,
                                                      float *__restrict__ raylen_state,
-                                                     float *__restrict__ corr, unsigned long long corr_surf,
+                                                     float *__restrict__ corr,
                                                      int skip_staged, const FpTex tex) {
     int i, j;
     if (!tile_pixel_t<WX, NW>(g, i, j)) return;
@@ -134,10 +134,7 @@ __global__ void __launch_bounds__(32 * NW) k_fp_corr(const GeomDev g, const View
     } else {
         L = raylen_state ? raylen_state[pix] : 0.0f;
     }
-    const float c = __fdiv_rn(__fsub_rn(ld_voxel(b + pix), sum), __fadd_rn(L, 1.0f));
-    corr[pix] = c;
-    // the copy the voxel-driven backprojector gathers from with tld4
-    if (corr_surf) surf2DLayeredwrite(c, corr_surf, i * (int)sizeof(float), j, 0, cudaBoundaryModeZero);
+    corr[pix] = __fdiv_rn(__fsub_rn(ld_voxel(b + pix), sum), __fadd_rn(L, 1.0f));
 }
 
 // BP-mode march (SingleScalarVolume.core.h:128-143, UpdateContributionSum
@@ -451,11 +448,11 @@ namespace {
 template <int WX, int NW, int G, bool PK = false, bool TX = false>
 void fp_corr_variant(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t, const ViewSel &sel,
                      const float *b_stack, float *raylen_state, float *corr, cudaStream_t s,
-                     unsigned long long corr_surf, int skip, const FpTex &tex = FpTex{}) {
+                     int skip, const FpTex &tex = FpTex{}) {
     constexpr int TH = (32 / WX) * NW;  // detector rows per block
     k_fp_corr<int, WX, NW, G, PK, float, float, TX>
         <<<dim3((g.W + WX - 1) / WX, (g.H + TH - 1) / TH, 1), 32 * NW, 0, s>>>(
-            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, corr_surf, skip, tex);
+            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, skip, tex);
 }
 
 // Device limits of pitch-linear 2D textures, read once per device.
@@ -588,7 +585,7 @@ void destroy_fp_tex(FpTex &t) {
 
 cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t,
                            const ViewSel &sel, const float *b_stack, float *raylen_state, float *corr,
-                           cudaStream_t s, unsigned long long corr_surf, const FpSlabMaps *maps, int *status,
+                           cudaStream_t s, const FpSlabMaps *maps, int *status,
                            int fp_variant, const FpTex *tex) {
     const int skip = maps && maps->ok && maps->esize == 4 && (!vol_t || maps->has_z);
     // a texture variant whose textures are missing, or do not cover vol_t,
@@ -599,33 +596,33 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *
     if (!vol_t) tx.z = 0;  // without the copy every view reads the volume, as the loads do
     if (skip) {
         cudaError_t e = launch_fp_corr_slab(g, views, *maps, vol, vol_t, sel, b_stack, raylen_state, corr, s,
-                                            corr_surf, status);
+                                            status);
         if (e != cudaSuccess) return e;
     }
     if (!small_volume(g)) {
         k_fp_corr<long long><<<ray_grid(g, 1), 128, 0, s>>>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr,
-                                                            corr_surf, skip, FpTex{});
+                                                            skip, FpTex{});
         return cudaGetLastError();
     }
     switch (fp_variant) {
-    case 1: fp_corr_variant<32, 2, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 2: fp_corr_variant<32, 8, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 3: fp_corr_variant<16, 4, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 4: fp_corr_variant<8, 4, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 5: fp_corr_variant<32, 4, 2>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 6: fp_corr_variant<32, 4, 8>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 7: fp_corr_variant<32, 4, 4, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 8: fp_corr_variant<32, 4, 8, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
-    case 9: fp_corr_variant<32, 8, 4, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
+    case 1: fp_corr_variant<32, 2, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 2: fp_corr_variant<32, 8, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 3: fp_corr_variant<16, 4, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 4: fp_corr_variant<8, 4, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 5: fp_corr_variant<32, 4, 2>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 6: fp_corr_variant<32, 4, 8>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 7: fp_corr_variant<32, 4, 4, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 8: fp_corr_variant<32, 4, 8, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
+    case 9: fp_corr_variant<32, 8, 4, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
     case 10:
-        fp_corr_variant<8, 4, 8, true, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf,
+        fp_corr_variant<8, 4, 8, true, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s,
                                              skip, tx);
         break;
     case 11:
-        fp_corr_variant<32, 4, 8, true, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf,
+        fp_corr_variant<32, 4, 8, true, true>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s,
                                               skip, tx);
         break;
-    default: fp_corr_variant<32, 4, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, corr_surf, skip); break;
+    default: fp_corr_variant<32, 4, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
     }
     return cudaGetLastError();
 }
@@ -678,13 +675,13 @@ cudaError_t launch_correction(long long n, const unsigned short *b, const float 
 
 cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigned short *vol,
                            const unsigned short *vol_t, const ViewSel &sel, const unsigned short *b_stack,
-                           float *raylen_state, float *corr, cudaStream_t s, unsigned long long corr_surf,
+                           float *raylen_state, float *corr, cudaStream_t s,
                            const FpSlabMaps *maps, int *status, int fp_variant16, const FpTex *tex) {
     typedef unsigned short U;
     const int skip = maps && maps->ok && maps->esize == 2 && (!vol_t || maps->has_z);
     if (skip) {
         cudaError_t e = launch_fp_corr_slab(g, views, *maps, vol, vol_t, sel, b_stack, raylen_state, corr, s,
-                                            corr_surf, status);
+                                            status);
         if (e != cudaSuccess) return e;
     }
     if (fp_variant16 == 1 && tex && tex->ok && tex->esize == 2 && (!vol_t || tex->z) && small_volume(g)) {
@@ -692,15 +689,15 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigne
         if (!vol_t) tx.z = 0;
         constexpr int WX = 8, NW = 4, TH = (32 / WX) * NW;
         k_fp_corr<int, WX, NW, 8, true, U, U, true><<<dim3((g.W + WX - 1) / WX, (g.H + TH - 1) / TH, 1), 32 * NW, 0, s>>>(
-            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, corr_surf, skip, tx);
+            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, skip, tx);
         return cudaGetLastError();
     }
     if (small_volume(g))
         k_fp_corr<int, 32, 4, FP_GROUP, false, U, U><<<ray_grid(g, 1), 128, 0, s>>>(
-            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, corr_surf, skip, FpTex{});
+            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, skip, FpTex{});
     else
         k_fp_corr<long long, 32, 4, FP_GROUP, false, U, U><<<ray_grid(g, 1), 128, 0, s>>>(
-            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, corr_surf, skip, FpTex{});
+            g, views, vol, vol_t, sel, b_stack, raylen_state, corr, skip, FpTex{});
     return cudaGetLastError();
 }
 

@@ -13,47 +13,130 @@ namespace stt {
 
 namespace {
 
-template <bool TEX, typename T>
-__global__ void __launch_bounds__(128) k_bp_voxel(const GeomDev g, const ViewRec *__restrict__ views,
-                                                  const ViewSel sel, const float *__restrict__ corr,
-                                                  T *__restrict__ vol, float alpha, float gmax,
-                                                  unsigned long long corr_tex) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= g.nx) return;
-    int local;
-    const ViewRec &v = views[sel_view(sel, local)];
-    if (TEX)
-        bp_voxel_at(g, v, BpRowsTex{corr_tex}, vol, x, blockIdx.y, blockIdx.z, alpha, gmax);
-    else
-        bp_voxel_at(g, v, BpRowsLdg{corr, g.W}, vol, x, blockIdx.y, blockIdx.z, alpha, gmax);
+// Voxel-based backprojection, columns of K voxels up y; a block has 32 (x) by
+// 4 (z) of them.  The detector column, the depth and the x weights are the
+// column's; the detector rows its voxels' windows cover are one run of about
+// K sdd/sid + 4.  Phase 1 forms the x-weighted sum of every row of every
+// column's run into a table in shared memory (4 loads each, none waiting for
+// another); phase 2 combines 4 row sums per voxel, four voxels' loads at a
+// time and one group ahead.  A warp is 8 x 4 columns in phase 1, whose rows and
+// taps lie close together on the detector whatever the view, and 32 x 1 in
+// phase 2, whose voxels are consecutive.
+// A column whose rows do not fit in the table (a magnification above
+// (BP_ROWS - 5) / (K - 1) rows per voxel) takes the walk (bp_column).
+//
+// Bound by L1 (tags and data of the row loads: 80 % of its peak) and issue
+// (62 %).  The form before walked the voxels up y and fetched each one's two new
+// rows with two tld4 of a texture copy of the correction, which ran at the
+// texture unit's rate.  Per view, mean of 12 views (that form -> this one, us):
+// 192^3 / 256^2 52.1 -> 28.1, 256^3 / 512^2 92.0 -> 68.6, 512^3 / 1024^2
+// 718 (626 with an L2 prefetch) -> 480.  Measured and not kept: warps of 32 x 1
+// columns in both phases (90-degree views 80 us at 256^3: their lanes' rows
+// differ), of 16 x 2 (69) and 8 x 4 (78, the volume in 32-byte pieces); 48
+// registers and 10 blocks (72); all K voxels loaded first (128 registers: 100).
+constexpr int BP_ROWS = 40, BP_G = 4;
+constexpr int BP_PITCH = 40;  // table columns of one z: 8 banks on from the last, so neither phase's warps conflict
+
+// One column of a rotation about y: whether any voxel of [y0, y1) may be
+// updated, and the run of rows (u does not fall with y: A[4] > 0).
+struct BpCol {
+    float ndepth, scale, ulo, uhi;
+    int r0, nr;
+    bool live;
+};
+__device__ __forceinline__ BpCol bp_col(const GeomDev &g, const ViewRec &v, float fx, float fz, int y0, int y1) {
+    BpCol c;
+    c.ndepth = -bp_cam(v, 2, fx, (float)y0, fz);
+    c.scale = bp_scale(g, c.ndepth);
+    c.ulo = bp_coord(g.cy, bp_cam(v, 1, fx, (float)y0, fz), c.scale);
+    c.uhi = bp_coord(g.cy, bp_cam(v, 1, fx, (float)(y1 - 1), fz), c.scale);
+    c.r0 = bp_tap(c.ulo, g.H) - 1;
+    c.nr = bp_tap(c.uhi, g.H) + 3 - c.r0;
+    const float camx = bp_cam(v, 0, fx, (float)y0, fz);
+    c.live = c.uhi >= 2.0f - BP_NEAR && c.ulo < (float)(g.H - 2) + BP_NEAR &&
+             bp_inside(g, bp_coord(g.cx, camx, c.scale), g.cx, camx, c.ndepth, g.W);
+    return c;
 }
 
-// Column form, texture taps (bp_column in stt_voxel.cuh): one thread per
-// (x, z) walks K voxels up y.  Column length K: 16 by default; the autotuner
-// may pick 8 or 32 (the voxels' values do not depend on which thread walks
-// them).
-constexpr int BP_COL = 16;
-
-// Ten 128-thread blocks per SM (48 registers, no spills): the walk is bound
-// by texture latency, so the extra warps pay (10 blocks: 104.1 ms per
-// iteration of the 10 x 256^3 solve against 106.6 ms with the compiler's
-// 52 registers and 9 blocks).
-//
-// PF: before the walk, every thread asks L2 for its column's K voxels
-// (prefetch.global.L2: no register, no scoreboard).  Where the volume does not
-// fit in L2 (512^3 FP32 is 512 MiB against 126 MB), the walk's one load per
-// voxel otherwise waits for HBM with a single load in flight per thread, and
-// ten blocks of them keep too few bytes in flight to cover HBM latency.  The
-// values read, and so the bits written, are the same.
-template <int K = BP_COL, typename T = float, bool PF = false>
-__global__ void __launch_bounds__(128, 10) k_bp_voxel_cols(const GeomDev g, const ViewRec *__restrict__ views,
-                                                       const ViewSel sel, T *__restrict__ vol, float alpha,
-                                                       float gmax, unsigned long long tex) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= g.nx) return;
+template <int K, int OCC, typename T>
+__global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, const ViewRec *__restrict__ views,
+                                                            const ViewSel sel, const float *__restrict__ corr,
+                                                            T *__restrict__ vol, float alpha, float gmax) {
+    __shared__ float table[BP_ROWS * 4 * BP_PITCH];
+    constexpr int RS = 4 * BP_PITCH;  // one row of every column
     int local;
     const ViewRec &v = views[sel_view(sel, local)];
-    bp_column<K, PF>(g, v, BpRowsTex{tex}, vol, x, blockIdx.y * K, blockIdx.z, alpha, gmax);
+    const int y0 = blockIdx.y * K, y1 = min(y0 + K, g.ny);
+    const bool rot_y = v.A[1] == 0.0f && v.A[7] == 0.0f;
+    if (rot_y) {
+        const int xl = (threadIdx.x >> 5) * 8 + (threadIdx.x & 7), zl = (threadIdx.x >> 3) & 3;
+        const int x = blockIdx.x * 32 + xl, z = blockIdx.z * 4 + zl;
+        const float fx = (float)x, fz = (float)z;
+        const BpCol c = bp_col(g, v, fx, fz, y0, y1);
+        if (x < g.nx && z < g.nz && c.live && c.nr <= BP_ROWS) {
+            const float upx = bp_coord(g.cx, bp_cam(v, 0, fx, (float)y0, fz), c.scale);
+            const int px = bp_tap(upx, g.W);
+            float wx[4];
+            bp_weights(upx - (float)px, wx);
+            float *row = table + zl * BP_PITCH + xl;
+            unsigned o = (unsigned)(c.r0 * g.W + px - 1);  // (W H < 2^31)
+#pragma unroll 4
+            for (int i = 0; i < c.nr; ++i, o += g.W) {
+                const float t[4] = {__ldg(corr + o), __ldg(corr + o + 1), __ldg(corr + o + 2), __ldg(corr + o + 3)};
+                row[RS * i] = bp_row(t, wx);
+            }
+        }
+    }
+    __syncthreads();
+    const int xl = threadIdx.x & 31, zl = threadIdx.x >> 5;
+    const int x = blockIdx.x * 32 + xl, z = blockIdx.z * 4 + zl;
+    if (x >= g.nx || z >= g.nz) return;
+    const float fx = (float)x, fz = (float)z;
+    const BpCol c = bp_col(g, v, fx, fz, y0, y1);
+    if (!rot_y || (c.live && c.nr > BP_ROWS)) {
+        bp_column<K>(g, v, BpRowsLdg{corr, g.W}, vol, x, y0, z, alpha, gmax);
+        return;
+    }
+    if (!c.live) return;
+    const float *row = table + zl * BP_PITCH + xl - RS * (c.r0 + 1);
+    const float top = bp_top(gmax);
+    T *col = vol + x + (size_t)y0 * g.nx + (size_t)z * g.nx * g.ny;
+    if (y1 - y0 == K && c.ulo >= 2.0f + BP_NEAR && c.uhi < (float)(g.H - 2) - BP_NEAR) {  // every voxel is updated
+        float vox[BP_G];
+#pragma unroll
+        for (int q = 0; q < BP_G; ++q) vox[q] = ld_stored(col + q * g.nx);
+#pragma unroll 1
+        for (int k = 0; k < K; k += BP_G) {
+            float next[BP_G];
+#pragma unroll
+            for (int q = 0; q < BP_G; ++q)
+                if (k + BP_G < K) next[q] = ld_stored(col + (BP_G + q) * g.nx);
+#pragma unroll
+            for (int q = 0; q < BP_G; ++q) {
+                const float upy = bp_coord(g.cy, bp_cam(v, 1, fx, (float)(y0 + k + q), fz), c.scale);
+                const int py = (int)upy;  // (inside: bp_tap leaves it)
+                float wy[4];
+                bp_weights(upy - (float)py, wy);
+                const float *w = row + RS * py;
+                const float s[4] = {w[0], w[RS], w[2 * RS], w[3 * RS]};
+                st_stored(col + q * g.nx, bp_value(vox[q], alpha, bp_sum(s, wy), top));
+            }
+            col += BP_G * g.nx;
+#pragma unroll
+            for (int q = 0; q < BP_G; ++q) vox[q] = next[q];
+        }
+        return;
+    }
+    for (int y = y0; y < y1; ++y, col += g.nx) {
+        const float camy = bp_cam(v, 1, fx, (float)y, fz), upy = bp_coord(g.cy, camy, c.scale);
+        if (!bp_inside(g, upy, g.cy, camy, c.ndepth, g.H)) continue;
+        const int py = bp_tap(upy, g.H);
+        float wy[4];
+        bp_weights(upy - (float)py, wy);
+        const float *w = row + RS * py;
+        const float s[4] = {w[0], w[RS], w[2 * RS], w[3 * RS]};
+        st_stored(col, bp_value(ld_stored(col), alpha, bp_sum(s, wy), top));
+    }
 }
 
 // The dual and primal steps of one frame (pd_dual_at, pd_primal_at in
@@ -187,28 +270,27 @@ cudaError_t launch_fill_seeded(long long n, unsigned long long seed, float *x, c
 }
 
 namespace {
-template <int K, typename T, bool PF = false>
-void bp_cols(const GeomDev &g, const ViewRec *views, const ViewSel &sel, T *vol, float alpha, float gmax,
-             cudaStream_t s, unsigned long long tex) {
-    k_bp_voxel_cols<K, T, PF><<<dim3((g.nx + 127) / 128, (g.ny + K - 1) / K, g.nz), 128, 0, s>>>(
-        g, views, sel, vol, alpha, gmax, tex);
+template <int K, int OCC, typename T>
+cudaError_t bp_cols(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr, T *vol, float alpha,
+                    float gmax, cudaStream_t s) {
+    k_bp_voxel_cols<K, OCC, T><<<dim3((g.nx + 31) / 32, (g.ny + K - 1) / K, (g.nz + 3) / 4), 128, 0, s>>>(
+        g, views, sel, corr, vol, alpha, gmax);
+    return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t bp_voxel_any(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr, T *vol,
-                         float alpha, float gmax, cudaStream_t s, unsigned long long corr_tex, int bp_variant) {
-    if (corr_tex) {
-        switch (bp_variant) {
-        case 1: bp_cols<8>(g, views, sel, vol, alpha, gmax, s, corr_tex); break;
-        case 2: bp_cols<32>(g, views, sel, vol, alpha, gmax, s, corr_tex); break;
-        case 3: bp_cols<16, T, true>(g, views, sel, vol, alpha, gmax, s, corr_tex); break;
-        case 4: bp_cols<32, T, true>(g, views, sel, vol, alpha, gmax, s, corr_tex); break;
-        default: bp_cols<BP_COL>(g, views, sel, vol, alpha, gmax, s, corr_tex); break;
-        }
-    } else {
-        k_bp_voxel<false, T><<<vox_grid(g.nx, g.ny, g.nz), 128, 0, s>>>(g, views, sel, corr, vol, alpha, gmax, 0);
+                         float alpha, float gmax, cudaStream_t s, int bp_variant) {
+    switch (bp_variant) {
+    case 1: return bp_cols<8, 8>(g, views, sel, corr, vol, alpha, gmax, s);
+    case 2: return bp_cols<20, 8>(g, views, sel, corr, vol, alpha, gmax, s);
+    case 3: return bp_cols<16, 6>(g, views, sel, corr, vol, alpha, gmax, s);
+    case 4: return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s);
+    default: break;
     }
-    return cudaGetLastError();
+    if (g.bp_len == 8) return bp_cols<8, 8>(g, views, sel, corr, vol, alpha, gmax, s);
+    if (g.bp_len == 12) return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s);
+    return bp_cols<16, 8>(g, views, sel, corr, vol, alpha, gmax, s);
 }
 
 template <typename T>
@@ -242,53 +324,31 @@ cudaError_t pd_extrapolate_any(const int *d, const int *cut, const T *vol, const
 }
 }  // namespace
 
-cudaError_t make_corr_tex(int W, int H, CorrTex &o) {
-    o = CorrTex{};
-    cudaChannelFormatDesc cd = cudaCreateChannelDesc<float>();
-    cudaError_t e = cudaMalloc3DArray(&o.arr, &cd, make_cudaExtent(W, H, 1), cudaArrayLayered | cudaArraySurfaceLoadStore);
-    if (e != cudaSuccess) return e;
-    cudaResourceDesc rd{};
-    rd.resType = cudaResourceTypeArray;
-    rd.res.array.array = o.arr;
-    cudaTextureDesc td{};
-    td.addressMode[0] = td.addressMode[1] = td.addressMode[2] = cudaAddressModeClamp;
-    td.filterMode = cudaFilterModePoint;
-    td.readMode = cudaReadModeElementType;
-    td.normalizedCoords = 0;
-    cudaTextureObject_t t = 0;
-    cudaSurfaceObject_t sf = 0;
-    if ((e = cudaCreateTextureObject(&t, &rd, &td, nullptr)) == cudaSuccess) e = cudaCreateSurfaceObject(&sf, &rd);
-    o.tex = t;
-    o.surf = sf;
-    o.W = W;
-    o.H = H;
-    if (e != cudaSuccess) free_corr_tex(o);
-    return e;
-}
-
-void free_corr_tex(CorrTex &o) {
-    if (o.surf) cudaDestroySurfaceObject((cudaSurfaceObject_t)o.surf);
-    if (o.tex) cudaDestroyTextureObject((cudaTextureObject_t)o.tex);
-    if (o.arr) cudaFreeArray(o.arr);
-    o = CorrTex{};
+int bp_default_len(double rows) {
+    // (K - 1) steps of `rows` between the first and the last voxel, their
+    // windows' 4 rows, and one for where the run starts within a row
+    for (int k : {16, 12})
+        if ((k - 1) * rows + 5.0 <= BP_ROWS) return k;
+    return 8;
 }
 
 const char *bp_variant_name(int v) {
-    static const char *names[kBpVariants] = {"columns of 16 voxels", "columns of 8 voxels", "columns of 32 voxels",
-                                             "columns of 16 voxels, L2 prefetch", "columns of 32 voxels, L2 prefetch"};
+    static const char *names[kBpVariants] = {"columns of 16, 12 or 8 voxels by the magnification, 8 blocks per SM",
+                                             "columns of 8 voxels, 8 blocks per SM",
+                                             "columns of 20 voxels, 8 blocks per SM",
+                                             "columns of 16 voxels, 6 blocks per SM",
+                                             "columns of 12 voxels, 8 blocks per SM"};
     return v >= 0 && v < kBpVariants ? names[v] : "?";
 }
 
 cudaError_t launch_bp_voxel(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                            float *vol, float alpha, float gmax, cudaStream_t s, unsigned long long corr_tex,
-                            int bp_variant) {
-    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, corr_tex, bp_variant);
+                            float *vol, float alpha, float gmax, cudaStream_t s, int bp_variant) {
+    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, bp_variant);
 }
 
 cudaError_t launch_bp_voxel(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                            unsigned short *vol, float alpha, float gmax, cudaStream_t s, unsigned long long corr_tex,
-                            int bp_variant) {
-    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, corr_tex, bp_variant);
+                            unsigned short *vol, float alpha, float gmax, cudaStream_t s, int bp_variant) {
+    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, bp_variant);
 }
 
 cudaError_t launch_pd_dual(const int *d, const PdParams &p, const float *xf, const float *xf1,

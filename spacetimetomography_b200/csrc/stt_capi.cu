@@ -141,7 +141,6 @@ stt_status stt_destroy(stt_ctx *ctx) {
     cudaFree(ctx->pwd);
     cudaFree(ctx->status);
     for (auto &e : ctx->fp_tex) stt::destroy_fp_tex(e.tex);
-    stt::free_corr_tex(ctx->corr_tex);
     delete ctx;
     return STT_OK;
 }
@@ -278,6 +277,8 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g) {
     d.cx = (float)((g->W - 1) * 0.5);
     d.cy = (float)((g->H - 1) * 0.5);
     d.sdd_ds = (float)(g->sdd / g->ds);
+    // detector rows per voxel where the volume comes nearest to the source (sid exceeds the reach, checked above)
+    d.bp_len = stt::bp_default_len(g->sdd / g->ds * g->sy / (g->sid - std::sqrt(hx * hx + hz * hz) - off));
     ctx->sp[0] = g->sx;
     ctx->sp[1] = g->sy;
     ctx->sp[2] = g->sz;
@@ -383,7 +384,7 @@ stt_status stt_fp_correction(stt_ctx *ctx, const float *vol, const float *b, flo
     if ((st = transposed_if_needed(ctx, vol, view, 1, S(stream), &volt))) return st;
     stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
     if (staged_mask(ctx, vol)) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
-    STT_CUDA(ctx, stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, b, raylen_state, corr, S(stream), 0, &maps,
+    STT_CUDA(ctx, stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, b, raylen_state, corr, S(stream), &maps,
                                       ctx->status, ctx->tuning.fp, stt::ctx_fp_tex(ctx, vol, volt)),
              "k_fp_corr launch");
     return STT_OK;
@@ -441,26 +442,6 @@ stt_status stt_fp_vjp(stt_ctx *ctx, const float *proj_bar, float *vol_bar, int v
 
 }  // extern "C"
 
-static void ensure_corr_tex(stt_ctx *ctx);
-
-// The caller's correction copied into the context's texture (stream-ordered,
-// W*H*4 bytes) for the column backprojection; 0 (the per-voxel load form)
-// for volumes under 2^23 voxels, or where the texture cannot be made or the
-// copy fails.  Measured per view, copy included: 256^3 / 512^2 102 us against
-// 130 us for the load form; 128^3 / 128^2 18.3 us against 13.9 us.
-static unsigned long long bp_corr_texture(stt_ctx *ctx, const float *corr, cudaStream_t s) {
-    if ((long long)ctx->g.nx * ctx->g.ny * ctx->g.nz < (1LL << 23)) return 0;
-    ensure_corr_tex(ctx);
-    if (!ctx->corr_tex.tex) return 0;
-    const size_t row = (size_t)ctx->g.W * sizeof(float);
-    if (cudaMemcpy2DToArrayAsync(ctx->corr_tex.arr, 0, 0, corr, row, row, ctx->g.H, cudaMemcpyDeviceToDevice, s) !=
-        cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    return ctx->corr_tex.tex;
-}
-
 extern "C" {
 
 stt_status stt_bp_voxel(stt_ctx *ctx, const float *corr, float *vol, double alpha, float gmax,
@@ -471,9 +452,7 @@ stt_status stt_bp_voxel(stt_ctx *ctx, const float *corr, float *vol, double alph
     if ((st = check_views(ctx, view, 1))) return st;
     if ((st = set_device(ctx))) return st;
     const stt::ViewSel sel{view, nullptr, 0, view};
-    const unsigned long long tex = bp_corr_texture(ctx, corr, S(stream));
-    STT_CUDA(ctx, stt::launch_bp_voxel(ctx->g, ctx->views_d, sel, corr, vol, (float)alpha, gmax, S(stream), tex,
-                                       ctx->tuning.bp),
+    STT_CUDA(ctx, stt::launch_bp_voxel(ctx->g, ctx->views_d, sel, corr, vol, (float)alpha, gmax, S(stream), ctx->tuning.bp),
              "k_bp_voxel launch");
     return STT_OK;
 }
@@ -488,9 +467,8 @@ stt_status stt_bp_voxel_typed(stt_ctx *ctx, const float *corr, void *vol, int dt
     if ((st = check_views(ctx, view, 1))) return st;
     if ((st = set_device(ctx))) return st;
     const stt::ViewSel sel{view, nullptr, 0, view};
-    const unsigned long long tex = bp_corr_texture(ctx, corr, S(stream));
     STT_CUDA(ctx, stt::launch_bp_voxel(ctx->g, ctx->views_d, sel, corr, static_cast<unsigned short *>(vol),
-                                       (float)alpha, gmax, S(stream), tex, ctx->tuning.bp),
+                                       (float)alpha, gmax, S(stream), ctx->tuning.bp),
              "k_bp_voxel launch");
     return STT_OK;
 }
@@ -554,34 +532,19 @@ stt_status stt_bp_ray_scatter(stt_ctx *ctx, const float *corr, float *contrib, f
 // The fused forward projection of one view of a sweep: FP32 through the tuned
 // gather variant and, where its maps apply, the slab-staged kernel; BF16
 // through the gather kernel and the slab kernel's BF16 boxes.
-// The context's texture copy of a W x H correction for the column
-// backprojection, made on first use (kept until stt_destroy or a detector of
-// another size); where it cannot be made, corr_tex.tex stays 0 and the
-// per-voxel load form runs (the same bits).
-static void ensure_corr_tex(stt_ctx *ctx) {
-    if (ctx->corr_tex.tex && ctx->corr_tex.W == ctx->g.W && ctx->corr_tex.H == ctx->g.H) return;
-    // another detector size: launches enqueued earlier (on any stream) may still
-    // gather from the old texture, so the device drains before it is destroyed
-    if (ctx->corr_tex.tex && cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
-    stt::free_corr_tex(ctx->corr_tex);
-    if (stt::make_corr_tex(ctx->g.W, ctx->g.H, ctx->corr_tex) != cudaSuccess) cudaGetLastError();
-}
-
-// surf: also write the correction into the context's texture copy (0: not).
 static cudaError_t sweep_fp_corr(stt_ctx *ctx, const float *vol, const float *volt, const stt::ViewSel &sel,
-                                 const float *stack, float *rl, cudaStream_t s, unsigned long long surf) {
+                                 const float *stack, float *rl, cudaStream_t s) {
     stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
     if (staged_mask(ctx, vol)) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
-    return stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, rl, ctx->corr, s, surf, &maps,
+    return stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, rl, ctx->corr, s, &maps,
                                ctx->status, ctx->tuning.fp, stt::ctx_fp_tex(ctx, vol, volt));
 }
 
 static cudaError_t sweep_fp_corr(stt_ctx *ctx, const unsigned short *vol, const unsigned short *volt,
-                                 const stt::ViewSel &sel, const unsigned short *stack, float *rl, cudaStream_t s,
-                                 unsigned long long surf) {
+                                 const stt::ViewSel &sel, const unsigned short *stack, float *rl, cudaStream_t s) {
     stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
     if (staged_mask(ctx, vol)) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
-    return stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, rl, ctx->corr, s, surf, &maps,
+    return stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, rl, ctx->corr, s, &maps,
                                ctx->status, ctx->tuning.fp16, stt::ctx_fp_tex(ctx, vol, volt));
 }
 
@@ -631,19 +594,17 @@ static stt_status sart_sweep_t(stt_ctx *ctx, T *vol, const T *proj_stack, const 
     const size_t npix = (size_t)ctx->g.W * ctx->g.H;
     if ((st = ensure(ctx, ctx->corr, ctx->corr_n, npix, "correction image"))) return st;
     if (bp_mode == 1 && (st = ensure_acc(ctx, s))) return st;
-    if (bp_mode == 0) ensure_corr_tex(ctx);
     for (int i = 0; i < nperm; ++i) {
         const stt::ViewSel sel{view_offset + perm[i], nullptr, 0, view_offset};
         const T *volt = nullptr;
         if ((st = transposed_if_needed(ctx, vol, view_offset + perm[i], 1, s, &volt))) return st;
         // ray-based mode: TypicalRayProducer::Initial zeroes the ray lengths
         // after every view, so missed rays see L = 0 (no sticky state)
-        STT_CUDA(ctx, sweep_fp_corr(ctx, vol, volt, sel, proj_stack, bp_mode == 0 ? raylen_state : nullptr, s,
-                                    bp_mode == 0 ? ctx->corr_tex.surf : 0),
+        STT_CUDA(ctx, sweep_fp_corr(ctx, vol, volt, sel, proj_stack, bp_mode == 0 ? raylen_state : nullptr, s),
                  "k_fp_corr launch");
         if (bp_mode == 0)
             STT_CUDA(ctx, stt::launch_bp_voxel(ctx->g, ctx->views_d, sel, ctx->corr, vol, (float)alpha, gmax, s,
-                                               ctx->corr_tex.tex, ctx->tuning.bp),
+                                               ctx->tuning.bp),
                      "k_bp_voxel launch");
         else
             STT_CUDA(ctx, stt::launch_bp_ray(ctx->g, ctx->views_d, sel, ctx->corr, ctx->acc, vol, gmax, s,

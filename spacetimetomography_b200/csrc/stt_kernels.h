@@ -27,8 +27,8 @@ int grid_stride_blocks(long long n, int threads);
 //         in flight and, for variants 10 and 11, corners fetched as two tld4
 //         texture gathers per sample instead of eight loads (fp_variant_name);
 //   slab: the box of the slab-staged projector (slab_variant_name);
-//   bp:   the column length of the voxel backprojection, and whether each
-//         column's voxels are first prefetched into L2 (bp_variant_name);
+//   bp:   the column length of the voxel backprojection and the blocks per SM
+//         it is compiled for (bp_variant_name);
 //   ray:  the scatter of the ray-driven backprojection (ray_variant_name):
 //         0 one global vector atomic per corner, 1 a shared-memory box per
 //         slab (volumes below 2^31 voxels).  Its sums differ in float order
@@ -72,11 +72,11 @@ bool make_fp_slab_maps(const GeomDev &g, const unsigned short *vol, const unsign
 bool encode_planes_map(CUtensorMap *m, const float *ptr, int nx, int ny, int nz, int nc, const unsigned box[4]);
 cudaError_t launch_fp_corr_slab(const GeomDev &g, const ViewRec *views, const FpSlabMaps &m, const float *vol,
                                 const float *vol_t, const ViewSel &sel, const float *b_stack, float *raylen_state,
-                                float *corr, cudaStream_t s, unsigned long long corr_surf, int *status);
+                                float *corr, cudaStream_t s, int *status);
 cudaError_t launch_fp_corr_slab(const GeomDev &g, const ViewRec *views, const FpSlabMaps &m,
                                 const unsigned short *vol, const unsigned short *vol_t, const ViewSel &sel,
                                 const unsigned short *b_stack, float *raylen_state, float *corr, cudaStream_t s,
-                                unsigned long long corr_surf, int *status);
+                                int *status);
 // Texture objects of the gather variants that fetch corners with tld4: the
 // volume as a pitch-linear 2D texture whose rows are its z slices (width
 // nx*ny texels, nz rows) and its z-fastest copy likewise (rows the x slices;
@@ -109,7 +109,7 @@ void destroy_fp_tex(FpTex &t);
 // same shape, which gives the same bits.
 cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t,
                            const ViewSel &sel, const float *b_stack, float *raylen_state, float *corr,
-                           cudaStream_t s, unsigned long long corr_surf = 0, const FpSlabMaps *maps = nullptr,
+                           cudaStream_t s, const FpSlabMaps *maps = nullptr,
                            int *status = nullptr, int fp_variant = 0, const FpTex *tex = nullptr);
 cudaError_t launch_transpose(const GeomDev &g, const float *in, float *out, cudaStream_t s);
 cudaError_t launch_fp_bf16(const GeomDev &g, const ViewRec *views, const unsigned short *vol,
@@ -137,7 +137,7 @@ constexpr int kFp16Variants = 2;
 const char *fp16_variant_name(int v);
 cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigned short *vol,
                            const unsigned short *vol_t, const ViewSel &sel, const unsigned short *b_stack,
-                           float *raylen_state, float *corr, cudaStream_t s, unsigned long long corr_surf = 0,
+                           float *raylen_state, float *corr, cudaStream_t s,
                            const FpSlabMaps *maps = nullptr, int *status = nullptr, int fp_variant16 = 0,
                            const FpTex *tex = nullptr);
 cudaError_t launch_correction(long long n, const unsigned short *b, const float *ax, const float *raylen,
@@ -192,25 +192,14 @@ cudaError_t launch_sweep_persistent(const SweepJob *jobs_d, int njobs, int nbloc
 cudaError_t launch_iter_persistent(const SweepJob *jobs_d, int njobs, int nblocks, bool bf16, bool wide,
                                    unsigned *gbar, int *status, cudaStream_t s);
 
-// The correction image held as a one-layer layered CUDA array: the texture
-// object the column backprojection gathers from (tld4) and the surface object
-// the fused forward projection writes (launch_fp_corr's corr_surf).
-struct CorrTex {
-    cudaArray_t arr = nullptr;
-    unsigned long long tex = 0, surf = 0;
-    int W = 0, H = 0;
-};
-cudaError_t make_corr_tex(int W, int H, CorrTex &o);
-void free_corr_tex(CorrTex &o);
-
-// Voxel-driven backprojection; with the correction as a texture (corr_tex)
-// the column walk of bp variant `bp_variant` runs, else the per-voxel form.
+// Voxel-driven backprojection, bp variant `bp_variant` (0: columns of g.bp_len voxels).
+// bp_default_len: the longest column whose detector rows fit in the kernel's
+// table at `rows` detector rows per voxel (the geometry's largest).
+int bp_default_len(double rows);
 cudaError_t launch_bp_voxel(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                            float *vol, float alpha, float gmax, cudaStream_t s, unsigned long long corr_tex = 0,
-                            int bp_variant = 0);
+                            float *vol, float alpha, float gmax, cudaStream_t s, int bp_variant = 0);
 cudaError_t launch_bp_voxel(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                            unsigned short *vol, float alpha, float gmax, cudaStream_t s,
-                            unsigned long long corr_tex = 0, int bp_variant = 0);
+                            unsigned short *vol, float alpha, float gmax, cudaStream_t s, int bp_variant = 0);
 // Sets the solver's device-side iteration counter (stream-ordered, no host memory read).
 cudaError_t launch_set_counter(unsigned long long *counter, unsigned long long v, cudaStream_t s);
 // View orders of `frames` local frames (at most 1024), local frame f being

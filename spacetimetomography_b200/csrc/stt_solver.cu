@@ -99,7 +99,6 @@ struct stt_solver {
     cudaGraphExec_t pexec[2] = {nullptr, nullptr};
     long long launches_per_iter = 0;
     long long phase_launches[2] = {0, 0};
-    std::vector<stt::CorrTex> corr_tex;  // batched modes: per frame, the correction as a texture
     std::vector<stt::FpSlabMaps> fpmaps;  // batched modes: per frame, TMA maps of the volume and its copy
     std::vector<stt::FpTex> fptex;  // batched modes, a tld4 gather form: per frame, the volume's textures
     stt::SweepJob *jobs_d = nullptr;  // STT_SOLVE_PERSISTENT: one job per frame
@@ -203,18 +202,17 @@ stt_status enqueue_primal(stt_solver *s, int f, cudaStream_t cs, long long &nl) 
 // gather variant and, where the maps apply, the slab-staged kernel; BF16
 // storage through the gather kernel.  Returns the kernels launched.
 int fp_corr(stt_solver *s, int f, const float *vol, const float *volt, const stt::ViewSel &sel, const float *stack,
-            float *rl, float *corr, cudaStream_t cs, unsigned long long surf, cudaError_t &e) {
+            float *rl, float *corr, cudaStream_t cs, cudaError_t &e) {
     const stt::FpSlabMaps *maps = s->fpmaps.empty() ? nullptr : &s->fpmaps[f];
-    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, surf, maps, s->status,
+    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status,
                             s->ctx->tuning.fp, s->fptex.empty() ? nullptr : &s->fptex[f]);
     return (maps && maps->ok) ? 2 : 1;  // slab-staged + gather kernels, or gather only
 }
 
 int fp_corr(stt_solver *s, int f, const unsigned short *vol, const unsigned short *volt, const stt::ViewSel &sel,
-            const unsigned short *stack, float *rl, float *corr, cudaStream_t cs, unsigned long long surf,
-            cudaError_t &e) {
+            const unsigned short *stack, float *rl, float *corr, cudaStream_t cs, cudaError_t &e) {
     const stt::FpSlabMaps *maps = s->fpmaps.empty() ? nullptr : &s->fpmaps[f];
-    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, surf, maps, s->status,
+    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status,
                             s->ctx->tuning.fp16, s->fptex.empty() ? nullptr : &s->fptex[f]);
     return (maps && maps->ok) ? 2 : 1;
 }
@@ -231,14 +229,12 @@ stt_status enqueue_sart_batched(stt_solver *s, int f, cudaStream_t cs, long long
     for (int i = 0; i < V; ++i) {
         const stt::ViewSel sel{0, s->perm + (size_t)f * V, i, f * V};
         SCUDA(s, stt::launch_transpose_for_view(g, s->views, sel, vol, volt, cs), "transpose");
-        const bool tex = voxel && !s->corr_tex.empty();
         cudaError_t e = cudaSuccess;
-        nl += fp_corr(s, f, vol, volt, sel, stack, voxel ? s->raylen + f * s->npix : nullptr, corr, cs,
-                      tex ? s->corr_tex[f].surf : 0, e);
+        nl += fp_corr(s, f, vol, volt, sel, stack, voxel ? s->raylen + f * s->npix : nullptr, corr, cs, e);
         SCUDA(s, e, "fp_corr");
         if (voxel)
             SCUDA(s, stt::launch_bp_voxel(g, s->views, sel, corr, vol, (float)s->cfg.alpha, s->cfg.pd.gmax, cs,
-                                          tex ? s->corr_tex[f].tex : 0, s->ctx->tuning.bp),
+                                          s->ctx->tuning.bp),
                   "bp_voxel");
         else
             SCUDA(s, stt::launch_bp_ray(g, s->views, sel, corr, s->acc + f * s->n, vol, s->cfg.pd.gmax, cs,
@@ -589,7 +585,7 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
     // no views staged for this storage (the tuner found one gather launch per
     // view faster than the two kernels): no maps, one launch per view
     const bool any_staged = (cfg->storage == STT_DTYPE_F32 ? ctx->staged_bins : ctx->staged_bins16) != 0;
-    // (the persistent sweep gathers with loads: no maps, textures or texture copy of the correction)
+    // (the persistent sweep gathers with loads: no maps or textures)
     const bool per_view_kernels = cfg->mode == STT_SOLVE_STREAMS || cfg->mode == STT_SOLVE_GRAPH;
     if (per_view_kernels && any_staged) {
         s->fpmaps.resize(F);
@@ -613,15 +609,6 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
         for (int f = 0; f < F; ++f)
             stt::make_fp_tex(*g, reinterpret_cast<const unsigned short *>(s->st.vol) + f * s->n,
                              static_cast<unsigned short *>(s->volt) + f * s->n, s->fptex[f]);
-    }
-    if (per_view_kernels && cfg->bp_mode == 0) {
-        s->corr_tex.resize(F);
-        for (int f = 0; f < F; ++f)
-            if (stt::make_corr_tex(g->W, g->H, s->corr_tex[f]) != cudaSuccess) {
-                cudaGetLastError();
-                stt_solver_destroy(s);
-                return STT_ERR_NOMEM;
-            }
     }
     if (cfg->mode == STT_SOLVE_PERSISTENT) {
         s->sweep_wide = (long long)g->nx * g->ny * g->nz >= (1LL << 31);  // 64-bit gather offsets
@@ -830,7 +817,6 @@ stt_status stt_solver_destroy(stt_solver *s) {
     for (auto e : s->ev_done)
         if (e) cudaEventDestroy(e);
     if (s->ev_fork) cudaEventDestroy(s->ev_fork);
-    for (auto &t : s->corr_tex) stt::free_corr_tex(t);
     for (auto &t : s->fptex) stt::destroy_fp_tex(t);
     cudaFree(s->jobs_d);
     cudaFree(s->sweep_bar);

@@ -55,8 +55,6 @@ struct Scratch {
     float2 *acc = nullptr;
     unsigned short *vol16 = nullptr, *volt16 = nullptr, *b16 = nullptr;  // BF16 copies for the BF16 choice
     stt::ViewRec *tv = nullptr;
-    cudaArray_t arr = nullptr;
-    cudaTextureObject_t tex = 0;
     stt::FpTex fptex;    // the textures of the tld4 gather variants over vol and volt
     stt::FpTex fptex16;  // the same over vol16 and volt16
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -73,8 +71,6 @@ struct Scratch {
         cudaFree(volt16);
         cudaFree(b16);
         cudaFree(tv);
-        if (tex) cudaDestroyTextureObject(tex);
-        if (arr) cudaFreeArray(arr);
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
     }
@@ -249,19 +245,6 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
         (e = cudaMalloc(&sc.corr, npix * sizeof(float))) || (e = cudaMalloc(&sc.tv, 2 * sizeof(stt::ViewRec))) ||
         (e = cudaEventCreate(&sc.e0)) || (e = cudaEventCreate(&sc.e1)))
         return fail(e, "scratch");
-    {  // the correction as a one-layer texture, as the solver's backprojection reads it
-        cudaChannelFormatDesc cd = cudaCreateChannelDesc<float>();
-        if ((e = cudaMalloc3DArray(&sc.arr, &cd, make_cudaExtent(g.W, g.H, 1), cudaArrayLayered)))
-            return fail(e, "texture array");
-        cudaResourceDesc rd{};
-        rd.resType = cudaResourceTypeArray;
-        rd.res.array.array = sc.arr;
-        cudaTextureDesc td{};
-        td.addressMode[0] = td.addressMode[1] = td.addressMode[2] = cudaAddressModeClamp;
-        td.filterMode = cudaFilterModePoint;
-        td.readMode = cudaReadModeElementType;
-        if ((e = cudaCreateTextureObject(&sc.tex, &rd, &td, nullptr))) return fail(e, "texture object");
-    }
     // the times do not depend on the values; these are positive and typical enough
     if ((e = stt::launch_fill_seeded((long long)n, 7, sc.vol, s)) || (e = stt::launch_transpose(g, sc.vol, sc.volt, s)) ||
         (e = cudaMemsetAsync(sc.b, 0, npix * sizeof(float), s)) || (e = cudaMemsetAsync(sc.rl, 0, npix * sizeof(float), s)))
@@ -296,7 +279,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
                 continue;
             }
             e = time_us(sc, s, [&] {
-                return stt::launch_fp_corr(g, sc.tv, sc.vol, sc.volt, gather_sel, sc.b, sc.rl, sc.corr, s, 0, nullptr,
+                return stt::launch_fp_corr(g, sc.tv, sc.vol, sc.volt, gather_sel, sc.b, sc.rl, sc.corr, s, nullptr,
                                            ctx->status, fv, &sc.fptex);
             }, tg[fv][b]);
             if (e) return fail(e, "gather projector");
@@ -306,7 +289,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
             while (!maps_ok[sv0]) ++sv0;
             e = time_us(sc, s, [&] {
                 return stt::launch_fp_corr_slab(g, sc.tv, maps[sv0], sc.vol, sc.volt, gather_sel, sc.b, sc.rl, sc.corr,
-                                                s, 0, ctx->status);
+                                                s, ctx->status);
             }, t_idle);
             if (e) return fail(e, "idle slab launch");
         }
@@ -314,7 +297,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
             if (!maps_ok[sv]) continue;
             e = time_us(sc, s, [&] {
                 return stt::launch_fp_corr_slab(g, sc.tv, maps[sv], sc.vol, sc.volt, slab_sel, sc.b, sc.rl, sc.corr, s,
-                                                0, ctx->status);
+                                                ctx->status);
             }, ts[sv][b]);
             if (e) return fail(e, "slab projector");
         }
@@ -397,20 +380,20 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
                 if (fv == 1 && !sc.fptex16.ok) continue;
                 e = time_us(sc, s, [&] {
                     return stt::launch_fp_corr(g, sc.tv, sc.vol16, sc.volt16, stt::ViewSel{0, nullptr, 0, 0}, sc.b16,
-                                               sc.rl, sc.corr, s, 0, nullptr, ctx->status, fv, &sc.fptex16);
+                                               sc.rl, sc.corr, s, nullptr, ctx->status, fv, &sc.fptex16);
                 }, tg16[fv][b]);
                 if (e) return fail(e, "BF16 gather projector");
             }
             if (!maps16) continue;
             e = time_us(sc, s, [&] {
                 return stt::launch_fp_corr_slab(g, sc.tv, m16, sc.vol16, sc.volt16, stt::ViewSel{1, nullptr, 0, 1},
-                                                sc.b16, sc.rl, sc.corr, s, 0, ctx->status);
+                                                sc.b16, sc.rl, sc.corr, s, ctx->status);
             }, ts16[b]);
             if (e) return fail(e, "BF16 slab projector");
             if (t_idle16 == 0.0f) {
                 e = time_us(sc, s, [&] {
                     return stt::launch_fp_corr_slab(g, sc.tv, m16, sc.vol16, sc.volt16, stt::ViewSel{0, nullptr, 0, 0},
-                                                    sc.b16, sc.rl, sc.corr, s, 0, ctx->status);
+                                                    sc.b16, sc.rl, sc.corr, s, ctx->status);
                 }, t_idle16);
                 if (e) return fail(e, "idle BF16 slab launch");
             }
@@ -443,9 +426,6 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
         }
     }
     // voxel backprojection: the column lengths on the views of the first and last classes present
-    if ((e = cudaMemcpy2DToArrayAsync(sc.arr, 0, 0, sc.corr, g.W * sizeof(float), g.W * sizeof(float), g.H,
-                                      cudaMemcpyDeviceToDevice, s)))
-        return fail(e, "texture fill");
     {
         int vb[2] = {-1, -1};
         for (int b = 0; b < 9; ++b)
@@ -464,7 +444,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
                 float us = 0.0f;
                 e = time_us(sc, s, [&] {
                     return stt::launch_bp_voxel(g, sc.tv, stt::ViewSel{0, nullptr, 0, 0}, sc.corr, sc.vol, 0.3f,
-                                                1e30f, s, sc.tex, bv);
+                                                1e30f, s, bv);
                 }, us);
                 if (e) return fail(e, "voxel backprojection");
                 tot += us;

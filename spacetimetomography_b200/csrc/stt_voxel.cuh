@@ -121,7 +121,7 @@ __device__ __forceinline__ void pd_primal_at(int i, int j, int k, int nx, int ny
 
 // Voxel-based backprojection (ST_Tomography.cpp:690-730): project the voxel
 // centre, Catmull-Rom 4x4 gather of the correction image (y first, then x),
-// vol += alpha*val, clamp to [0, gmax]; voxels whose footprint leaves
+// vol += alpha*val, clamp to [0, gmax]; voxels projecting outside
 // [2, W-2) x [2, H-2) are untouched.  Every product and sum is rounded on its
 // own (explicit intrinsics), so the per-voxel and the column forms below give
 // the same bits whichever way their taps are fetched.
@@ -131,70 +131,80 @@ __device__ __forceinline__ float bp_cam(const ViewRec &v, int r, float fx, float
     return __fadd_rn(__fmaf_rn(v.A[3 * r + 2], fz, __fmaf_rn(v.A[3 * r + 1], fy, __fmul_rn(v.A[3 * r], fx))), v.b[r]);
 }
 
-// Detector coordinate c + cam/(-depth) * sdd/ds.
-__device__ __forceinline__ float bp_pixel(float c, float cam, float ndepth, float sdd_ds) {
-    return __fmaf_rn(__fdiv_rn(cam, ndepth), sdd_ds, c);
-}
+// One detector axis of a voxel: the coordinate u = c + cam sdd/(ds depth), its
+// 4-tap window's second tap p and the fraction d, and whether the voxel is
+// used at all (2 <= u < n - 2, the reference's cutoff).  sdd/(ds depth) is
+// formed once per depth (bp_scale), so a coordinate is one multiply-add; the
+// cutoff, which is a jump, is decided within BP_NEAR pixels of a border by the
+// coordinate as ST_Tomography.cpp:698-709 forms it, c + (cam/depth) sdd/ds, in
+// its operation order.  u does not fall as cam grows.
+constexpr float BP_NEAR = 0.0625f;
 
-// Catmull-Rom weights of taps (-1, 0, +1, +2) at fraction d.
+__device__ __forceinline__ float bp_scale(const GeomDev &g, float ndepth) { return __fdiv_rn(g.sdd_ds, ndepth); }
+__device__ __forceinline__ float bp_coord(float c, float cam, float scale) { return __fmaf_rn(cam, scale, c); }
+__device__ __forceinline__ bool bp_inside(const GeomDev &g, float u, float c, float cam, float ndepth, int n) {
+    const float lo = 2.0f, hi = (float)(n - 2);
+    if (u >= lo + BP_NEAR && u < hi - BP_NEAR) return true;
+    if (!(u >= lo - BP_NEAR && u < hi + BP_NEAR)) return false;
+    const float e = __fmaf_rn(__fdiv_rn(cam, ndepth), g.sdd_ds, c);
+    return e >= lo && e < hi;
+}
+__device__ __forceinline__ int bp_tap(float u, int n) { return min(max((int)u, 2), n - 3); }
+
+// Catmull-Rom weights of taps (-1, 0, +1, +2) at fraction d, in Horner form.
 __device__ __forceinline__ void bp_weights(float d, float w[4]) {
-    const float d2 = __fmul_rn(d, d), d3 = __fmul_rn(d2, d);
-    w[0] = __fmul_rn(0.5f, __fsub_rn(__fmaf_rn(2.0f, d2, -d), d3));
-    w[1] = __fadd_rn(1.0f, __fmul_rn(0.5f, __fmaf_rn(3.0f, d3, __fmul_rn(-5.0f, d2))));
-    w[2] = __fmul_rn(0.5f, __fmaf_rn(-3.0f, d3, __fmaf_rn(4.0f, d2, d)));
-    w[3] = __fmul_rn(0.5f, __fsub_rn(d3, d2));
+    w[0] = __fmul_rn(d, __fmaf_rn(d, __fmaf_rn(-0.5f, d, 1.0f), -0.5f));
+    w[1] = __fmaf_rn(__fmul_rn(d, d), __fmaf_rn(1.5f, d, -2.5f), 1.0f);
+    w[2] = __fmul_rn(d, __fmaf_rn(d, __fmaf_rn(-1.5f, d, 2.0f), 0.5f));
+    w[3] = __fmul_rn(__fmul_rn(d, d), __fmaf_rn(0.5f, d, -0.5f));
 }
 
-// sum_a wx[a] * sum_b wy[b] * tap[a][b]; tap[a][b] is column px-1+a, row py-1+b.
-__device__ __forceinline__ float bp_sum(const float tap[4][4], const float wx[4], const float wy[4]) {
-    float val = 0.0f;
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const float s = __fmaf_rn(wy[3], tap[a][3],
-                                  __fmaf_rn(wy[2], tap[a][2], __fmaf_rn(wy[1], tap[a][1], __fmul_rn(wy[0], tap[a][0]))));
-        val = a == 0 ? __fmul_rn(wx[0], s) : __fmaf_rn(wx[a], s, val);
-    }
-    return val;
+// The window's sum, rows first: bp_row is one detector row's four taps
+// (columns px-1 .. px+2) under the x weights, bp_sum the four rows' sums
+// under the y weights.  A row's sum depends on the row and the column's x
+// weights only, so a column of voxels shares it (bp_column keeps a window of
+// four, k_bp_voxel_cols a table).
+__device__ __forceinline__ float bp_row(const float tap[4], const float wx[4]) {
+    return __fmaf_rn(wx[3], tap[3], __fmaf_rn(wx[2], tap[2], __fmaf_rn(wx[1], tap[1], __fmul_rn(wx[0], tap[0]))));
+}
+__device__ __forceinline__ float bp_sum(const float row[4], const float wy[4]) {
+    return __fmaf_rn(wy[3], row[3], __fmaf_rn(wy[2], row[2], __fmaf_rn(wy[1], row[1], __fmul_rn(wy[0], row[0]))));
 }
 
+// The updated voxel: v + alpha*val clamped to [0, gmax] as the reference's
+// macros clamp (a NaN becomes 0).  top = bp_top(gmax), so that two plain
+// minimum / maximum operations do it.
+__device__ __forceinline__ float bp_top(float gmax) { return gmax != gmax ? INFINITY : fmaxf(gmax, 0.0f); }
+__device__ __forceinline__ float bp_value(float v, float alpha, float val, float top) {
+    return fminf(top, fmaxf(__fmaf_rn(alpha, val, v), 0.0f));
+}
 // T: the volume's storage (float, or BF16 bits widened to FP32 and rounded
 // back to nearest even on store).
 template <typename T>
-__device__ __forceinline__ void bp_update(T *__restrict__ vol, size_t o, float alpha, float val, float gmax) {
-    const float nv = __fmaf_rn(alpha, val, ld_stored(vol + o));
-    st_stored(vol + o, rmax(rmin(gmax, nv), 0.0f));
+__device__ __forceinline__ void bp_update(T *__restrict__ vol, size_t o, float alpha, float val, float top) {
+    st_stored(vol + o, bp_value(ld_stored(vol + o), alpha, val, top));
 }
 
-// Fetchers of two correction rows, pyr and pyr + 1, at columns px-1 .. px+2
-// (r0[a], r1[a]: column px-1+a).  All three return the stored values.
-// From the correction's one-layer texture copy: two tld4 gathers.
-struct BpRowsTex {
-    unsigned long long tex;
-    __device__ __forceinline__ void operator()(int px, int pyr, float r0[4], float r1[4]) const {
-        const float4 gc = gather_layer(tex, px - 1, pyr, 0), gd = gather_layer(tex, px + 1, pyr, 0);
-        r0[0] = gc.w, r0[1] = gc.z, r0[2] = gd.w, r0[3] = gd.z;
-        r1[0] = gc.x, r1[1] = gc.y, r1[2] = gd.x, r1[3] = gd.y;
-    }
-};
+// Fetchers of one correction row, pyr, at columns px-1 .. px+2.
 // From the correction array through the read-only path (written by an
 // earlier launch).
 struct BpRowsLdg {
     const float *corr;
     int W;
-    __device__ __forceinline__ void operator()(int px, int pyr, float r0[4], float r1[4]) const {
-        const float *c0 = corr + (size_t)pyr * W + (px - 1);
+    __device__ __forceinline__ void operator()(int px, int pyr, float r[4]) const {
+        const float *c = corr + (size_t)pyr * W + (px - 1);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) r0[a] = __ldg(c0 + a), r1[a] = __ldg(c0 + W + a);
+        for (int a = 0; a < 4; ++a) r[a] = __ldg(c + a);
     }
 };
 // From the correction array with plain loads (written by the same launch).
 struct BpRowsLoad {
     const float *corr;
     int W;
-    __device__ __forceinline__ void operator()(int px, int pyr, float r0[4], float r1[4]) const {
-        const float *c0 = corr + (size_t)pyr * W + (px - 1);
+    __device__ __forceinline__ void operator()(int px, int pyr, float r[4]) const {
+        const float *c = corr + (size_t)pyr * W + (px - 1);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) r0[a] = ld_stored(c0 + a), r1[a] = ld_stored(c0 + W + a);
+        for (int a = 0; a < 4; ++a) r[a] = ld_stored(c + a);
     }
 };
 
@@ -204,29 +214,30 @@ __device__ __forceinline__ void bp_voxel_at(const GeomDev &g, const ViewRec &v, 
                                             int x, int y, int z, float alpha, float gmax) {
     const float fx = (float)x, fy = (float)y, fz = (float)z;
     const float ndepth = -bp_cam(v, 2, fx, fy, fz);
-    const float upx = bp_pixel(g.cx, bp_cam(v, 0, fx, fy, fz), ndepth, g.sdd_ds);
-    const float upy = bp_pixel(g.cy, bp_cam(v, 1, fx, fy, fz), ndepth, g.sdd_ds);
-    if (!(upx >= 2.0f && upx < (float)(g.W - 2) && upy >= 2.0f && upy < (float)(g.H - 2))) return;
-    const int px = (int)upx, py = (int)upy;
-    float wx[4], wy[4], tap[4][4], r0[4], r1[4], r2[4], r3[4];
+    const float scale = bp_scale(g, ndepth), camx = bp_cam(v, 0, fx, fy, fz), camy = bp_cam(v, 1, fx, fy, fz);
+    const float upx = bp_coord(g.cx, camx, scale), upy = bp_coord(g.cy, camy, scale);
+    if (!bp_inside(g, upx, g.cx, camx, ndepth, g.W) || !bp_inside(g, upy, g.cy, camy, ndepth, g.H)) return;
+    const int px = bp_tap(upx, g.W), py = bp_tap(upy, g.H);
+    float wx[4], wy[4], s[4];
     bp_weights(upx - (float)px, wx);
     bp_weights(upy - (float)py, wy);
-    rows(px, py - 1, r0, r1);
-    rows(px, py + 1, r2, r3);
 #pragma unroll
-    for (int a = 0; a < 4; ++a) tap[a][0] = r0[a], tap[a][1] = r1[a], tap[a][2] = r2[a], tap[a][3] = r3[a];
-    bp_update(vol, x + (size_t)y * g.nx + (size_t)z * g.nx * g.ny, alpha, bp_sum(tap, wx, wy), gmax);
+    for (int b = 0; b < 4; ++b) {
+        float r[4];
+        rows(px, py - 1 + b, r);
+        s[b] = bp_row(r, wx);
+    }
+    bp_update(vol, x + (size_t)y * g.nx + (size_t)z * g.nx * g.ny, alpha, bp_sum(s, wy), bp_top(gmax));
 }
 
 // The column walk: voxels (x, y0 .. y0+K-1, z).  For a view whose matrix has
 // A[1] == A[7] == 0 (every rotation about y) the voxel's detector column and
 // depth do not depend on y: they are computed once (the y term of their sums
 // is an exact zero, so the values are the per-voxel ones).  The detector row
-// moves by about sdd/sid per voxel, and the 4x4 window's rows are kept in
-// registers: a step of s = 0, 1 or 2 rows reuses two of them and fetches the
-// two new ones.  Other views take the per-voxel form.
-// PF: first ask L2 for the column's voxels (prefetch.global.L2).
-template <int K, bool PF, typename Rows, typename T>
+// moves by about sdd/sid per voxel, and the window's four row sums are kept in
+// registers: a step of 0 to 3 rows reuses the overlap and forms the new ones.
+// Other views take the per-voxel form.
+template <int K, typename Rows, typename T>
 __device__ __forceinline__ void bp_column(const GeomDev &g, const ViewRec &v, const Rows &rows, T *__restrict__ vol,
                                           int x, int y0, int z, float alpha, float gmax) {
     const int y1 = min(y0 + K, g.ny);
@@ -236,45 +247,33 @@ __device__ __forceinline__ void bp_column(const GeomDev &g, const ViewRec &v, co
     }
     const float fx = (float)x, fz = (float)z;
     const float ndepth = -bp_cam(v, 2, fx, (float)y0, fz);
-    const float upx = bp_pixel(g.cx, bp_cam(v, 0, fx, (float)y0, fz), ndepth, g.sdd_ds);
-    if (!(upx >= 2.0f && upx < (float)(g.W - 2))) return;
-    const int px = (int)upx;
-    if (PF) {
-        const T *col = vol + x + (size_t)z * g.nx * g.ny;
-        for (int y = y0; y < y1; ++y) asm volatile("prefetch.global.L2 [%0];" ::"l"(col + (size_t)y * g.nx));
-    }
+    const float scale = bp_scale(g, ndepth), camx = bp_cam(v, 0, fx, (float)y0, fz), upx = bp_coord(g.cx, camx, scale);
+    if (!bp_inside(g, upx, g.cx, camx, ndepth, g.W)) return;
+    const int px = bp_tap(upx, g.W);
     float wx[4];
     bp_weights(upx - (float)px, wx);
-    float R[4][4];  // R[a][b]: column px-1+a, row pyc-1+b
+    float s[4];  // s[b]: the sum of row pyc-1+b
     int pyc = INT_MIN / 2;
     for (int y = y0; y < y1; ++y) {
-        const float upy = bp_pixel(g.cy, bp_cam(v, 1, fx, (float)y, fz), ndepth, g.sdd_ds);
-        if (!(upy >= 2.0f && upy < (float)(g.H - 2))) continue;
-        const int py = (int)upy;
+        const float camy = bp_cam(v, 1, fx, (float)y, fz), upy = bp_coord(g.cy, camy, scale);
+        if (!bp_inside(g, upy, g.cy, camy, ndepth, g.H)) continue;
+        const int py = bp_tap(upy, g.H);
         float wy[4];
         bp_weights(upy - (float)py, wy);
-        const int s = py - pyc;
-        float r0[4], r1[4];  // rows py-1, py
-        if (s >= 0 && s <= 2) {
+        int have = 0;  // rows kept
+        if (py >= pyc && py <= pyc + 3) {
+            have = 4 - (py - pyc);
+            for (int k = pyc; k < py; ++k) s[0] = s[1], s[1] = s[2], s[2] = s[3];
+        }
 #pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                r0[a] = s == 0 ? R[a][0] : (s == 1 ? R[a][1] : R[a][2]);
-                r1[a] = s == 0 ? R[a][1] : (s == 1 ? R[a][2] : R[a][3]);
+        for (int b = 0; b < 4; ++b)
+            if (b >= have) {
+                float r[4];
+                rows(px, py - 1 + b, r);
+                s[b] = bp_row(r, wx);
             }
-        } else {
-            rows(px, py - 1, r0, r1);
-        }
-        float r2[4], r3[4];  // rows py+1, py+2
-        rows(px, py + 1, r2, r3);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            R[a][0] = r0[a];
-            R[a][1] = r1[a];
-            R[a][2] = r2[a];
-            R[a][3] = r3[a];
-        }
         pyc = py;
-        bp_update(vol, x + (size_t)y * g.nx + (size_t)z * g.nx * g.ny, alpha, bp_sum(R, wx, wy), gmax);
+        bp_update(vol, x + (size_t)y * g.nx + (size_t)z * g.nx * g.ny, alpha, bp_sum(s, wy), bp_top(gmax));
     }
 }
 
