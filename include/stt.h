@@ -121,7 +121,8 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g);
  *                gathers of the FP32 volume bound as a pitch-linear 2D texture
  *                (the context keeps one texture object per array it is given,
  *                until stt_destroy; where the device's texture limits do not
- *                admit the array, the load-based variant of the same shape runs);
+ *                admit the array, the load-based variant of the same shape runs;
+ *                views of few rays share each ray between a block's warps);
  *   slab_variant the box the slab-staged projector stages with TMA;
  *   bp_variant   the column length of the voxel backprojection (0: by the
  *                geometry's magnification) and the blocks per SM;
@@ -136,7 +137,9 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g);
  * and caches the choice per device and geometry shape for later contexts.  It
  * synchronises `stream` and rewrites the context's view table, so call it
  * (and stt_set_tuning) while no launch of this context is in flight; launches
- * enqueued after it use the choice, and a solver uses the choice current when
+ * enqueued after it use the choice (a context that is not tuned gathers every
+ * view with tld4 where the volume binds, else uses load variant 0 and stages the
+ * classes from 25 degrees on), and a solver uses the choice current when
  * it is created (stt_solve_cfg.autotune runs the tuner then).  out (may be
  * NULL) receives the choice and the timings (microseconds per launch, 0 where
  * a variant was not timed).  stt_get_tuning reads the current choice;
@@ -162,8 +165,8 @@ stt_status stt_get_tuning(const stt_ctx *ctx, stt_tuning *out);
 stt_status stt_set_tuning(stt_ctx *ctx, const stt_tuning *t);
 /* Whether the tld4 gather variants (fp_variant 10, 11) bind `vol` on this
  * device: *ok = 1 when the device's limits on pitch-linear 2D textures admit
- * the volume (nx*ny texels a row, nz rows, its base aligned) and its z-fastest
- * copy; 0 when those variants run as their load-based forms for it. */
+ * the volume (nx*ny texels a row, nz rows, its base and its rows aligned); 0
+ * when those variants run as their load-based forms for it. */
 stt_status stt_fp_texture_ok(stt_ctx *ctx, const float *vol, int *ok);
 /* The same for a volume stored as `dtype` (STT_DTYPE_BF16: 16-bit texels,
  * the gather form fp_variant_bf16 1). */

@@ -6,11 +6,12 @@
 // warp is 32 consecutive detector columns of one row, so at every step its 32
 // samples lie along the detector's u axis in the volume.  For views whose rays
 // run mostly along z, u maps to the volume's x axis, which is contiguous in
-// memory; for views whose rays run mostly along x, u maps to z and the forward
-// projector gathers from a z-fastest transposed copy (ViewRec::layout), so
-// either way a warp's gathers touch few cache lines.  The volume is read
-// through the read-only path (ld.global.nc); at the headline sizes (256^3 fp32
-// = 64 MiB) it stays resident in the 126 MB L2.
+// memory; for views whose rays run mostly along x, u maps to z and the load
+// forms of the forward projector gather from a z-fastest transposed copy
+// (ViewRec::layout), so either way a warp's gathers touch few cache lines.  The
+// texture forms (two tld4 per sample) read the volume itself for every view.
+// The volume is read through the read-only path (ld.global.nc); at the headline
+// sizes (256^3 fp32 = 64 MiB) it stays resident in the 126 MB L2.
 #include "stt_internal.cuh"
 #include "stt_kernels.h"
 
@@ -33,20 +34,13 @@ __device__ __forceinline__ float fp_ray_sum_from(const GeomDev &g, const T *__re
         g, [=](int, const FpCell &c, float v[8]) { fp_corners<FAST, I>(src, st, c, v); }, r, count);
 }
 
-// The ray sum through the textures of FpTex: the transposed copy's for
-// layout-1 views when there is one, as fp_ray_sum reads the arrays.
+// The ray sum through the texture of FpTex.
 template <int G = FP_GROUP, bool PK = false, typename T = float>
-__device__ __forceinline__ float fp_ray_sum_tex(const GeomDev &g, const ViewRec &v, const FpTex &tex, const Ray &r) {
-    if (tex.z && v.layout == 1) {
-        const unsigned long long t = tex.z;
-        const int row = g.nz;
-        return fp_ray_sum_with<G, PK>(
-            g, [=](int, const FpCell &c, float w[8]) { fp_corners_tex<2, T>(t, row, c, w); }, r, nullptr);
-    }
+__device__ __forceinline__ float fp_ray_sum_tex(const GeomDev &g, const FpTex &tex, const Ray &r, int *count) {
     const unsigned long long t = tex.x;
-    const int row = g.nx;
+    const int nx = g.nx;
     return fp_ray_sum_with<G, PK>(
-        g, [=](int, const FpCell &c, float w[8]) { fp_corners_tex<0, T>(t, row, c, w); }, r, nullptr);
+        g, [=](int, const FpCell &c, float w[8]) { fp_corners_tex<T>(t, nx, c, w); }, r, count);
 }
 
 template <typename I, int G = FP_GROUP, bool PK = false, typename T>
@@ -71,20 +65,27 @@ __device__ __forceinline__ bool tile_pixel_t(const GeomDev &g, int &i, int &j) {
 // GenerateImage_MT (S/ImageFormationModel/TypicalRayProducer.core.h:168-224)
 // for views [view0, view0 + gridDim.z).  T = float, or unsigned short for a
 // BF16-stored volume (taps widened to FP32; the march and the sums are FP32).
-template <typename I, typename T>
+// TX: the tile, samples in flight and corners of gather variant 10.
+template <typename I, typename T, bool TX = false>
 __global__ void __launch_bounds__(128) k_fp(const GeomDev g, const ViewRec *__restrict__ views,
                                             const T *__restrict__ vol, const T *__restrict__ vol_t,
                                             int view0, float *__restrict__ proj, float *__restrict__ raylen,
-                                            float *__restrict__ weight) {
+                                            float *__restrict__ weight, const FpTex tex) {
     int i, j;
-    if (!tile_pixel(g, i, j)) return;
+    if (!tile_pixel_t<TX ? 8 : 32, 4>(g, i, j)) return;
     const int v = blockIdx.z;
     const ViewRec &vr = views[view0 + v];
     Ray r;
     make_ray(g, vr, i, j, r);
     int count = 0;
     const bool hit = r.tnear < r.tfar;
-    const float sum = hit ? fp_ray_sum<I>(g, vr, vol, vol_t, r, &count) : 0.0f;
+    float sum = 0.0f;
+    if (hit) {
+        if constexpr (TX)
+            sum = fp_ray_sum_tex<8, true, T>(g, tex, r, &count);
+        else
+            sum = fp_ray_sum<I>(g, vr, vol, vol_t, r, &count);
+    }
     const size_t o = (size_t)v * g.W * g.H + i + (size_t)j * g.W;
     proj[o] = sum;
     if (raylen && hit) raylen[o] = r.tfar - r.tnear;
@@ -103,8 +104,8 @@ __global__ void __launch_bounds__(128) k_fp(const GeomDev g, const ViewRec *__re
 // never a ray's arithmetic.
 // T, B: the storage of the volume and of the sinogram stack (float, or BF16
 // bits widened exactly to FP32).
-// TX: the corners come from the textures of `tex` (FP32 volumes below 2^31
-// voxels), not from vol and vol_t.
+// TX: the corners come from the texture of `tex` (volumes below 2^31 voxels),
+// not from vol and vol_t.
 template <typename I, int WX = 32, int NW = 4, int G = FP_GROUP, bool PK = false, typename T = float,
           typename B = float, bool TX = false>
 __global__ void __launch_bounds__(32 * NW) k_fp_corr(const GeomDev g, const ViewRec *__restrict__ views,
@@ -126,7 +127,7 @@ __global__ void __launch_bounds__(32 * NW) k_fp_corr(const GeomDev g, const View
     float L, sum = 0.0f;
     if (r.tnear < r.tfar) {
         if constexpr (TX)
-            sum = fp_ray_sum_tex<G, PK, T>(g, vr, tex, r);
+            sum = fp_ray_sum_tex<G, PK, T>(g, tex, r, nullptr);
         else
             sum = fp_ray_sum<I, G, PK>(g, vr, vol, vol_t, r, nullptr);
         L = r.tfar - r.tnear;
@@ -301,9 +302,11 @@ __global__ void __launch_bounds__(256) k_transpose_xz(int nx, int ny, int nz, co
 template <typename T>
 __global__ void __launch_bounds__(256) k_transpose_for_view(int nx, int ny, int nz,
                                                             const ViewRec *__restrict__ views, const ViewSel sel,
-                                                            const T *__restrict__ in, T *__restrict__ out) {
+                                                            const T *__restrict__ in, T *__restrict__ out,
+                                                            bool staged_only) {
     int local;
-    if (views[sel_view(sel, local)].layout != 1) return;
+    const ViewRec &v = views[sel_view(sel, local)];
+    if (v.layout != 1 || (staged_only && !view_staged<T>(v))) return;
     transpose_tile(nx, ny, nz, in, out);
 }
 
@@ -372,7 +375,7 @@ __global__ void __launch_bounds__(128) k_gather_ceiling(const GeomDev g, const V
 #pragma unroll
             for (int s = 0; s < G; ++s) {
                 if constexpr (TX)
-                    fp_corners_tex<FAST>(tex, FAST ? g.nz : g.nx, c[s], v[s]);
+                    fp_corners_tex(tex, g.nx, c[s], v[s]);
                 else
                     fp_corners<FAST, int>(src, st, c[s], v[s]);
             }
@@ -393,7 +396,7 @@ __global__ void __launch_bounds__(128) k_gather_ceiling(const GeomDev g, const V
             fp_cell(g, p, c);
             float v[8];
             if constexpr (TX)
-                fp_corners_tex<FAST>(tex, FAST ? g.nz : g.nx, c, v);
+                fp_corners_tex(tex, g.nx, c, v);
             else
                 fp_corners<FAST, int>(src, st, c, v);
             sum = __fadd_rn(sum, trilerp(v, c));
@@ -433,13 +436,34 @@ int grid_stride_blocks(long long n, int threads) {
     return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
 
-cudaError_t launch_fp(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t, int view0,
-                      int nviews, float *proj, float *raylen, float *weight, cudaStream_t s) {
-    if (small_volume(g))
-        k_fp<int, float><<<ray_grid(g, nviews), 128, 0, s>>>(g, views, vol, vol_t, view0, proj, raylen, weight);
-    else
-        k_fp<long long, float><<<ray_grid(g, nviews), 128, 0, s>>>(g, views, vol, vol_t, view0, proj, raylen, weight);
+namespace {
+template <typename T>
+cudaError_t fp_any(const GeomDev &g, const ViewRec *views, const T *vol, const T *vol_t, int view0, int nviews,
+                   float *proj, float *raylen, float *weight, cudaStream_t s, const FpTex *tex) {
+    if (tex && tex->ok && tex->esize == (int)sizeof(T) && small_volume(g)) {
+        if ((long long)g.W * g.H * nviews <= FP_SPLIT_RAYS)
+            return launch_fp_split(g, views, view0, nviews, proj, raylen, weight, s, *tex);
+        k_fp<int, T, true><<<dim3((g.W + 7) / 8, (g.H + 15) / 16, nviews), 128, 0, s>>>(g, views, vol, vol_t, view0, proj,
+                                                                                      raylen, weight, *tex);
+    } else if (small_volume(g)) {
+        k_fp<int, T><<<ray_grid(g, nviews), 128, 0, s>>>(g, views, vol, vol_t, view0, proj, raylen, weight, FpTex{});
+    } else {
+        k_fp<long long, T><<<ray_grid(g, nviews), 128, 0, s>>>(g, views, vol, vol_t, view0, proj, raylen, weight,
+                                                                FpTex{});
+    }
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_fp(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t, int view0,
+                      int nviews, float *proj, float *raylen, float *weight, cudaStream_t s, const FpTex *tex) {
+    return fp_any(g, views, vol, vol_t, view0, nviews, proj, raylen, weight, s, tex);
+}
+
+cudaError_t launch_fp(const GeomDev &g, const ViewRec *views, const unsigned short *vol, const unsigned short *vol_t,
+                      int view0, int nviews, float *proj, float *raylen, float *weight, cudaStream_t s,
+                      const FpTex *tex) {
+    return fp_any(g, views, vol, vol_t, view0, nviews, proj, raylen, weight, s, tex);
 }
 
 namespace {
@@ -542,44 +566,28 @@ const char *fp16_variant_name(int v) {
 
 namespace {
 template <typename T>
-bool make_fp_tex_any(const GeomDev &g, const T *vol, const T *vol_t, FpTex &t) {
+bool make_fp_tex_any(const GeomDev &g, const T *vol, FpTex &t) {
     t = FpTex{};
     TexLimits l;
     if (!small_volume(g) || !tex_limits(l)) return false;
-    const unsigned long long x = slices_texture(l, vol, (long long)g.nx * g.ny, g.nz);
-    if (!x) return false;
-    unsigned long long z = 0;
-    if (vol_t && !(z = slices_texture(l, vol_t, (long long)g.nz * g.ny, g.nx))) {
-        cudaDestroyTextureObject((cudaTextureObject_t)x);
-        return false;
-    }
-    t.x = x;
-    t.z = z;
-    t.ok = 1;
+    t.x = slices_texture(l, vol, (long long)g.nx * g.ny, g.nz);
+    t.ok = t.x != 0;
     t.esize = (int)sizeof(T);
-    return true;
+    return t.ok != 0;
 }
 }  // namespace
 
-bool make_fp_tex(const GeomDev &g, const float *vol, const float *vol_t, FpTex &t) {
-    return make_fp_tex_any(g, vol, vol_t, t);
-}
+bool make_fp_tex(const GeomDev &g, const float *vol, FpTex &t) { return make_fp_tex_any(g, vol, t); }
 
-bool make_fp_tex(const GeomDev &g, const unsigned short *vol, const unsigned short *vol_t, FpTex &t) {
-    return make_fp_tex_any(g, vol, vol_t, t);
-}
+bool make_fp_tex(const GeomDev &g, const unsigned short *vol, FpTex &t) { return make_fp_tex_any(g, vol, t); }
 
 bool fp_tex_fits(const GeomDev &g, const void *vol, int esize) {
     TexLimits l;
-    if (!small_volume(g) || !tex_limits(l)) return false;
-    const void *aligned = reinterpret_cast<const void *>((uintptr_t)(l.base_align > 0 ? l.base_align : 256));
-    return slices_fit(l, vol, (long long)g.nx * g.ny, g.nz, esize) &&
-           slices_fit(l, aligned, (long long)g.nz * g.ny, g.nx, esize);
+    return small_volume(g) && tex_limits(l) && slices_fit(l, vol, (long long)g.nx * g.ny, g.nz, esize);
 }
 
 void destroy_fp_tex(FpTex &t) {
     if (t.x) cudaDestroyTextureObject((cudaTextureObject_t)t.x);
-    if (t.z) cudaDestroyTextureObject((cudaTextureObject_t)t.z);
     t = FpTex{};
 }
 
@@ -588,12 +596,9 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *
                            cudaStream_t s, const FpSlabMaps *maps, int *status,
                            int fp_variant, const FpTex *tex) {
     const int skip = maps && maps->ok && maps->esize == 4 && (!vol_t || maps->has_z);
-    // a texture variant whose textures are missing, or do not cover vol_t,
-    // runs the load-based variant of the same shape
-    if (is_tex_fp_variant(fp_variant) && !(tex && tex->ok && tex->esize == 4 && (!vol_t || tex->z)))
-        fp_variant = fp_variant == 10 ? 4 : 8;
-    FpTex tx = tex ? *tex : FpTex{};
-    if (!vol_t) tx.z = 0;  // without the copy every view reads the volume, as the loads do
+    // a texture variant without a usable texture runs the load-based variant of the same shape
+    if (is_tex_fp_variant(fp_variant) && !(tex && tex->ok && tex->esize == 4)) fp_variant = fp_variant == 10 ? 4 : 8;
+    const FpTex tx = tex ? *tex : FpTex{};
     if (skip) {
         cudaError_t e = launch_fp_corr_slab(g, views, *maps, vol, vol_t, sel, b_stack, raylen_state, corr, s,
                                             status);
@@ -604,6 +609,8 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *
                                                             skip, FpTex{});
         return cudaGetLastError();
     }
+    if (is_tex_fp_variant(fp_variant) && (long long)g.W * g.H <= FP_SPLIT_RAYS)
+        return launch_fp_corr_split(g, views, sel, b_stack, raylen_state, corr, s, tx, skip);
     switch (fp_variant) {
     case 1: fp_corr_variant<32, 2, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
     case 2: fp_corr_variant<32, 8, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
@@ -632,32 +639,23 @@ cudaError_t launch_transpose(const GeomDev &g, const float *in, float *out, cuda
     return cudaGetLastError();
 }
 
-cudaError_t launch_fp_bf16(const GeomDev &g, const ViewRec *views, const unsigned short *vol,
-                           const unsigned short *vol_t, int view0, int nviews, float *proj, float *raylen,
-                           float *weight, cudaStream_t s) {
-    if (small_volume(g))
-        k_fp<int, unsigned short><<<ray_grid(g, nviews), 128, 0, s>>>(g, views, vol, vol_t, view0, proj, raylen, weight);
-    else
-        k_fp<long long, unsigned short><<<ray_grid(g, nviews), 128, 0, s>>>(g, views, vol, vol_t, view0, proj, raylen,
-                                                                            weight);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_transpose_bf16(const GeomDev &g, const unsigned short *in, unsigned short *out, cudaStream_t s) {
     k_transpose_xz<unsigned short><<<transpose_grid(g), dim3(32, 8), 0, s>>>(g.nx, g.ny, g.nz, in, out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_transpose_for_view(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *in,
-                                      float *out, cudaStream_t s) {
-    k_transpose_for_view<float><<<transpose_grid(g), dim3(32, 8), 0, s>>>(g.nx, g.ny, g.nz, views, sel, in, out);
+                                      float *out, cudaStream_t s, bool staged_only) {
+    k_transpose_for_view<float><<<transpose_grid(g), dim3(32, 8), 0, s>>>(g.nx, g.ny, g.nz, views, sel, in, out,
+                                                                         staged_only);
     return cudaGetLastError();
 }
 
 cudaError_t launch_transpose_for_view(const GeomDev &g, const ViewRec *views, const ViewSel &sel,
-                                      const unsigned short *in, unsigned short *out, cudaStream_t s) {
+                                      const unsigned short *in, unsigned short *out, cudaStream_t s,
+                                      bool staged_only) {
     k_transpose_for_view<unsigned short><<<transpose_grid(g), dim3(32, 8), 0, s>>>(g.nx, g.ny, g.nz, views, sel, in,
-                                                                                  out);
+                                                                                  out, staged_only);
     return cudaGetLastError();
 }
 
@@ -684,9 +682,10 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigne
                                             status);
         if (e != cudaSuccess) return e;
     }
-    if (fp_variant16 == 1 && tex && tex->ok && tex->esize == 2 && (!vol_t || tex->z) && small_volume(g)) {
-        FpTex tx = *tex;
-        if (!vol_t) tx.z = 0;
+    if (fp_variant16 == 1 && tex && tex->ok && tex->esize == 2 && small_volume(g)) {
+        const FpTex tx = *tex;
+        if ((long long)g.W * g.H <= FP_SPLIT_RAYS)
+            return launch_fp_corr_split(g, views, sel, b_stack, raylen_state, corr, s, tx, skip);
         constexpr int WX = 8, NW = 4, TH = (32 / WX) * NW;
         k_fp_corr<int, WX, NW, 8, true, U, U, true><<<dim3((g.W + WX - 1) / WX, (g.H + TH - 1) / TH, 1), 32 * NW, 0, s>>>(
             g, views, vol, vol_t, sel, b_stack, raylen_state, corr, skip, tx);
@@ -755,14 +754,13 @@ cudaError_t launch_gather_ceiling(const GeomDev &g, const ViewRec *views, const 
                                   const float *vol, const float *vol_t, int packed, float *out, int *count,
                                   cudaStream_t s, const FpTex *tex) {
     if (!small_volume(g)) return cudaErrorInvalidValue;
-    const bool zf = vol_t && host_view.layout == 1;
-    const float *src = zf ? vol_t : vol;
     if (tex) {  // packed pairs, tld4 corners
-        if (!tex->ok || (zf && !tex->z)) return cudaErrorInvalidValue;
-        if (zf) k_gather_ceiling<2, true, true><<<ray_grid(g, 1), 128, 0, s>>>(g, views, view, src, tex->z, out, count);
-        else k_gather_ceiling<0, true, true><<<ray_grid(g, 1), 128, 0, s>>>(g, views, view, src, tex->x, out, count);
+        if (!tex->ok) return cudaErrorInvalidValue;
+        k_gather_ceiling<0, true, true><<<ray_grid(g, 1), 128, 0, s>>>(g, views, view, vol, tex->x, out, count);
         return cudaGetLastError();
     }
+    const bool zf = vol_t && host_view.layout == 1;
+    const float *src = zf ? vol_t : vol;
     if (zf && packed) k_gather_ceiling<2, true><<<ray_grid(g, 1), 128, 0, s>>>(g, views, view, src, 0, out, count);
     else if (zf) k_gather_ceiling<2, false><<<ray_grid(g, 1), 128, 0, s>>>(g, views, view, src, 0, out, count);
     else if (packed) k_gather_ceiling<0, true><<<ray_grid(g, 1), 128, 0, s>>>(g, views, view, src, 0, out, count);

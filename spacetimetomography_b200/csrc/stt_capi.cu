@@ -287,18 +287,10 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g) {
     return STT_OK;
 }
 
-// When a view in [view0, view0+nviews) gathers from the z-fastest copy,
-// refresh the context's copy of `vol` and return it in *volt.
 }  // extern "C"
 
-// The z-fastest copy of the volume when a view in [view0, view0 + nviews)
-// gathers along x (FP32 and BF16 storage).
-static stt_status transposed_if_needed(stt_ctx *ctx, const float *vol, int view0, int nviews, cudaStream_t s,
-                                       const float **volt) {
-    *volt = nullptr;
-    bool any = false;
-    for (int v = view0; v < view0 + nviews && !any; ++v) any = ctx->views_h[v].layout == 1;
-    if (!any) return STT_OK;
+// The context's z-fastest copy of `vol`, refreshed (FP32 and BF16 storage).
+static stt_status make_copy(stt_ctx *ctx, const float *vol, cudaStream_t s, const float **volt) {
     stt_status st = ensure(ctx, ctx->volt, ctx->volt_n, (size_t)nvox(ctx), "transposed volume");
     if (st) return st;
     STT_CUDA(ctx, stt::launch_transpose(ctx->g, vol, ctx->volt, s), "k_transpose launch");
@@ -306,12 +298,7 @@ static stt_status transposed_if_needed(stt_ctx *ctx, const float *vol, int view0
     return STT_OK;
 }
 
-static stt_status transposed_if_needed(stt_ctx *ctx, const unsigned short *vol, int view0, int nviews,
-                                       cudaStream_t s, const unsigned short **volt) {
-    *volt = nullptr;
-    bool any = false;
-    for (int v = view0; v < view0 + nviews && !any; ++v) any = ctx->views_h[v].layout == 1;
-    if (!any) return STT_OK;
+static stt_status make_copy(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s, const unsigned short **volt) {
     stt_status st = ensure(ctx, ctx->volt16, ctx->volt16_n, (size_t)nvox(ctx), "transposed BF16 volume");
     if (st) return st;
     STT_CUDA(ctx, stt::launch_transpose_bf16(ctx->g, vol, ctx->volt16, s), "k_transpose launch");
@@ -319,9 +306,15 @@ static stt_status transposed_if_needed(stt_ctx *ctx, const unsigned short *vol, 
     return STT_OK;
 }
 
-// The staged-class mask for a volume of this storage (0: no view is staged).
-static unsigned staged_mask(const stt_ctx *ctx, const float *) { return ctx->staged_bins; }
-static unsigned staged_mask(const stt_ctx *ctx, const unsigned short *) { return ctx->staged_bins16; }
+// The copy when a view in [view0, view0 + nviews) gathers along x.
+template <typename T>
+static stt_status transposed_if_needed(stt_ctx *ctx, const T *vol, int view0, int nviews, cudaStream_t s,
+                                       const T **volt) {
+    *volt = nullptr;
+    for (int v = view0; v < view0 + nviews; ++v)
+        if (ctx->views_h[v].layout == 1) return make_copy(ctx, vol, s, volt);
+    return STT_OK;
+}
 
 extern "C" {
 
@@ -331,45 +324,61 @@ static stt_status check_views(stt_ctx *ctx, int view0, int nviews) {
     return STT_OK;
 }
 
-stt_status stt_fp(stt_ctx *ctx, const float *vol, float *proj, float *raylen, float *weight,
-                  int view0, int nviews, void *stream) {
-    stt_status st = need_geom(ctx);
+}  // extern "C"
+
+// Projections of [view0, view0 + nviews): corners from the volume's texture
+// where it binds (no copy), else by loads.
+template <typename T>
+static stt_status project(stt_ctx *ctx, const T *vol, float *proj, float *raylen, float *weight, int view0, int nviews,
+                          cudaStream_t s) {
+    const stt::FpTex *tex = stt::ctx_fp_tex(ctx, vol);
+    const T *volt = nullptr;
+    stt_status st = tex ? STT_OK : transposed_if_needed(ctx, vol, view0, nviews, s, &volt);
     if (st) return st;
-    if (!vol || !proj) return fail(ctx, STT_ERR_INVALID, "null vol or proj");
-    if ((st = check_views(ctx, view0, nviews))) return st;
-    if (nviews == 0) return STT_OK;
-    if ((st = set_device(ctx))) return st;
-    const float *volt = nullptr;
-    if ((st = transposed_if_needed(ctx, vol, view0, nviews, S(stream), &volt))) return st;
-    STT_CUDA(ctx, stt::launch_fp(ctx->g, ctx->views_d, vol, volt, view0, nviews, proj, raylen, weight, S(stream)),
+    STT_CUDA(ctx, stt::launch_fp(ctx->g, ctx->views_d, vol, volt, view0, nviews, proj, raylen, weight, s, tex),
              "k_fp launch");
     return STT_OK;
 }
 
+// The fused forward projection and correction of one view: the gather form of
+// the context's choice and, where its maps apply, the slab-staged kernel.
+template <typename T>
+static stt_status project_corr(stt_ctx *ctx, const T *vol, const stt::ViewSel &sel, const T *stack, float *raylen,
+                               float *corr, cudaStream_t s) {
+    const stt::FpTex *tex = stt::ctx_fp_tex(ctx, vol);
+    const stt::FpChoice c = stt::fp_choice(ctx, vol, tex != nullptr);
+    const stt::ViewRec &v = ctx->views_h[sel.view];
+    const T *volt = nullptr;
+    if (stt::fp_needs_copy(c, v, (sizeof(T) == 2 ? v.staged16 : v.staged) != 0))
+        if (stt_status st = make_copy(ctx, vol, s, &volt)) return st;
+    stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
+    if (c.stage) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
+    STT_CUDA(ctx, stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, raylen, corr, s, &maps, ctx->status,
+                                      c.variant, c.tex ? tex : nullptr),
+             "k_fp_corr launch");
+    return STT_OK;
+}
+
+extern "C" {
+
+stt_status stt_fp(stt_ctx *ctx, const float *vol, float *proj, float *raylen, float *weight,
+                  int view0, int nviews, void *stream) {
+    return stt_fp_typed(ctx, vol, STT_DTYPE_F32, proj, raylen, weight, view0, nviews, stream);
+}
+
 stt_status stt_fp_typed(stt_ctx *ctx, const void *vol, int dtype, float *proj, float *raylen, float *weight,
                         int view0, int nviews, void *stream) {
-    if (dtype == STT_DTYPE_F32)
-        return stt_fp(ctx, static_cast<const float *>(vol), proj, raylen, weight, view0, nviews, stream);
     stt_status st = need_geom(ctx);
     if (st) return st;
-    if (dtype != STT_DTYPE_BF16) return fail(ctx, STT_ERR_INVALID, "dtype must be STT_DTYPE_F32 or STT_DTYPE_BF16");
+    if (dtype != STT_DTYPE_F32 && dtype != STT_DTYPE_BF16)
+        return fail(ctx, STT_ERR_INVALID, "dtype must be STT_DTYPE_F32 or STT_DTYPE_BF16");
     if (!vol || !proj) return fail(ctx, STT_ERR_INVALID, "null vol or proj");
     if ((st = check_views(ctx, view0, nviews))) return st;
     if (nviews == 0) return STT_OK;
     if ((st = set_device(ctx))) return st;
-    const unsigned short *v16 = static_cast<const unsigned short *>(vol);
-    const unsigned short *vt16 = nullptr;
-    bool any = false;
-    for (int v = view0; v < view0 + nviews && !any; ++v) any = ctx->views_h[v].layout == 1;
-    if (any) {
-        if ((st = ensure(ctx, ctx->volt16, ctx->volt16_n, (size_t)nvox(ctx), "transposed BF16 volume"))) return st;
-        STT_CUDA(ctx, stt::launch_transpose_bf16(ctx->g, v16, ctx->volt16, S(stream)), "k_transpose launch");
-        vt16 = ctx->volt16;
-    }
-    STT_CUDA(ctx, stt::launch_fp_bf16(ctx->g, ctx->views_d, v16, vt16, view0, nviews, proj, raylen, weight,
-                                      S(stream)),
-             "k_fp launch");
-    return STT_OK;
+    if (dtype == STT_DTYPE_F32)
+        return project(ctx, static_cast<const float *>(vol), proj, raylen, weight, view0, nviews, S(stream));
+    return project(ctx, static_cast<const unsigned short *>(vol), proj, raylen, weight, view0, nviews, S(stream));
 }
 
 stt_status stt_fp_correction(stt_ctx *ctx, const float *vol, const float *b, float *raylen_state,
@@ -379,15 +388,7 @@ stt_status stt_fp_correction(stt_ctx *ctx, const float *vol, const float *b, flo
     if (!vol || !b || !corr) return fail(ctx, STT_ERR_INVALID, "null vol, b or corr");
     if ((st = check_views(ctx, view, 1))) return st;
     if ((st = set_device(ctx))) return st;
-    const stt::ViewSel sel{view, nullptr, 0, view};
-    const float *volt = nullptr;
-    if ((st = transposed_if_needed(ctx, vol, view, 1, S(stream), &volt))) return st;
-    stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
-    if (staged_mask(ctx, vol)) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
-    STT_CUDA(ctx, stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, b, raylen_state, corr, S(stream), &maps,
-                                      ctx->status, ctx->tuning.fp, stt::ctx_fp_tex(ctx, vol, volt)),
-             "k_fp_corr launch");
-    return STT_OK;
+    return project_corr(ctx, vol, stt::ViewSel{view, nullptr, 0, view}, b, raylen_state, corr, S(stream));
 }
 
 stt_status stt_fp_texture_ok_typed(stt_ctx *ctx, const void *vol, int dtype, int *ok) {
@@ -414,12 +415,13 @@ stt_status stt_gather_ceiling(stt_ctx *ctx, const float *vol, int view, int pack
         return fail(ctx, STT_ERR_UNSUPPORTED, "the gather ceiling takes volumes below 2^31 voxels");
     if ((st = set_device(ctx))) return st;
     const float *volt = nullptr;
-    if ((st = transposed_if_needed(ctx, vol, view, 1, S(stream), &volt))) return st;
     const stt::FpTex *tex = nullptr;
     if (packed & 2) {  // tld4 corners
-        tex = stt::ctx_fp_tex_any(ctx, vol, volt);
-        if (!tex || !tex->ok)
+        tex = stt::ctx_fp_tex(ctx, vol);
+        if (!tex)
             return fail(ctx, STT_ERR_UNSUPPORTED, "the device's texture limits do not admit this volume");
+    } else if ((st = transposed_if_needed(ctx, vol, view, 1, S(stream), &volt))) {
+        return st;
     }
     STT_CUDA(ctx, stt::launch_gather_ceiling(ctx->g, ctx->views_d, ctx->views_h[view], view, vol, volt, packed & 1, out,
                                              count, S(stream), tex),
@@ -529,25 +531,6 @@ stt_status stt_bp_ray_scatter(stt_ctx *ctx, const float *corr, float *contrib, f
 
 }  // extern "C"
 
-// The fused forward projection of one view of a sweep: FP32 through the tuned
-// gather variant and, where its maps apply, the slab-staged kernel; BF16
-// through the gather kernel and the slab kernel's BF16 boxes.
-static cudaError_t sweep_fp_corr(stt_ctx *ctx, const float *vol, const float *volt, const stt::ViewSel &sel,
-                                 const float *stack, float *rl, cudaStream_t s) {
-    stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
-    if (staged_mask(ctx, vol)) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
-    return stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, rl, ctx->corr, s, &maps,
-                               ctx->status, ctx->tuning.fp, stt::ctx_fp_tex(ctx, vol, volt));
-}
-
-static cudaError_t sweep_fp_corr(stt_ctx *ctx, const unsigned short *vol, const unsigned short *volt,
-                                 const stt::ViewSel &sel, const unsigned short *stack, float *rl, cudaStream_t s) {
-    stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
-    if (staged_mask(ctx, vol)) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
-    return stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, rl, ctx->corr, s, &maps,
-                               ctx->status, ctx->tuning.fp16, stt::ctx_fp_tex(ctx, vol, volt));
-}
-
 template <typename T>
 static stt_status sart_sweep_t(stt_ctx *ctx, T *vol, const T *proj_stack, const int *perm, int nperm,
                                int view_offset, double alpha, float gmax, int bp_mode, float *raylen_state,
@@ -596,12 +579,11 @@ static stt_status sart_sweep_t(stt_ctx *ctx, T *vol, const T *proj_stack, const 
     if (bp_mode == 1 && (st = ensure_acc(ctx, s))) return st;
     for (int i = 0; i < nperm; ++i) {
         const stt::ViewSel sel{view_offset + perm[i], nullptr, 0, view_offset};
-        const T *volt = nullptr;
-        if ((st = transposed_if_needed(ctx, vol, view_offset + perm[i], 1, s, &volt))) return st;
         // ray-based mode: TypicalRayProducer::Initial zeroes the ray lengths
         // after every view, so missed rays see L = 0 (no sticky state)
-        STT_CUDA(ctx, sweep_fp_corr(ctx, vol, volt, sel, proj_stack, bp_mode == 0 ? raylen_state : nullptr, s),
-                 "k_fp_corr launch");
+        if ((st = project_corr(ctx, static_cast<const T *>(vol), sel, proj_stack, bp_mode == 0 ? raylen_state : nullptr,
+                               ctx->corr, s)))
+            return st;
         if (bp_mode == 0)
             STT_CUDA(ctx, stt::launch_bp_voxel(ctx->g, ctx->views_d, sel, ctx->corr, vol, (float)alpha, gmax, s,
                                                ctx->tuning.bp),

@@ -43,13 +43,12 @@ struct stt_ctx {
     unsigned staged_bins16 = 0x1E0u;  // the same for a BF16-stored volume (ViewRec::staged16)
     bool tuned = false;
     stt_tuning report{};
-    // Texture objects of the tld4 gather variants for the arrays the entry
-    // points were given, keyed by the arrays and the dimensions (at most
-    // kFpTexCache; past that the load-based variant of the same shape runs).
-    // Kept until stt_destroy, so a stream capture of an entry point that
-    // bound one stays valid.
+    // Texture objects of the tld4 gather forms for the arrays the entry points
+    // were given, keyed by the array and the dimensions (at most kFpTexCache;
+    // past that the load-based forms run).  Kept until stt_destroy, so a stream
+    // capture of an entry point that bound one stays valid.
     struct FpTexEntry {
-        const void *vol, *volt;
+        const void *vol;
         int nx, ny, nz, esize;
         stt::FpTex tex;
     };
@@ -65,11 +64,22 @@ inline int off_axis_bin(float deg) {
 }
 // Applies ctx->staged_bins and staged_bins16 to every view (host and device tables).
 stt_status apply_staged_bins(stt_ctx *ctx);
-// The textures of the tuned gather variant for (vol, vol_t) when it is a tld4
-// variant (created on first use, cached in the context); nullptr otherwise.
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol, const float *vol_t);
-// The same whatever the tuned variant (nullptr only when the cache is full).
-const FpTex *ctx_fp_tex_any(stt_ctx *ctx, const float *vol, const float *vol_t);
-// The BF16 volume's textures when the tuned BF16 gather form is the tld4 one.
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, const unsigned short *vol_t);
+// The texture of `vol` (created on first use, cached in the context), whatever
+// the tuned variant; nullptr where it does not bind or the cache is full.
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol);
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol);
+// How the correction projector runs on volumes of one storage: a tuned context's
+// choices; untuned, tld4 corners and no view staged where the textures bind
+// (FP_DEFAULT_TEX), else load variant 0 with the oblique views staged.
+struct FpChoice {
+    int variant;  // launch_fp_corr's fp_variant (FP32) or fp_variant16 (BF16)
+    bool tex;     // its corners come from the volume's texture
+    bool stage;   // some view class goes to the slab-staged projector
+};
+FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds);
+FpChoice fp_choice(const stt_ctx *ctx, const unsigned short *, bool tex_binds);
+// Whether a view gathers from the z-fastest copy under that choice.
+inline bool fp_needs_copy(const FpChoice &c, const ViewRec &v, bool staged) {
+    return v.layout == 1 && (!c.tex || (c.stage && staged));
+}
 }  // namespace stt

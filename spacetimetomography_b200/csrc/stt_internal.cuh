@@ -304,13 +304,11 @@ __device__ __forceinline__ void fp_corners(const T *src, const Strides &st, cons
 }
 
 // The same 8 corners through two tld4 gathers of a pitch-linear 2D texture
-// whose rows are the array's slices across its slowest axis: for the volume
-// (FAST 0) texel (x + nx*y, z); for the z-fastest copy (FAST 2) texel
-// (z + nz*y, x).  A gather at texel (u, v) returns {u, u+1} x {v, v+1} (.w =
-// (u, v), .z = (u+1, v), .x = (u, v+1), .y = (u+1, v+1)): the fast-axis pair
-// of two neighbouring slices; the second gather, one row of `row` texels on,
-// is the y+1 pair.  The cell's base is at most dims-2 on every axis, so no
-// gather leaves the array or crosses into another row of slices.
+// whose rows are the volume's z slices: texel (x + nx*y, z).  A gather at texel
+// (u, v) returns {u, u+1} x {v, v+1} (.w = (u, v), .z = (u+1, v), .x = (u, v+1),
+// .y = (u+1, v+1)): the x pair of two neighbouring slices; the second gather,
+// nx texels on, is the y+1 pair.  The cell's base is at most dims-2 on every
+// axis, so no gather leaves the array or crosses into another slice.
 // T: the texels' storage; BF16 (unsigned short bits, a 16-bit unsigned
 // texture) is widened exactly to FP32 as ld_voxel does.
 __device__ __forceinline__ float4 gather_texels(unsigned long long tex, float u, float v, const float *) {
@@ -322,19 +320,14 @@ __device__ __forceinline__ float4 gather_texels(unsigned long long tex, float u,
                        __uint_as_float((unsigned)r.z << 16), __uint_as_float((unsigned)r.w << 16));
 }
 
-template <int FAST, typename T = float>
-__device__ __forceinline__ void fp_corners_tex(unsigned long long tex, int row, const FpCell &c, float v[8]) {
-    const int u = FAST == 0 ? c.ix + row * c.iy : c.iz + row * c.iy;
-    const float fv = (float)(FAST == 0 ? c.iz : c.ix) + 1.0f;
+template <typename T = float>
+__device__ __forceinline__ void fp_corners_tex(unsigned long long tex, int nx, const FpCell &c, float v[8]) {
+    const int u = c.ix + nx * c.iy;
+    const float fv = (float)c.iz + 1.0f;
     const float4 a = gather_texels(tex, (float)u + 1.0f, fv, (const T *)nullptr);
-    const float4 b = gather_texels(tex, (float)(u + row) + 1.0f, fv, (const T *)nullptr);
-    if (FAST == 0) {  // u along x, v along z
-        v[0] = a.w, v[1] = a.z, v[4] = a.x, v[5] = a.y;
-        v[2] = b.w, v[3] = b.z, v[6] = b.x, v[7] = b.y;
-    } else {  // u along z, v along x
-        v[0] = a.w, v[4] = a.z, v[1] = a.x, v[5] = a.y;
-        v[2] = b.w, v[6] = b.z, v[3] = b.x, v[7] = b.y;
-    }
+    const float4 b = gather_texels(tex, (float)(u + nx) + 1.0f, fv, (const T *)nullptr);
+    v[0] = a.w, v[1] = a.z, v[4] = a.x, v[5] = a.y;
+    v[2] = b.w, v[3] = b.z, v[6] = b.x, v[7] = b.y;
 }
 
 template <int FAST, typename I, typename T>

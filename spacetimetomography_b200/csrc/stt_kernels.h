@@ -47,8 +47,13 @@ const char *ray_variant_name(int v);
 // 512^3 it is the faster form; at 256^3 and below the global scatter is).
 int default_ray_variant(const GeomDev &g);
 
+// The projection of nviews views: corners through the textures of `tex` where
+// it is usable (the same values), else by loads from vol, or from vol_t for
+// the views along x when it is given.
+struct FpTex;
 cudaError_t launch_fp(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t, int view0,
-                      int nviews, float *proj, float *raylen, float *weight, cudaStream_t s);
+                      int nviews, float *proj, float *raylen, float *weight, cudaStream_t s,
+                      const FpTex *tex = nullptr);
 // Slab-staged forward projector (k_fp_slab.cu) for the views marked `staged`:
 // the same outputs as the gather form bit for bit, the volume read through
 // TMA boxes.  The tensor maps cover the volume and its z-fastest copy (vol_t
@@ -77,30 +82,46 @@ cudaError_t launch_fp_corr_slab(const GeomDev &g, const ViewRec *views, const Fp
                                 const unsigned short *vol, const unsigned short *vol_t, const ViewSel &sel,
                                 const unsigned short *b_stack, float *raylen_state, float *corr, cudaStream_t s,
                                 int *status);
-// Texture objects of the gather variants that fetch corners with tld4: the
-// volume as a pitch-linear 2D texture whose rows are its z slices (width
-// nx*ny texels, nz rows) and its z-fastest copy likewise (rows the x slices;
-// z = 0 without a copy); FP32 texels, or for a BF16-stored volume 16-bit
-// unsigned texels holding its bits.  Point sampling returns stored values
-// exactly, so the samples are those of the loads they replace.
-// make_fp_tex returns false (and creates nothing) where the device's limits
-// on linear 2D textures do not admit the arrays: a row of more than the
-// maximum width or pitch, more rows than the maximum height, a base not
-// aligned to the texture alignment.  The caller owns the objects
-// (destroy_fp_tex).
+// Texture object of the gather forms that fetch corners with tld4: the volume
+// as a pitch-linear 2D texture whose rows are its z slices (width nx*ny texels,
+// nz rows); FP32 texels, or for a BF16-stored volume 16-bit unsigned texels
+// holding its bits.  Point sampling returns stored values exactly, so the
+// samples are those of the loads they replace.  A gather's footprint is two
+// texels of two slices whatever the ray's direction, so every view reads the
+// volume itself: no z-fastest copy.  make_fp_tex returns false (and creates
+// nothing) where the device's limits on linear 2D textures do not admit the
+// array: a row of more than the maximum width or pitch, more rows than the
+// maximum height, a base not aligned to the texture alignment.  The caller owns
+// the object (destroy_fp_tex).
 struct FpTex {
-    unsigned long long x = 0, z = 0;
+    unsigned long long x = 0;
     int ok = 0;
     int esize = 0;  // bytes per texel: 4 (FP32) or 2 (BF16)
 };
 bool is_tex_fp_variant(int fp_variant);
-bool make_fp_tex(const GeomDev &g, const float *vol, const float *vol_t, FpTex &t);
-bool make_fp_tex(const GeomDev &g, const unsigned short *vol, const unsigned short *vol_t, FpTex &t);
-// Whether make_fp_tex admits `vol` (esize bytes per voxel) and a z-fastest
-// copy at an aligned base on this device (checks the limits only; creates
-// nothing).
+bool make_fp_tex(const GeomDev &g, const float *vol, FpTex &t);
+bool make_fp_tex(const GeomDev &g, const unsigned short *vol, FpTex &t);
+// Whether make_fp_tex admits `vol` (esize bytes per voxel) on this device
+// (checks the limits only; creates nothing).
 bool fp_tex_fits(const GeomDev &g, const void *vol, int esize);
 void destroy_fp_tex(FpTex &t);
+// Projections of at most this many rays in one launch share each ray between
+// the 4 warps of a block when their corners come from a texture (k_fp_split.cu).
+constexpr long long FP_SPLIT_RAYS = 24576;
+cudaError_t launch_fp_split(const GeomDev &g, const ViewRec *views, int view0, int nviews, float *proj, float *raylen,
+                            float *weight, cudaStream_t s, const FpTex &tex);
+cudaError_t launch_fp_corr_split(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *b_stack,
+                                 float *raylen_state, float *corr, cudaStream_t s, const FpTex &tex, int skip_staged);
+cudaError_t launch_fp_corr_split(const GeomDev &g, const ViewRec *views, const ViewSel &sel,
+                                 const unsigned short *b_stack, float *raylen_state, float *corr, cudaStream_t s,
+                                 const FpTex &tex, int skip_staged);
+// The gather form an untuned context uses where the texture binds: tld4
+// corners, no view staged.  Measured against loads with the oblique views
+// staged (the form before), per view, us, views at 0 / 45 / 90 degrees:
+// 64^3 / 96^2 19/31/28 -> 10/11/10, 128^3 / 128^2 33/59/46 -> 15/14/15,
+// 192^3 / 256^2 45/93/66 -> 31/36/30, 256^3 / 512^2 124/213/176 -> 118/122/116
+// (the times before include the z-fastest copy of the views along x).
+constexpr int FP_DEFAULT_TEX = 10;
 // Forward projection of one view fused with the SART correction.  With usable
 // slab maps, staged views run in the slab-staged kernel and the others in the
 // gather kernel (both are launched; each leaves the other's views alone).
@@ -111,15 +132,22 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *
                            const ViewSel &sel, const float *b_stack, float *raylen_state, float *corr,
                            cudaStream_t s, const FpSlabMaps *maps = nullptr,
                            int *status = nullptr, int fp_variant = 0, const FpTex *tex = nullptr);
+cudaError_t launch_fp_corr_split(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t,
+                                 const ViewSel &sel, const float *b_stack, float *raylen_state, float *corr,
+                                 cudaStream_t s, const FpTex *tex, int form);
 cudaError_t launch_transpose(const GeomDev &g, const float *in, float *out, cudaStream_t s);
-cudaError_t launch_fp_bf16(const GeomDev &g, const ViewRec *views, const unsigned short *vol,
-                           const unsigned short *vol_t, int view0, int nviews, float *proj, float *raylen,
-                           float *weight, cudaStream_t s);
+cudaError_t launch_fp(const GeomDev &g, const ViewRec *views, const unsigned short *vol, const unsigned short *vol_t,
+                      int view0, int nviews, float *proj, float *raylen, float *weight, cudaStream_t s,
+                      const FpTex *tex = nullptr);
 cudaError_t launch_transpose_bf16(const GeomDev &g, const unsigned short *in, unsigned short *out, cudaStream_t s);
+// The copy for the selected view, if it gathers from one: a view along x, and
+// with staged_only (the gather form reads the volume's texture) only one that
+// the slab-staged kernel projects.
 cudaError_t launch_transpose_for_view(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *in,
-                                      float *out, cudaStream_t s);
+                                      float *out, cudaStream_t s, bool staged_only = false);
 cudaError_t launch_transpose_for_view(const GeomDev &g, const ViewRec *views, const ViewSel &sel,
-                                      const unsigned short *in, unsigned short *out, cudaStream_t s);
+                                      const unsigned short *in, unsigned short *out, cudaStream_t s,
+                                      bool staged_only = false);
 
 // BF16 storage (the raw upper halves of FP32 values; the solver's
 // stt_solve_cfg.storage): the overloads below on unsigned short arrays read

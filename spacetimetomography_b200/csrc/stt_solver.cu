@@ -83,7 +83,7 @@ struct stt_solver {
     float *warpbuf = nullptr;  // F volumes: backward-warped X_bar[f+1], then forward-warped Y_bc[f-1]
     float *corr = nullptr;     // F correction images
     float *ax = nullptr;       // plain form: forward projection image
-    void *volt = nullptr;      // F z-fastest volume copies (views gathering along x), in the state's storage
+    void *volt = nullptr;      // F z-fastest volume copies (null where no view gathers from one), in the state's storage
     float *raylen = nullptr;   // F sticky ray-length images
     float2 *acc = nullptr;     // ray-based BP accumulators, F volumes
     int *perm = nullptr;       // F x V device view order
@@ -100,7 +100,8 @@ struct stt_solver {
     long long launches_per_iter = 0;
     long long phase_launches[2] = {0, 0};
     std::vector<stt::FpSlabMaps> fpmaps;  // batched modes: per frame, TMA maps of the volume and its copy
-    std::vector<stt::FpTex> fptex;  // batched modes, a tld4 gather form: per frame, the volume's textures
+    std::vector<stt::FpTex> fptex;  // batched modes, a tld4 gather form: per frame, the volume's texture
+    stt::FpChoice fp{};             // batched modes: the projector's form
     stt::SweepJob *jobs_d = nullptr;  // STT_SOLVE_PERSISTENT: one job per frame
     unsigned *sweep_bar = nullptr;    // the jobs' barrier and ticket words (4 per frame), then the grid's
     int sweep_blocks = 0;
@@ -204,16 +205,16 @@ stt_status enqueue_primal(stt_solver *s, int f, cudaStream_t cs, long long &nl) 
 int fp_corr(stt_solver *s, int f, const float *vol, const float *volt, const stt::ViewSel &sel, const float *stack,
             float *rl, float *corr, cudaStream_t cs, cudaError_t &e) {
     const stt::FpSlabMaps *maps = s->fpmaps.empty() ? nullptr : &s->fpmaps[f];
-    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status,
-                            s->ctx->tuning.fp, s->fptex.empty() ? nullptr : &s->fptex[f]);
+    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status, s->fp.variant,
+                            s->fp.tex ? &s->fptex[f] : nullptr);
     return (maps && maps->ok) ? 2 : 1;  // slab-staged + gather kernels, or gather only
 }
 
 int fp_corr(stt_solver *s, int f, const unsigned short *vol, const unsigned short *volt, const stt::ViewSel &sel,
             const unsigned short *stack, float *rl, float *corr, cudaStream_t cs, cudaError_t &e) {
     const stt::FpSlabMaps *maps = s->fpmaps.empty() ? nullptr : &s->fpmaps[f];
-    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status,
-                            s->ctx->tuning.fp16, s->fptex.empty() ? nullptr : &s->fptex[f]);
+    e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status, s->fp.variant,
+                            s->fp.tex ? &s->fptex[f] : nullptr);
     return (maps && maps->ok) ? 2 : 1;
 }
 
@@ -225,10 +226,13 @@ stt_status enqueue_sart_batched(stt_solver *s, int f, cudaStream_t cs, long long
     float *corr = s->corr + f * s->npix;
     const T *stack = reinterpret_cast<const T *>(s->st.proj) + (size_t)f * V * s->npix;
     const int voxel = s->cfg.bp_mode == 0;
-    T *volt = reinterpret_cast<T *>(s->volt) + f * s->n;
+    T *volt = s->volt ? reinterpret_cast<T *>(s->volt) + f * s->n : nullptr;  // none: no view gathers from a copy
     for (int i = 0; i < V; ++i) {
         const stt::ViewSel sel{0, s->perm + (size_t)f * V, i, f * V};
-        SCUDA(s, stt::launch_transpose_for_view(g, s->views, sel, vol, volt, cs), "transpose");
+        if (volt) {
+            SCUDA(s, stt::launch_transpose_for_view(g, s->views, sel, vol, volt, cs, s->fp.tex), "transpose");
+            ++nl;
+        }
         cudaError_t e = cudaSuccess;
         nl += fp_corr(s, f, vol, volt, sel, stack, voxel ? s->raylen + f * s->npix : nullptr, corr, cs, e);
         SCUDA(s, e, "fp_corr");
@@ -240,7 +244,7 @@ stt_status enqueue_sart_batched(stt_solver *s, int f, cudaStream_t cs, long long
             SCUDA(s, stt::launch_bp_ray(g, s->views, sel, corr, s->acc + f * s->n, vol, s->cfg.pd.gmax, cs,
                                         s->ctx->tuning.ray),
                   "bp_ray");
-        nl += voxel ? 2 : 3;
+        nl += voxel ? 1 : 2;
     }
     const int d[3] = {g.nx, g.ny, g.nz};
     SCUDA(s, stt::launch_roi_apply(d, s->cfg.roi_cut, s->cfg.pd.cut, vol, vol_of<T>(s, s->st.xprev, f),
@@ -459,16 +463,6 @@ stt_status run_plain(stt_solver *s, cudaStream_t cs, long long &nl, int phase) {
     return bf16(s) ? run_plain_t<unsigned short>(s, cs, nl, phase) : run_plain_t<float>(s, cs, nl, phase);
 }
 
-cudaError_t fp_view(const stt::GeomDev &g, const stt::ViewRec *views, const float *vol, const float *volt, int view,
-                    float *ax, float *rl, cudaStream_t cs) {
-    return stt::launch_fp(g, views, vol, volt, view, 1, ax, rl, nullptr, cs);
-}
-
-cudaError_t fp_view(const stt::GeomDev &g, const stt::ViewRec *views, const unsigned short *vol,
-                    const unsigned short *volt, int view, float *ax, float *rl, cudaStream_t cs) {
-    return stt::launch_fp_bf16(g, views, vol, volt, view, 1, ax, rl, nullptr, cs);
-}
-
 template <typename T>
 stt_status plain_frame_tail(stt_solver *s, int f, cudaStream_t cs, long long &nl) {
     const stt::GeomDev &g = *s->g;
@@ -489,7 +483,7 @@ stt_status plain_frame_tail(stt_solver *s, int f, cudaStream_t cs, long long &nl
             SCUDA(s, stt::launch_transpose_for_view(g, s->views, sel, vol, volt, cs), "transpose");
             ++nl;
             if (voxel) {
-                SCUDA(s, fp_view(g, s->views, vol, volt, view, s->ax, rl, cs), "fp");
+                SCUDA(s, stt::launch_fp(g, s->views, vol, volt, view, 1, s->ax, rl, nullptr, cs), "fp");
                 SCUDA(s, stt::launch_correction((long long)s->npix, b, s->ax, rl, corr, cs), "correction");
                 SCUDA(s, stt::launch_bp_voxel(g, s->views, sel, corr, vol, (float)s->cfg.alpha, s->cfg.pd.gmax, cs),
                       "bp_voxel");
@@ -497,7 +491,7 @@ stt_status plain_frame_tail(stt_solver *s, int f, cudaStream_t cs, long long &nl
             } else {
                 // ray-based: the producer is reset after every view (L = 0 on a miss)
                 SCUDA(s, stt::launch_fill_zero(rl, (long long)s->npix, cs), "fill");
-                SCUDA(s, fp_view(g, s->views, vol, volt, view, s->ax, rl, cs), "fp");
+                SCUDA(s, stt::launch_fp(g, s->views, vol, volt, view, 1, s->ax, rl, nullptr, cs), "fp");
                 SCUDA(s, stt::launch_correction((long long)s->npix, b, s->ax, rl, corr, cs), "correction");
                 SCUDA(s, stt::launch_bp_ray(g, s->views, sel, corr, s->acc + f * s->n, vol, s->cfg.pd.gmax, cs,
                                             s->ctx->tuning.ray),
@@ -568,11 +562,6 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
     if (!e) e = alloc(s, s->warpbuf, (size_t)F * s->n, "warp buffers");
     if (!e) e = alloc(s, s->corr, (size_t)F * s->npix, "corrections");
     if (!e) e = alloc(s, s->ax, s->npix, "projection");
-    if (!e) {
-        unsigned char *vt = nullptr;
-        e = alloc(s, vt, (size_t)F * s->n * (cfg->storage == STT_DTYPE_BF16 ? 2 : 4), "transposed volumes");
-        s->volt = vt;
-    }
     if (!e) e = alloc(s, s->raylen, (size_t)F * s->npix, "ray lengths");
     if (!e) e = alloc(s, s->perm, (size_t)F * s->V, "view order");
     if (!e) e = alloc(s, s->counter, 1, "iteration counter");
@@ -582,33 +571,44 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
         stt_solver_destroy(s);
         return e;
     }
-    // no views staged for this storage (the tuner found one gather launch per
-    // view faster than the two kernels): no maps, one launch per view
-    const bool any_staged = (cfg->storage == STT_DTYPE_F32 ? ctx->staged_bins : ctx->staged_bins16) != 0;
-    // (the persistent sweep gathers with loads: no maps or textures)
+    // The projector's form: the texture only where every frame's volume binds.
+    // (The plain and persistent forms gather with loads.)
+    const bool f32 = cfg->storage == STT_DTYPE_F32;
     const bool per_view_kernels = cfg->mode == STT_SOLVE_STREAMS || cfg->mode == STT_SOLVE_GRAPH;
-    if (per_view_kernels && any_staged) {
+    const unsigned short *vol16 = reinterpret_cast<const unsigned short *>(s->st.vol);
+    if (per_view_kernels) {
+        auto choice = [&](bool binds) {
+            return f32 ? stt::fp_choice(ctx, s->st.vol, binds) : stt::fp_choice(ctx, vol16, binds);
+        };
+        bool binds = choice(true).tex;
+        if (binds) {
+            s->fptex.resize(F);
+            for (int f = 0; f < F && binds; ++f)
+                binds = f32 ? stt::make_fp_tex(*g, s->st.vol + f * s->n, s->fptex[f])
+                            : stt::make_fp_tex(*g, vol16 + f * s->n, s->fptex[f]);
+        }
+        s->fp = choice(binds);
+    }
+    // the z-fastest copies, where a view may gather from one
+    if (!per_view_kernels || !s->fp.tex || s->fp.stage) {
+        unsigned char *vt = nullptr;
+        if ((e = alloc(s, vt, (size_t)F * s->n * (f32 ? 4 : 2), "transposed volumes"))) {
+            stt_solver_destroy(s);
+            return e;
+        }
+        s->volt = vt;
+    }
+    // no views staged (one gather launch per view): no maps
+    if (per_view_kernels && s->fp.stage) {
         s->fpmaps.resize(F);
         for (int f = 0; f < F; ++f) {  // where the maps do not apply, ok stays 0 and every view gathers
-            if (cfg->storage == STT_DTYPE_F32)
+            if (f32)
                 stt::make_fp_slab_maps(*g, s->st.vol + f * s->n, static_cast<float *>(s->volt) + f * s->n,
                                        s->fpmaps[f], ctx->tuning.slab);
             else
-                stt::make_fp_slab_maps(*g, reinterpret_cast<const unsigned short *>(s->st.vol) + f * s->n,
-                                       static_cast<unsigned short *>(s->volt) + f * s->n, s->fpmaps[f],
-                                       ctx->tuning.slab);
+                stt::make_fp_slab_maps(*g, vol16 + f * s->n, static_cast<unsigned short *>(s->volt) + f * s->n,
+                                       s->fpmaps[f], ctx->tuning.slab);
         }
-    }
-    if (per_view_kernels && cfg->storage == STT_DTYPE_F32 && stt::is_tex_fp_variant(ctx->tuning.fp)) {
-        s->fptex.resize(F);  // where they cannot be made, ok stays 0 and the loads run
-        for (int f = 0; f < F; ++f)
-            stt::make_fp_tex(*g, s->st.vol + f * s->n, static_cast<float *>(s->volt) + f * s->n, s->fptex[f]);
-    }
-    if (per_view_kernels && cfg->storage == STT_DTYPE_BF16 && ctx->tuning.fp16 == 1) {
-        s->fptex.resize(F);
-        for (int f = 0; f < F; ++f)
-            stt::make_fp_tex(*g, reinterpret_cast<const unsigned short *>(s->st.vol) + f * s->n,
-                             static_cast<unsigned short *>(s->volt) + f * s->n, s->fptex[f]);
     }
     if (cfg->mode == STT_SOLVE_PERSISTENT) {
         s->sweep_wide = (long long)g->nx * g->ny * g->nz >= (1LL << 31);  // 64-bit gather offsets

@@ -55,8 +55,8 @@ struct Scratch {
     float2 *acc = nullptr;
     unsigned short *vol16 = nullptr, *volt16 = nullptr, *b16 = nullptr;  // BF16 copies for the BF16 choice
     stt::ViewRec *tv = nullptr;
-    stt::FpTex fptex;    // the textures of the tld4 gather variants over vol and volt
-    stt::FpTex fptex16;  // the same over vol16 and volt16
+    stt::FpTex fptex;    // the texture of the tld4 gather variants over vol
+    stt::FpTex fptex16;  // the same over vol16
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     ~Scratch() {
         stt::destroy_fp_tex(fptex);
@@ -118,32 +118,36 @@ stt_status apply_staged_bins(stt_ctx *ctx) {
     return STT_OK;
 }
 
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol, const float *vol_t) {
-    return is_tex_fp_variant(ctx->tuning.fp) ? ctx_fp_tex_any(ctx, vol, vol_t) : nullptr;
-}
-
 namespace {
 template <typename T>
-const FpTex *cached_tex(stt_ctx *ctx, const T *vol, const T *vol_t) {
+const FpTex *cached_tex(stt_ctx *ctx, const T *vol) {
     const GeomDev &g = ctx->g;
     const int es = (int)sizeof(T);
     for (const auto &e : ctx->fp_tex)
-        if (e.vol == vol && e.volt == vol_t && e.nx == g.nx && e.ny == g.ny && e.nz == g.nz && e.esize == es)
-            return &e.tex;
+        if (e.vol == vol && e.nx == g.nx && e.ny == g.ny && e.nz == g.nz && e.esize == es)
+            return e.tex.ok ? &e.tex : nullptr;
     if ((int)ctx->fp_tex.size() >= stt_ctx::kFpTexCache) return nullptr;
-    stt_ctx::FpTexEntry e{vol, vol_t, g.nx, g.ny, g.nz, es, FpTex{}};
-    make_fp_tex(g, vol, vol_t, e.tex);  // where it fails, tex.ok = 0 is cached too: the loads run
+    stt_ctx::FpTexEntry e{vol, g.nx, g.ny, g.nz, es, FpTex{}};
+    make_fp_tex(g, vol, e.tex);  // where it fails, tex.ok = 0 is cached too: the loads run
     ctx->fp_tex.push_back(e);
-    return &ctx->fp_tex.back().tex;
+    return ctx->fp_tex.back().tex.ok ? &ctx->fp_tex.back().tex : nullptr;
 }
 }  // namespace
 
-const FpTex *ctx_fp_tex_any(stt_ctx *ctx, const float *vol, const float *vol_t) {
-    return cached_tex(ctx, vol, vol_t);
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol) { return cached_tex(ctx, vol); }
+
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol) { return cached_tex(ctx, vol); }
+
+FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds) {
+    if (ctx->tuned) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), ctx->staged_bins != 0};
+    if (tex_binds) return {FP_DEFAULT_TEX, true, false};
+    return {0, false, ctx->staged_bins != 0};
 }
 
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, const unsigned short *vol_t) {
-    return ctx->tuning.fp16 == 1 ? cached_tex(ctx, vol, vol_t) : nullptr;
+FpChoice fp_choice(const stt_ctx *ctx, const unsigned short *, bool tex_binds) {
+    if (ctx->tuned) return {ctx->tuning.fp16, tex_binds && ctx->tuning.fp16 == 1, ctx->staged_bins16 != 0};
+    if (tex_binds) return {1, true, false};
+    return {0, false, ctx->staged_bins16 != 0};
 }
 
 }  // namespace stt
@@ -264,7 +268,16 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
     bool slab_ok = false;
     for (int sv = 0; sv < stt::kSlabVariants; ++sv)
         slab_ok |= maps_ok[sv] = stt::make_fp_slab_maps(g, sc.vol, sc.volt, maps[sv], sv);
-    stt::make_fp_tex(g, sc.vol, sc.volt, sc.fptex);  // where it fails, ok = 0 and the tld4 variants are skipped
+    // the loads and the staged boxes read the z-fastest copy for the views along
+    // x, made anew for every view of a sweep; the textures read the volume
+    float t_copy = 0.0f, along_x[9] = {};
+    if ((e = time_us(sc, s, [&] { return stt::launch_transpose(g, sc.vol, sc.volt, s); }, t_copy)))
+        return fail(e, "copy");
+    for (size_t v = 0; v < ctx->views_h.size(); ++v) {
+        const int b = stt::off_axis_bin(ctx->off_axis_deg[v]);
+        if (ctx->views_h[v].layout == 1) along_x[b] += 1.0f / (float)count[b];
+    }
+    stt::make_fp_tex(g, sc.vol, sc.fptex);  // where it fails, ok = 0 and the tld4 variants are skipped
     for (int b = 0; b < 9; ++b) {
         if (rep[b] < 0) continue;
         stt::ViewRec two[2] = {ctx->views_h[rep[b]], ctx->views_h[rep[b]]};
@@ -283,6 +296,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
                                            ctx->status, fv, &sc.fptex);
             }, tg[fv][b]);
             if (e) return fail(e, "gather projector");
+            if (!stt::is_tex_fp_variant(fv)) tg[fv][b] += t_copy * along_x[b];
         }
         if (slab_ok && t_idle == 0.0f) {
             int sv0 = 0;
@@ -300,6 +314,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
                                                 ctx->status);
             }, ts[sv][b]);
             if (e) return fail(e, "slab projector");
+            ts[sv][b] += t_copy * along_x[b];
         }
     }
     // the gather variant with the least time over all views; then the box
@@ -363,7 +378,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
             (e = cudaMemsetAsync(sc.volt16, 0x3F, n * sizeof(unsigned short), s)) ||
             (e = cudaMemsetAsync(sc.b16, 0, npix * sizeof(unsigned short), s)))
             return fail(e, "BF16 scratch");
-        stt::make_fp_tex(g, sc.vol16, sc.volt16, sc.fptex16);  // where it fails, ok = 0: loads only
+        stt::make_fp_tex(g, sc.vol16, sc.fptex16);  // where it fails, ok = 0: loads only
         stt::FpSlabMaps m16;
         const bool maps16 = stt::make_fp_slab_maps(g, sc.vol16, sc.volt16, m16, t.slab_variant);
         float tg16[stt::kFp16Variants][9] = {}, ts16[9] = {};
@@ -383,6 +398,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
                                                sc.rl, sc.corr, s, nullptr, ctx->status, fv, &sc.fptex16);
                 }, tg16[fv][b]);
                 if (e) return fail(e, "BF16 gather projector");
+                if (fv == 0) tg16[fv][b] += 0.5f * t_copy * along_x[b];
             }
             if (!maps16) continue;
             e = time_us(sc, s, [&] {
@@ -390,6 +406,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
                                                 sc.b16, sc.rl, sc.corr, s, ctx->status);
             }, ts16[b]);
             if (e) return fail(e, "BF16 slab projector");
+            ts16[b] += 0.5f * t_copy * along_x[b];
             if (t_idle16 == 0.0f) {
                 e = time_us(sc, s, [&] {
                     return stt::launch_fp_corr_slab(g, sc.tv, m16, sc.vol16, sc.volt16, stt::ViewSel{0, nullptr, 0, 0},
