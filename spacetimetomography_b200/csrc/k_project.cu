@@ -310,6 +310,21 @@ __global__ void __launch_bounds__(256) k_transpose_for_view(int nx, int ny, int 
     transpose_tile(nx, ny, nz, in, out);
 }
 
+// A volume's slices to their places in its mirror, four elements a thread.
+template <typename T>
+__global__ void __launch_bounds__(256) k_mirror(int slice, int pitch, const T *__restrict__ vol, T *__restrict__ mirror) {
+    const T *in = vol + (size_t)blockIdx.y * slice;
+    T *out = mirror + (size_t)blockIdx.y * pitch;
+    const int k0 = blockIdx.x * 1024 + threadIdx.x;
+    T v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (k0 + 256 * q < slice) v[q] = in[k0 + 256 * q];
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (k0 + 256 * q < slice) out[k0 + 256 * q] = v[q];
+}
+
 __global__ void k_fill_zero(long long n, float *__restrict__ p) {
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
          k += (long long)gridDim.x * blockDim.x)
@@ -506,8 +521,7 @@ bool tex_limits(TexLimits &l) {
     return true;
 }
 
-bool slices_fit(const TexLimits &l, const void *p, long long width, long long rows, int esize) {
-    const long long pitch = width * (long long)esize;
+bool slices_fit(const TexLimits &l, const void *p, long long width, long long rows, long long pitch) {
     return p && width >= 2 && rows >= 2 && width <= l.width && rows <= l.height && pitch <= l.pitch &&
            !(l.pitch_align > 0 && pitch % l.pitch_align) && !(l.base_align > 0 && (uintptr_t)p % l.base_align);
 }
@@ -516,9 +530,8 @@ bool slices_fit(const TexLimits &l, const void *p, long long width, long long ro
 // linear memory (FP32 texels, or 16-bit unsigned ones holding BF16 bits); 0
 // where the limits do not admit it.
 template <typename T>
-unsigned long long slices_texture(const TexLimits &l, const T *p, long long width, long long rows) {
-    const long long pitch = width * (long long)sizeof(T);
-    if (!slices_fit(l, p, width, rows, (int)sizeof(T))) return 0;
+unsigned long long slices_texture(const TexLimits &l, const T *p, long long width, long long rows, long long pitch) {
+    if (!slices_fit(l, p, width, rows, pitch)) return 0;
     cudaResourceDesc rd{};
     rd.resType = cudaResourceTypePitch2D;
     rd.res.pitch2D.devPtr = const_cast<T *>(p);
@@ -566,24 +579,46 @@ const char *fp16_variant_name(int v) {
 
 namespace {
 template <typename T>
-bool make_fp_tex_any(const GeomDev &g, const T *vol, FpTex &t) {
+bool make_fp_tex_any(const GeomDev &g, const T *vol, FpTex &t, size_t pitch) {
     t = FpTex{};
     TexLimits l;
     if (!small_volume(g) || !tex_limits(l)) return false;
-    t.x = slices_texture(l, vol, (long long)g.nx * g.ny, g.nz);
+    const long long slice = (long long)g.nx * g.ny;
+    t.x = slices_texture(l, vol, slice, g.nz, (pitch ? (long long)pitch : slice) * (long long)sizeof(T));
     t.ok = t.x != 0;
     t.esize = (int)sizeof(T);
     return t.ok != 0;
 }
 }  // namespace
 
-bool make_fp_tex(const GeomDev &g, const float *vol, FpTex &t) { return make_fp_tex_any(g, vol, t); }
+bool make_fp_tex(const GeomDev &g, const float *vol, FpTex &t, size_t pitch) { return make_fp_tex_any(g, vol, t, pitch); }
 
-bool make_fp_tex(const GeomDev &g, const unsigned short *vol, FpTex &t) { return make_fp_tex_any(g, vol, t); }
+bool make_fp_tex(const GeomDev &g, const unsigned short *vol, FpTex &t, size_t pitch) {
+    return make_fp_tex_any(g, vol, t, pitch);
+}
 
-bool fp_tex_fits(const GeomDev &g, const void *vol, int esize) {
+namespace {
+template <typename T>
+cudaError_t mirror_any(const GeomDev &g, const T *vol, T *mirror, cudaStream_t s) {
+    const int slice = g.nx * g.ny;  // (a mirrored volume has fewer than 2^31 voxels)
+    const int nb = (slice + 1023) / 1024;
+    k_mirror<T><<<dim3(nb, g.nz), 256, 0, s>>>(slice, (int)fp_mirror_pitch(slice), vol, mirror);
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_mirror(const GeomDev &g, const float *vol, float *mirror, cudaStream_t s) {
+    return mirror_any(g, vol, mirror, s);
+}
+
+cudaError_t launch_mirror(const GeomDev &g, const unsigned short *vol, unsigned short *mirror, cudaStream_t s) {
+    return mirror_any(g, vol, mirror, s);
+}
+
+bool fp_tex_fits(const GeomDev &g, const void *vol, int esize, size_t pitch) {
     TexLimits l;
-    return small_volume(g) && tex_limits(l) && slices_fit(l, vol, (long long)g.nx * g.ny, g.nz, esize);
+    const long long slice = (long long)g.nx * g.ny;
+    return small_volume(g) && tex_limits(l) && slices_fit(l, vol, slice, g.nz, (pitch ? (long long)pitch : slice) * esize);
 }
 
 void destroy_fp_tex(FpTex &t) {

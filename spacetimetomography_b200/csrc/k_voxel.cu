@@ -58,10 +58,12 @@ __device__ __forceinline__ BpCol bp_col(const GeomDev &g, const ViewRec &v, floa
     return c;
 }
 
-template <int K, int OCC, typename T>
+// MIR: every voxel written goes to `mirror` (slices mpitch elements apart) too.
+template <int K, int OCC, typename T, bool MIR>
 __global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, const ViewRec *__restrict__ views,
                                                             const ViewSel sel, const float *__restrict__ corr,
-                                                            T *__restrict__ vol, float alpha, float gmax) {
+                                                            T *__restrict__ vol, float alpha, float gmax,
+                                                            T *__restrict__ mirror, size_t mpitch) {
     __shared__ float table[BP_ROWS * 4 * BP_PITCH];
     constexpr int RS = 4 * BP_PITCH;  // one row of every column
     int local;
@@ -93,14 +95,17 @@ __global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, con
     if (x >= g.nx || z >= g.nz) return;
     const float fx = (float)x, fz = (float)z;
     const BpCol c = bp_col(g, v, fx, fz, y0, y1);
+    T *col = vol + x + (size_t)y0 * g.nx + (size_t)z * g.nx * g.ny;
+    T *mcol = MIR ? mirror + x + (size_t)y0 * g.nx + z * mpitch : nullptr;
     if (!rot_y || (c.live && c.nr > BP_ROWS)) {
         bp_column<K>(g, v, BpRowsLdg{corr, g.W}, vol, x, y0, z, alpha, gmax);
+        if (MIR)
+            for (int y = y0; y < y1; ++y, col += g.nx, mcol += g.nx) *mcol = *col;
         return;
     }
     if (!c.live) return;
     const float *row = table + zl * BP_PITCH + xl - RS * (c.r0 + 1);
     const float top = bp_top(gmax);
-    T *col = vol + x + (size_t)y0 * g.nx + (size_t)z * g.nx * g.ny;
     if (y1 - y0 == K && c.ulo >= 2.0f + BP_NEAR && c.uhi < (float)(g.H - 2) - BP_NEAR) {  // every voxel is updated
         float vox[BP_G];
 #pragma unroll
@@ -119,15 +124,18 @@ __global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, con
                 bp_weights(upy - (float)py, wy);
                 const float *w = row + RS * py;
                 const float s[4] = {w[0], w[RS], w[2 * RS], w[3 * RS]};
-                st_stored(col + q * g.nx, bp_value(vox[q], alpha, bp_sum(s, wy), top));
+                const float nv = bp_value(vox[q], alpha, bp_sum(s, wy), top);
+                st_stored(col + q * g.nx, nv);
+                if (MIR) st_stored(mcol + q * g.nx, nv);
             }
             col += BP_G * g.nx;
+            if (MIR) mcol += BP_G * g.nx;
 #pragma unroll
             for (int q = 0; q < BP_G; ++q) vox[q] = next[q];
         }
         return;
     }
-    for (int y = y0; y < y1; ++y, col += g.nx) {
+    for (int y = y0; y < y1; ++y, col += g.nx, mcol += MIR ? g.nx : 0) {
         const float camy = bp_cam(v, 1, fx, (float)y, fz), upy = bp_coord(g.cy, camy, c.scale);
         if (!bp_inside(g, upy, g.cy, camy, c.ndepth, g.H)) continue;
         const int py = bp_tap(upy, g.H);
@@ -135,7 +143,9 @@ __global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, con
         bp_weights(upy - (float)py, wy);
         const float *w = row + RS * py;
         const float s[4] = {w[0], w[RS], w[2 * RS], w[3 * RS]};
-        st_stored(col, bp_value(ld_stored(col), alpha, bp_sum(s, wy), top));
+        const float nv = bp_value(ld_stored(col), alpha, bp_sum(s, wy), top);
+        st_stored(col, nv);
+        if (MIR) st_stored(mcol, nv);
     }
 }
 
@@ -272,25 +282,29 @@ cudaError_t launch_fill_seeded(long long n, unsigned long long seed, float *x, c
 namespace {
 template <int K, int OCC, typename T>
 cudaError_t bp_cols(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr, T *vol, float alpha,
-                    float gmax, cudaStream_t s) {
-    k_bp_voxel_cols<K, OCC, T><<<dim3((g.nx + 31) / 32, (g.ny + K - 1) / K, (g.nz + 3) / 4), 128, 0, s>>>(
-        g, views, sel, corr, vol, alpha, gmax);
+                    float gmax, cudaStream_t s, T *mirror) {
+    const dim3 grid((g.nx + 31) / 32, (g.ny + K - 1) / K, (g.nz + 3) / 4);
+    if (mirror)
+        k_bp_voxel_cols<K, OCC, T, true><<<grid, 128, 0, s>>>(g, views, sel, corr, vol, alpha, gmax, mirror,
+                                                              fp_mirror_pitch((size_t)g.nx * g.ny));
+    else
+        k_bp_voxel_cols<K, OCC, T, false><<<grid, 128, 0, s>>>(g, views, sel, corr, vol, alpha, gmax, mirror, 0);
     return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t bp_voxel_any(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr, T *vol,
-                         float alpha, float gmax, cudaStream_t s, int bp_variant) {
+                         float alpha, float gmax, cudaStream_t s, int bp_variant, T *mirror) {
     switch (bp_variant) {
-    case 1: return bp_cols<8, 8>(g, views, sel, corr, vol, alpha, gmax, s);
-    case 2: return bp_cols<20, 8>(g, views, sel, corr, vol, alpha, gmax, s);
-    case 3: return bp_cols<16, 6>(g, views, sel, corr, vol, alpha, gmax, s);
-    case 4: return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s);
+    case 1: return bp_cols<8, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
+    case 2: return bp_cols<20, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
+    case 3: return bp_cols<16, 6>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
+    case 4: return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
     default: break;
     }
-    if (g.bp_len == 8) return bp_cols<8, 8>(g, views, sel, corr, vol, alpha, gmax, s);
-    if (g.bp_len == 12) return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s);
-    return bp_cols<16, 8>(g, views, sel, corr, vol, alpha, gmax, s);
+    if (g.bp_len == 8) return bp_cols<8, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
+    if (g.bp_len == 12) return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
+    return bp_cols<16, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
 }
 
 template <typename T>
@@ -342,13 +356,14 @@ const char *bp_variant_name(int v) {
 }
 
 cudaError_t launch_bp_voxel(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                            float *vol, float alpha, float gmax, cudaStream_t s, int bp_variant) {
-    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, bp_variant);
+                            float *vol, float alpha, float gmax, cudaStream_t s, int bp_variant, float *mirror) {
+    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, bp_variant, mirror);
 }
 
 cudaError_t launch_bp_voxel(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                            unsigned short *vol, float alpha, float gmax, cudaStream_t s, int bp_variant) {
-    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, bp_variant);
+                            unsigned short *vol, float alpha, float gmax, cudaStream_t s, int bp_variant,
+                            unsigned short *mirror) {
+    return bp_voxel_any(g, views, sel, corr, vol, alpha, gmax, s, bp_variant, mirror);
 }
 
 cudaError_t launch_pd_dual(const int *d, const PdParams &p, const float *xf, const float *xf1,

@@ -141,6 +141,10 @@ stt_status stt_destroy(stt_ctx *ctx) {
     cudaFree(ctx->pwd);
     cudaFree(ctx->status);
     for (auto &e : ctx->fp_tex) stt::destroy_fp_tex(e.tex);
+    for (auto &m : ctx->mirror) {
+        stt::destroy_fp_tex(m.tex);
+        cudaFree(m.p);
+    }
     delete ctx;
     return STT_OK;
 }
@@ -326,27 +330,52 @@ static stt_status check_views(stt_ctx *ctx, int view0, int nviews) {
 
 }  // extern "C"
 
-// Projections of [view0, view0 + nviews): corners from the volume's texture
-// where it binds (no copy), else by loads.
+// Where a call's projections fetch their corners: the volume's own texture, a
+// mirror's (made from the volume here; `mirror` set), or loads (tex null).
+template <typename T>
+struct FpSource {
+    const stt::FpTex *tex = nullptr;
+    T *mirror = nullptr;
+};
+
+template <typename T>
+static stt_status fp_source(stt_ctx *ctx, const T *vol, cudaStream_t s, FpSource<T> &src) {
+    src = FpSource<T>{};
+    if ((src.tex = stt::ctx_fp_tex(ctx, vol, s))) return STT_OK;
+    if (!(src.tex = stt::ctx_mirror_tex(ctx, s, &src.mirror))) return STT_OK;
+    STT_CUDA(ctx, stt::launch_mirror(ctx->g, vol, src.mirror, s), "k_mirror launch");
+    return STT_OK;
+}
+
+// Projections of [view0, view0 + nviews): corners from a texture where one
+// binds (no z-fastest copy), else by loads.
 template <typename T>
 static stt_status project(stt_ctx *ctx, const T *vol, float *proj, float *raylen, float *weight, int view0, int nviews,
                           cudaStream_t s) {
-    const stt::FpTex *tex = stt::ctx_fp_tex(ctx, vol);
-    const T *volt = nullptr;
-    stt_status st = tex ? STT_OK : transposed_if_needed(ctx, vol, view0, nviews, s, &volt);
+    FpSource<T> src;
+    stt_status st = fp_source(ctx, vol, s, src);
     if (st) return st;
-    STT_CUDA(ctx, stt::launch_fp(ctx->g, ctx->views_d, vol, volt, view0, nviews, proj, raylen, weight, s, tex),
+    const T *volt = nullptr;
+    if (!src.tex && (st = transposed_if_needed(ctx, vol, view0, nviews, s, &volt))) return st;
+    STT_CUDA(ctx, stt::launch_fp(ctx->g, ctx->views_d, vol, volt, view0, nviews, proj, raylen, weight, s, src.tex),
              "k_fp launch");
     return STT_OK;
+}
+
+// What project_corr fetches from: a texture only if the context's choice of
+// form is one.
+template <typename T>
+static stt_status corr_source(stt_ctx *ctx, const T *vol, cudaStream_t s, FpSource<T> &src) {
+    src = FpSource<T>{};
+    return stt::fp_choice(ctx, vol, true).tex ? fp_source(ctx, vol, s, src) : STT_OK;
 }
 
 // The fused forward projection and correction of one view: the gather form of
 // the context's choice and, where its maps apply, the slab-staged kernel.
 template <typename T>
-static stt_status project_corr(stt_ctx *ctx, const T *vol, const stt::ViewSel &sel, const T *stack, float *raylen,
-                               float *corr, cudaStream_t s) {
-    const stt::FpTex *tex = stt::ctx_fp_tex(ctx, vol);
-    const stt::FpChoice c = stt::fp_choice(ctx, vol, tex != nullptr);
+static stt_status project_corr(stt_ctx *ctx, const T *vol, const FpSource<T> &src, const stt::ViewSel &sel,
+                               const T *stack, float *raylen, float *corr, cudaStream_t s) {
+    const stt::FpChoice c = stt::fp_choice(ctx, vol, src.tex != nullptr);
     const stt::ViewRec &v = ctx->views_h[sel.view];
     const T *volt = nullptr;
     if (stt::fp_needs_copy(c, v, (sizeof(T) == 2 ? v.staged16 : v.staged) != 0))
@@ -354,7 +383,7 @@ static stt_status project_corr(stt_ctx *ctx, const T *vol, const stt::ViewSel &s
     stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
     if (c.stage) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
     STT_CUDA(ctx, stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, raylen, corr, s, &maps, ctx->status,
-                                      c.variant, c.tex ? tex : nullptr),
+                                      c.variant, c.tex ? src.tex : nullptr),
              "k_fp_corr launch");
     return STT_OK;
 }
@@ -388,7 +417,9 @@ stt_status stt_fp_correction(stt_ctx *ctx, const float *vol, const float *b, flo
     if (!vol || !b || !corr) return fail(ctx, STT_ERR_INVALID, "null vol, b or corr");
     if ((st = check_views(ctx, view, 1))) return st;
     if ((st = set_device(ctx))) return st;
-    return project_corr(ctx, vol, stt::ViewSel{view, nullptr, 0, view}, b, raylen_state, corr, S(stream));
+    FpSource<float> src;
+    if ((st = corr_source(ctx, vol, S(stream), src))) return st;
+    return project_corr(ctx, vol, src, stt::ViewSel{view, nullptr, 0, view}, b, raylen_state, corr, S(stream));
 }
 
 stt_status stt_fp_texture_ok_typed(stt_ctx *ctx, const void *vol, int dtype, int *ok) {
@@ -417,7 +448,7 @@ stt_status stt_gather_ceiling(stt_ctx *ctx, const float *vol, int view, int pack
     const float *volt = nullptr;
     const stt::FpTex *tex = nullptr;
     if (packed & 2) {  // tld4 corners
-        tex = stt::ctx_fp_tex(ctx, vol);
+        tex = stt::ctx_fp_tex(ctx, vol, S(stream));
         if (!tex)
             return fail(ctx, STT_ERR_UNSUPPORTED, "the device's texture limits do not admit this volume");
     } else if ((st = transposed_if_needed(ctx, vol, view, 1, S(stream), &volt))) {
@@ -577,21 +608,25 @@ static stt_status sart_sweep_t(stt_ctx *ctx, T *vol, const T *proj_stack, const 
     const size_t npix = (size_t)ctx->g.W * ctx->g.H;
     if ((st = ensure(ctx, ctx->corr, ctx->corr_n, npix, "correction image"))) return st;
     if (bp_mode == 1 && (st = ensure_acc(ctx, s))) return st;
+    FpSource<T> src;
+    if (nperm > 0 && (st = corr_source(ctx, static_cast<const T *>(vol), s, src))) return st;
     for (int i = 0; i < nperm; ++i) {
         const stt::ViewSel sel{view_offset + perm[i], nullptr, 0, view_offset};
         // ray-based mode: TypicalRayProducer::Initial zeroes the ray lengths
         // after every view, so missed rays see L = 0 (no sticky state)
-        if ((st = project_corr(ctx, static_cast<const T *>(vol), sel, proj_stack, bp_mode == 0 ? raylen_state : nullptr,
+        if ((st = project_corr(ctx, static_cast<const T *>(vol), src, sel, proj_stack, bp_mode == 0 ? raylen_state : nullptr,
                                ctx->corr, s)))
             return st;
         if (bp_mode == 0)
             STT_CUDA(ctx, stt::launch_bp_voxel(ctx->g, ctx->views_d, sel, ctx->corr, vol, (float)alpha, gmax, s,
-                                               ctx->tuning.bp),
+                                               ctx->tuning.bp, src.mirror),
                      "k_bp_voxel launch");
         else
             STT_CUDA(ctx, stt::launch_bp_ray(ctx->g, ctx->views_d, sel, ctx->corr, ctx->acc, vol, gmax, s,
                                              ctx->tuning.ray),
                      "k_bp_ray launch");
+        if (bp_mode == 1 && src.mirror && i + 1 < nperm)
+            STT_CUDA(ctx, stt::launch_mirror(ctx->g, static_cast<const T *>(vol), src.mirror, s), "k_mirror launch");
     }
     if (bp_mode == 1 && raylen_state)
         STT_CUDA(ctx, cudaMemsetAsync(raylen_state, 0, npix * sizeof(float), s), "cudaMemsetAsync(raylen)");

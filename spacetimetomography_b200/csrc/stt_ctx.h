@@ -54,6 +54,14 @@ struct stt_ctx {
     };
     static constexpr int kFpTexCache = 32;
     std::vector<FpTexEntry> fp_tex;
+    // The mirror of a volume no texture binds (launch_mirror), by storage:
+    // [0] FP32, [1] BF16.  Written anew by every call that projects from it.
+    struct Mirror {
+        void *p = nullptr;
+        size_t bytes = 0;
+        int nx = 0, ny = 0, nz = 0;
+        stt::FpTex tex;
+    } mirror[2];
 };
 
 namespace stt {
@@ -65,9 +73,14 @@ inline int off_axis_bin(float deg) {
 // Applies ctx->staged_bins and staged_bins16 to every view (host and device tables).
 stt_status apply_staged_bins(stt_ctx *ctx);
 // The texture of `vol` (created on first use, cached in the context), whatever
-// the tuned variant; nullptr where it does not bind or the cache is full.
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol);
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol);
+// the tuned variant; nullptr where it does not bind, the cache is full, or it
+// would have to be created while `s` is being captured.
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol, cudaStream_t s);
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s);
+// The texture of the context's mirror for volumes of this storage, and the
+// mirror (allocated on first use; nullptr as above, or without memory).
+const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, float **mirror);
+const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, unsigned short **mirror);
 // How the correction projector runs on volumes of one storage: a tuned context's
 // choices; untuned, tld4 corners and no view staged where the textures bind
 // (FP_DEFAULT_TEX), else load variant 0 with the oblique views staged.

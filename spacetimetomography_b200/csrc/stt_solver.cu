@@ -100,7 +100,8 @@ struct stt_solver {
     long long launches_per_iter = 0;
     long long phase_launches[2] = {0, 0};
     std::vector<stt::FpSlabMaps> fpmaps;  // batched modes: per frame, TMA maps of the volume and its copy
-    std::vector<stt::FpTex> fptex;  // batched modes, a tld4 gather form: per frame, the volume's texture
+    std::vector<stt::FpTex> fptex;  // batched modes, a tld4 gather form: per frame, the volume's or its mirror's texture
+    void *mirror = nullptr;         // F mirrors (launch_mirror) where a frame's volume does not bind itself
     stt::FpChoice fp{};             // batched modes: the projector's form
     stt::SweepJob *jobs_d = nullptr;  // STT_SOLVE_PERSISTENT: one job per frame
     unsigned *sweep_bar = nullptr;    // the jobs' barrier and ticket words (4 per frame), then the grid's
@@ -226,6 +227,11 @@ stt_status enqueue_sart_batched(stt_solver *s, int f, cudaStream_t cs, long long
     float *corr = s->corr + f * s->npix;
     const T *stack = reinterpret_cast<const T *>(s->st.proj) + (size_t)f * V * s->npix;
     const int voxel = s->cfg.bp_mode == 0;
+    T *mirror = s->mirror ? reinterpret_cast<T *>(s->mirror) + f * stt::fp_mirror_stride((size_t)g.nx * g.ny, g.nz) : nullptr;
+    if (mirror) {  // (the primal step has just written the volume)
+        SCUDA(s, stt::launch_mirror(g, static_cast<const T *>(vol), mirror, cs), "mirror");
+        ++nl;
+    }
     T *volt = s->volt ? reinterpret_cast<T *>(s->volt) + f * s->n : nullptr;  // none: no view gathers from a copy
     for (int i = 0; i < V; ++i) {
         const stt::ViewSel sel{0, s->perm + (size_t)f * V, i, f * V};
@@ -238,13 +244,17 @@ stt_status enqueue_sart_batched(stt_solver *s, int f, cudaStream_t cs, long long
         SCUDA(s, e, "fp_corr");
         if (voxel)
             SCUDA(s, stt::launch_bp_voxel(g, s->views, sel, corr, vol, (float)s->cfg.alpha, s->cfg.pd.gmax, cs,
-                                          s->ctx->tuning.bp),
+                                          s->ctx->tuning.bp, mirror),
                   "bp_voxel");
         else
             SCUDA(s, stt::launch_bp_ray(g, s->views, sel, corr, s->acc + f * s->n, vol, s->cfg.pd.gmax, cs,
                                         s->ctx->tuning.ray),
                   "bp_ray");
         nl += voxel ? 1 : 2;
+        if (!voxel && mirror && i + 1 < V) {
+            SCUDA(s, stt::launch_mirror(g, static_cast<const T *>(vol), mirror, cs), "mirror");
+            ++nl;
+        }
     }
     const int d[3] = {g.nx, g.ny, g.nz};
     SCUDA(s, stt::launch_roi_apply(d, s->cfg.roi_cut, s->cfg.pd.cut, vol, vol_of<T>(s, s->st.xprev, f),
@@ -580,12 +590,34 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
         auto choice = [&](bool binds) {
             return f32 ? stt::fp_choice(ctx, s->st.vol, binds) : stt::fp_choice(ctx, vol16, binds);
         };
-        bool binds = choice(true).tex;
+        bool binds = choice(true).tex, itself = true;
         if (binds) {
-            s->fptex.resize(F);
-            for (int f = 0; f < F && binds; ++f)
-                binds = f32 ? stt::make_fp_tex(*g, s->st.vol + f * s->n, s->fptex[f])
-                            : stt::make_fp_tex(*g, vol16 + f * s->n, s->fptex[f]);
+            const int es = f32 ? 4 : 2;
+            const size_t slice = (size_t)g->nx * g->ny, pitch = stt::fp_mirror_pitch(slice);
+            const size_t mn = stt::fp_mirror_stride(slice, g->nz);
+            for (int f = 0; f < F; ++f)
+                itself &= stt::fp_tex_fits(*g, reinterpret_cast<const char *>(s->st.vol) + f * s->n * es, es);
+            if (!itself) binds = stt::fp_tex_fits(*g, reinterpret_cast<const void *>((uintptr_t)4096), es, pitch);
+            if (binds && !itself) {
+                unsigned char *m = nullptr;
+                if ((e = alloc(s, m, (size_t)F * mn * es, "mirrors"))) {
+                    stt_solver_destroy(s);
+                    return e;
+                }
+                s->mirror = m;
+            }
+            const float *base = itself ? s->st.vol : static_cast<const float *>(s->mirror);
+            const unsigned short *base16 = reinterpret_cast<const unsigned short *>(base);
+            if (binds) s->fptex.resize(F);
+            for (int f = 0; f < F && binds; ++f) {
+                const size_t o = f * (itself ? s->n : mn);
+                binds = f32 ? stt::make_fp_tex(*g, base + o, s->fptex[f], itself ? 0 : pitch)
+                            : stt::make_fp_tex(*g, base16 + o, s->fptex[f], itself ? 0 : pitch);
+            }
+            if (!binds) {
+                cudaFree(s->mirror);
+                s->mirror = nullptr;
+            }
         }
         s->fp = choice(binds);
     }
@@ -824,6 +856,7 @@ stt_status stt_solver_destroy(stt_solver *s) {
     cudaFree(s->corr);
     cudaFree(s->ax);
     cudaFree(s->volt);
+    cudaFree(s->mirror);
     cudaFree(s->raylen);
     cudaFree(s->acc);
     cudaFree(s->perm);

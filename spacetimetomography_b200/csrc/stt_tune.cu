@@ -51,7 +51,7 @@ std::string shape_key(const stt_ctx *ctx) {
 
 // Device scratch of one tuning run, released on every return path.
 struct Scratch {
-    float *vol = nullptr, *volt = nullptr, *b = nullptr, *rl = nullptr, *corr = nullptr;
+    float *vol = nullptr, *volt = nullptr, *b = nullptr, *rl = nullptr, *corr = nullptr, *mirror = nullptr;
     float2 *acc = nullptr;
     unsigned short *vol16 = nullptr, *volt16 = nullptr, *b16 = nullptr;  // BF16 copies for the BF16 choice
     stt::ViewRec *tv = nullptr;
@@ -63,6 +63,7 @@ struct Scratch {
         stt::destroy_fp_tex(fptex16);
         cudaFree(vol);
         cudaFree(volt);
+        cudaFree(mirror);
         cudaFree(b);
         cudaFree(rl);
         cudaFree(corr);
@@ -119,24 +120,73 @@ stt_status apply_staged_bins(stt_ctx *ctx) {
 }
 
 namespace {
+// While a stream is captured nothing is allocated or created for it: the call
+// takes the form that needs neither.
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
 template <typename T>
-const FpTex *cached_tex(stt_ctx *ctx, const T *vol) {
+const FpTex *cached_tex(stt_ctx *ctx, const T *vol, cudaStream_t s) {
     const GeomDev &g = ctx->g;
     const int es = (int)sizeof(T);
+    if (!fp_tex_fits(g, vol, es)) return nullptr;
     for (const auto &e : ctx->fp_tex)
         if (e.vol == vol && e.nx == g.nx && e.ny == g.ny && e.nz == g.nz && e.esize == es)
             return e.tex.ok ? &e.tex : nullptr;
-    if ((int)ctx->fp_tex.size() >= stt_ctx::kFpTexCache) return nullptr;
+    if ((int)ctx->fp_tex.size() >= stt_ctx::kFpTexCache || capturing(s)) return nullptr;
     stt_ctx::FpTexEntry e{vol, g.nx, g.ny, g.nz, es, FpTex{}};
     make_fp_tex(g, vol, e.tex);  // where it fails, tex.ok = 0 is cached too: the loads run
     ctx->fp_tex.push_back(e);
     return ctx->fp_tex.back().tex.ok ? &ctx->fp_tex.back().tex : nullptr;
 }
+
+template <typename T>
+const FpTex *mirror_tex(stt_ctx *ctx, cudaStream_t s, T **mirror) {
+    const GeomDev &g = ctx->g;
+    stt_ctx::Mirror &m = ctx->mirror[sizeof(T) == 2];
+    if (m.nx != g.nx || m.ny != g.ny || m.nz != g.nz) {
+        const size_t pitch = fp_mirror_pitch((size_t)g.nx * g.ny), bytes = pitch * g.nz * sizeof(T);
+        // (a base as aligned as cudaMalloc's: whether the mirror's own texture would bind)
+        if (capturing(s) || !fp_tex_fits(g, reinterpret_cast<const void *>((uintptr_t)4096), (int)sizeof(T), pitch))
+            return nullptr;
+        // another size: launches enqueued earlier (on any stream) may still gather
+        // from the old texture, so the device drains before it goes
+        if (m.p && cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+        destroy_fp_tex(m.tex);
+        m.nx = m.ny = m.nz = 0;
+        if (m.bytes < bytes) {
+            cudaFree(m.p);
+            m.p = nullptr;
+            m.bytes = 0;
+            if (cudaMalloc(&m.p, bytes) != cudaSuccess) {
+                cudaGetLastError();
+                m.p = nullptr;
+                return nullptr;
+            }
+            m.bytes = bytes;
+        }
+        m.nx = g.nx, m.ny = g.ny, m.nz = g.nz;
+        make_fp_tex(g, static_cast<const T *>(m.p), m.tex, pitch);
+    }
+    if (!m.tex.ok) return nullptr;
+    *mirror = static_cast<T *>(m.p);
+    return &m.tex;
+}
 }  // namespace
 
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol) { return cached_tex(ctx, vol); }
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol, cudaStream_t s) { return cached_tex(ctx, vol, s); }
 
-const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol) { return cached_tex(ctx, vol); }
+const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s) { return cached_tex(ctx, vol, s); }
+
+const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, float **mirror) { return mirror_tex(ctx, s, mirror); }
+
+const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, unsigned short **mirror) { return mirror_tex(ctx, s, mirror); }
 
 FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds) {
     if (ctx->tuned) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), ctx->staged_bins != 0};
@@ -277,7 +327,15 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
         const int b = stt::off_axis_bin(ctx->off_axis_deg[v]);
         if (ctx->views_h[v].layout == 1) along_x[b] += 1.0f / (float)count[b];
     }
-    stt::make_fp_tex(g, sc.vol, sc.fptex);  // where it fails, ok = 0 and the tld4 variants are skipped
+    if (!stt::make_fp_tex(g, sc.vol, sc.fptex)) {  // through a mirror, as the sweeps do
+        const size_t pitch = stt::fp_mirror_pitch((size_t)g.nx * g.ny);
+        if (stt::fp_tex_fits(g, reinterpret_cast<const void *>((uintptr_t)4096), 4, pitch)) {
+            if ((e = cudaMalloc(&sc.mirror, pitch * g.nz * sizeof(float))) ||
+                (e = stt::launch_mirror(g, sc.vol, sc.mirror, s)))
+                return fail(e, "mirror");
+            stt::make_fp_tex(g, sc.mirror, sc.fptex, pitch);
+        }
+    }  // where it fails, ok = 0 and the tld4 variants are skipped
     for (int b = 0; b < 9; ++b) {
         if (rep[b] < 0) continue;
         stt::ViewRec two[2] = {ctx->views_h[rep[b]], ctx->views_h[rep[b]]};
@@ -378,7 +436,9 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
             (e = cudaMemsetAsync(sc.volt16, 0x3F, n * sizeof(unsigned short), s)) ||
             (e = cudaMemsetAsync(sc.b16, 0, npix * sizeof(unsigned short), s)))
             return fail(e, "BF16 scratch");
-        stt::make_fp_tex(g, sc.vol16, sc.fptex16);  // where it fails, ok = 0: loads only
+        if (!stt::make_fp_tex(g, sc.vol16, sc.fptex16) && sc.mirror)
+            stt::make_fp_tex(g, reinterpret_cast<const unsigned short *>(sc.mirror), sc.fptex16,
+                             stt::fp_mirror_pitch((size_t)g.nx * g.ny));  // where it fails, ok = 0: loads only
         stt::FpSlabMaps m16;
         const bool maps16 = stt::make_fp_slab_maps(g, sc.vol16, sc.volt16, m16, t.slab_variant);
         float tg16[stt::kFp16Variants][9] = {}, ts16[9] = {};

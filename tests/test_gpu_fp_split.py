@@ -2,7 +2,8 @@
 bit: views of few rays (each ray shared between the warps of a block), the
 boundary between the two texture forms, ragged detectors, rays that miss, the
 march's restart before the entry (a non-zero boundary, an off-centre volume),
-both storages, and the volumes no texture binds.  A context's default choice,
+both storages, volumes projected from a mirror (their slices are not aligned) and
+volumes no texture takes.  A context's default choice,
 each tuned variant and the slab-staged kernel with textures beside it agree."""
 import numpy as np
 import pytest
@@ -17,7 +18,10 @@ CASES = [  # dims, detector, spacing, offset
     ((16, 8, 12), (90, 71), 1.0, (0.0, 0.0, 0.0)),        # most rays miss
     ((48, 40, 44), (192, 128), 1.0, (0.5, -0.3, 0.2)),    # 24576 rays: the last shared view
     ((48, 40, 44), (193, 128), 1.0, (0.5, -0.3, 0.2)),    # the first that is not
-    ((33, 17, 21), (40, 37), 1.0, (0.0, 0.0, 0.0)),       # no texture binds: its slices are not aligned
+    ((33, 17, 21), (40, 37), 1.0, (0.0, 0.0, 0.0)),       # unaligned slices: through a mirror
+    ((2, 2, 2), (40, 37), 1.0, (0.0, 0.0, 0.0)),
+    ((30, 31, 29), (200, 160), 1.0, (0.3, 0.0, 0.0)),     # a mirror, and rays past the shared views
+    ((1024, 130, 6), (64, 40), 1.0, (0.0, 0.0, 0.0)),     # slices past the texture width: loads
 ]
 ANGLES = np.array([0.0, 0.05, 0.5, 0.785, 1.3, np.pi / 2, 2.36, 3.3, 4.4, 5.5])
 
@@ -84,3 +88,51 @@ def test_texture_forms_equal_loads(cuda, case, storage):
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
     ctx.close()
     load.close()
+
+
+@pytest.mark.parametrize("storage", ["f32", "bf16"])
+@pytest.mark.parametrize("bp_mode", [0, 1])
+def test_solver_frames_through_mirrors(cuda, storage, bp_mode):
+    """Two frames of unaligned slices: the projector's default form (each frame's
+    mirror kept current by the backprojection) against loads.  Voxel
+    backprojection bit for bit; ray backprojection within the reordering of its
+    float atomics."""
+    import torch
+
+    import spacetimetomography_b200 as stt
+
+    F, V, dims, det = 2, 7, (29, 27, 31), (44, 40)
+    nx, ny, nz = dims
+    W, H = det
+    g = torch.Generator(device=cuda)
+    g.manual_seed(3)
+    rand = lambda *s: torch.rand(s, device=cuda, generator=g)  # noqa: E731
+    vol, proj = rand(F + 1, nz, ny, nx), rand(F, V, H, W) * 20
+    flow = (rand(F, 3, nz, ny, nx) - 0.5) * 2
+    cut = (3, 3, 3, 5, 3, 3, 6, 5)
+    outs = []
+    for tuned in (False, True):
+        ctx = stt.Context(0)
+        ctx.set_geometry(dims, (1.0, 1.0, 1.0), det, 1.0, 600.0, 1000.0, np.arange(F * V) * 0.7, (0.0, 0.0, 0.0))
+        if tuned:
+            ctx.set_tuning(0, 0, 0, staged_bins=0, fp_variant_bf16=0)
+        z = lambda *s: torch.zeros(s, device=cuda)  # noqa: E731
+        st = dict(vol=vol.clone(), xbar=vol.clone(), xprev=z(F, nz, ny, nx), ytv=z(F, 3, nz, ny, nx),
+                  ytp=z(F, nz, ny, nx), ybc=z(F, nz, ny, nx), flow=flow, proj=proj)
+        if storage == "bf16":
+            for k in ("vol", "xbar", "xprev", "proj"):
+                st[k] = st[k].to(torch.bfloat16)
+        s = stt.Solver(ctx, st, F, V, stt.PdParams(gmax=5.0, cut=cut), bp_mode=bp_mode, roi_cut=cut, seed=5,
+                       storage=storage)
+        s.iterate(2)
+        torch.cuda.synchronize()
+        s.poll_status()
+        outs.append({k: st[k].float().cpu().numpy() for k in ("vol", "xbar", "xprev", "ytv", "ytp", "ybc")})
+        s.close()
+        ctx.close()
+    for k in outs[0]:
+        if bp_mode == 0:
+            np.testing.assert_array_equal(outs[0][k], outs[1][k], err_msg=k)
+        else:
+            scale = np.linalg.norm(outs[1][k])
+            assert np.linalg.norm(outs[0][k] - outs[1][k]) <= (1e-2 if storage == "bf16" else 1e-4) * scale, k
