@@ -410,16 +410,16 @@ typedef struct stt_flow_params {
 typedef struct stt_flow stt_flow;
 
 /* Allocates every buffer of a multiscale solve for volumes of size dims
- * (HOST int[3]) on `device`: about 200 bytes per voxel. */
+ * (HOST int[3]) on `device`: about 320 bytes per voxel. */
 stt_status stt_flow_create(int device, const int *dims, const stt_flow_params *p, stt_flow **out);
 const char *stt_flow_last_error(const stt_flow *f);
 stt_status stt_flow_destroy(stt_flow *f);
 /* L1Huber_OF_MultiScale3D: V holds the initial flow and receives the
  * finest-level flow; Y0 (10 planes, NULL = zeros) is the initial dual.
  * This and stt_flow_level enqueue their work on `stream`; to stop enqueuing a
- * warp's iterations once its residual check has stopped it, they keep at most
- * 200 of a warp's iterations queued ahead of the device and wait for it
- * (an event of `stream`) past that.  While `stream` is being captured every
+ * warp's iterations once its residual check has stopped it, they queue at most
+ * 16 iterations past a check and then wait for its outcome (an event of
+ * `stream`).  While `stream` is being captured every
  * iteration is enqueued and nothing waits. */
 stt_status stt_flow_multiscale(stt_flow *f, const float *I1, const float *I2, float *V, const float *Y0,
                                void *stream);

@@ -11,12 +11,11 @@
 // the flow reproduces the reference's CPU result bit for bit (the residual
 // sums, which the reference accumulates in a racy loop, are the exception).
 //
-// Layout: planar x-fastest fields, idx = x + y*nx + z*nx*ny, channel planes of
-// n = nx*ny*nz floats (CImg's layout).  Dual field y: 10 planes Y1|Y2|Y3|Y4.
-// Per iteration the primal step reads y, u, tau and the flow and writes the
-// next flow into a second buffer; the dual step reads both flows (K v and
-// K v_old), u and sigma2 and updates y in place: 53 floats per voxel instead
-// of the 70 of the reference's layout, which also stores K v (10 floats).
+// Layout: the caller's fields are planar and x-fastest, idx = x + y*nx +
+// z*nx*ny, channel planes of n = nx*ny*nz floats (CImg's layout; dual field y: 10
+// planes Y1|Y2|Y3|Y4).  The iterations work on vectors per voxel (FlowVec below),
+// packed when a level starts.  Between residual checks one kernel runs the dual
+// step of an iteration and the primal step of the next (k_flow_step).
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
@@ -145,15 +144,16 @@ __global__ void __launch_bounds__(128) k_warp_box(const Dims d, const float bx, 
 // its K v_old (the reference keeps Kx across warps, optical_flow.h:246, 394).
 __global__ void __launch_bounds__(128) k_flow_setup(const Dims d, const FlowRoi roi, const float *__restrict__ i2w,
                                                     const float *__restrict__ i1, const float *__restrict__ v,
-                                                    float *__restrict__ u, float *__restrict__ tau,
-                                                    float *__restrict__ sig2, float *__restrict__ k4prev) {
+                                                    float4 *__restrict__ u, float4 *__restrict__ steps,
+                                                    float *__restrict__ k4prev) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
     if (i >= d.x) return;
     const long long sy = d.x, sz = (long long)d.x * d.y, n = sz * d.z;
     const long long p = i + j * sy + k * sz;
     const float v1 = __ldg(v + p), v2 = __ldg(v + n + p), v3 = __ldg(v + 2 * n + p);
-    k4prev[p] = u[p] * v1 + u[n + p] * v2 + u[2 * n + p] * v3;
+    const float4 up = u[p];
+    k4prev[p] = up.x * v1 + up.y * v2 + up.z * v3;
     float ux = 0.0f, uy = 0.0f, uz = 0.0f, ut = 0.0f;
     if (in_roi(roi, d, i, j, k)) {
         const long long xm = i > 0 ? p - 1 : p, xp = i < d.x - 1 ? p + 1 : p;
@@ -164,14 +164,47 @@ __global__ void __launch_bounds__(128) k_flow_setup(const Dims d, const FlowRoi 
         uz = (__ldg(i2w + zp) - __ldg(i2w + zm)) / 2;
         ut = __ldg(i2w + p) - __ldg(i1 + p) - ux * v1 - uy * v2 - uz * v3;
     }
-    u[p] = ux;
-    u[n + p] = uy;
-    u[2 * n + p] = uz;
-    u[3 * n + p] = ut;
-    tau[p] = 1.0f / (4.0f / 1.0f + fabsf(ux));
-    tau[n + p] = 1.0f / (4.0f / 1.0f + fabsf(uy));
-    tau[2 * n + p] = 1.0f / (4.0f / 1.0f + fabsf(uz));
-    sig2[p] = 1.0f / (fabsf(ux) + fabsf(uy) + fabsf(uz));
+    u[p] = make_float4(ux, uy, uz, ut);
+    steps[p] = make_float4(1.0f / (4.0f / 1.0f + fabsf(ux)), 1.0f / (4.0f / 1.0f + fabsf(uy)),
+                           1.0f / (4.0f / 1.0f + fabsf(uz)), 1.0f / (fabsf(ux) + fabsf(uy) + fabsf(uz)));
+}
+
+// The iterations' fields, a vector per voxel: a planar field costs a load and
+// an address per float, and the step's 42 loads' addresses were most of its
+// instructions.  v: (v1, v2, v3, unused) float4; u: (ux, uy, uz, ut); steps: (tau1,
+// tau2, tau3, sigma2); y: n float4 (Y1x, Y1y, Y1z, Y2x), n float4 (Y2y, Y2z, Y3x,
+// Y3y), n float2 (Y3z, Y4), one after the other.
+struct Dual {
+    float y[10];
+};
+__device__ __forceinline__ float4 ld4(const float4 *p) { return __ldg(p); }
+__device__ __forceinline__ Dual load_dual(const float *y, unsigned n, unsigned p) {
+    const float4 *ya = reinterpret_cast<const float4 *>(y), *yb = ya + n;
+    const float4 a = ld4(ya + p), b = ld4(yb + p);
+    const float2 c = __ldg(reinterpret_cast<const float2 *>(yb + n) + p);
+    return Dual{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y}};
+}
+__device__ __forceinline__ void store_dual(float *y, unsigned n, unsigned p, const float yn[9], float y4) {
+    float4 *ya = reinterpret_cast<float4 *>(y), *yb = ya + n;
+    ya[p] = make_float4(yn[0], yn[1], yn[2], yn[3]);
+    yb[p] = make_float4(yn[4], yn[5], yn[6], yn[7]);
+    reinterpret_cast<float2 *>(yb + n)[p] = make_float2(yn[8], y4);
+}
+__device__ __forceinline__ void spread(const float4 &a, float o[3]) { o[0] = a.x, o[1] = a.y, o[2] = a.z; }
+
+// Start of a level: the caller's dual and flow packed; the flow into all three
+// buffers (outside the ROI it is never updated).
+__global__ void __launch_bounds__(256) k_flow_pack(unsigned n, const float *__restrict__ Y, const float *__restrict__ V,
+                                                   float *__restrict__ y, float4 *__restrict__ v0,
+                                                   float4 *__restrict__ v1, float4 *__restrict__ v2) {
+    const unsigned p = blockIdx.x * 256 + threadIdx.x;
+    if (p >= n) return;
+    float q[10];
+#pragma unroll
+    for (int c = 0; c < 10; ++c) q[c] = __ldg(Y + (size_t)c * n + p);
+    store_dual(y, n, p, q, q[9]);
+    v0[p] = v1[p] = v2[p] =
+        make_float4(__ldg(V + p), __ldg(V + (size_t)n + p), __ldg(V + (size_t)2 * n + p), 0.0f);
 }
 
 // Backward difference of S/ImageFormationModel/tools.cpp:146-192 (dxm3, dym3,
@@ -200,13 +233,20 @@ __device__ __forceinline__ void add_resid(double *resid, float r) {
 // Offsets inside one level are 32-bit: the host keeps 10 * voxels < 2^31.
 // Every load of a voxel's neighbourhood is issued before the arithmetic.
 
+// K^T y at one voxel (optical_flow.h:329-345): a: its dual, b: the lower
+// neighbours' components (x, y, z of each flow component), u: the gradient.
+__device__ __forceinline__ float kty_of(const float a[3], const float b[3], int i, int j, int k, const Dims &d, float u,
+                                        float y4) {
+    // -stepsizeD * dxm3 - ... with unit step sizes: (-1 * x) == -x and 1 * x == x exactly
+    return -dm(a[0], b[0], i, d.x) - dm(a[1], b[1], j, d.y) - dm(a[2], b[2], k, d.z) + u * y4;
+}
+
 // Primal step over the ROI (optical_flow.h:314-370):
 // Kty_c = -div_b(y_c) + u_c*y4; v_c -= tau_c*Kty_c, read from v_in and
-// written to v_out (the dual step needs both).  Outside the ROI v_in and
-// v_out hold the same, never-updated values.
+// written to v_out (the dual step needs both).
 __global__ void __launch_bounds__(128) k_flow_primal(const Dims d, const FlowRoi roi, const float *__restrict__ y,
-                                                     const float *__restrict__ u, const float *__restrict__ tau,
-                                                     const float *__restrict__ v_in, float *__restrict__ v_out,
+                                                     const float4 *__restrict__ u, const float4 *__restrict__ steps,
+                                                     const float4 *__restrict__ v_in, float4 *__restrict__ v_out,
                                                      float *__restrict__ kty, int flags, double *__restrict__ resid,
                                                      const int *__restrict__ done) {
     if (*done) return;
@@ -214,40 +254,59 @@ __global__ void __launch_bounds__(128) k_flow_primal(const Dims d, const FlowRoi
     const int j = blockIdx.y, k = blockIdx.z;
     float pr = 0.0f;
     if (i < d.x && in_roi(roi, d, i, j, k)) {
-        const int sy = d.x, sz = d.x * d.y, n = sz * d.z;
-        const long long p = i + (long long)j * sy + (long long)k * sz;
-        const float *yp = y + p;
-        const int ox = i > 0 ? 1 : 0, oy = j > 0 ? sy : 0, oz = k > 0 ? sz : 0;
-        float a[9], b[9];
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            const int off = q * n, st = (q % 3 == 0) ? ox : (q % 3 == 1 ? oy : oz);
-            a[q] = __ldg(yp + off);
-            b[q] = __ldg(yp + off - st);
-        }
-        const float y4 = __ldg(yp + 9 * n);
-        float uc[3], vo[3], t[3];
+        const unsigned sy = d.x, sz = d.x * d.y, n = sz * d.z;
+        const unsigned p = i + j * sy + k * sz;
+        const Dual a = load_dual(y, n, p), bx = load_dual(y, n, i > 0 ? p - 1 : p);
+        const Dual by = load_dual(y, n, j > 0 ? p - sy : p), bz = load_dual(y, n, k > 0 ? p - sz : p);
+        const float4 up = ld4(u + p), vp = ld4(v_in + p), sp = ld4(steps + p);
+        float uc[3], vo[3], t[3], vn[3];
+        spread(up, uc), spread(vp, vo), spread(sp, t);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            uc[c] = __ldg(u + p + c * n);
-            vo[c] = __ldg(v_in + p + c * n);
-            t[c] = __ldg(tau + p + c * n);
-        }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            // -stepsizeD * dxm3 - ... with unit step sizes: (-1 * x) == -x and 1 * x == x exactly
-            const float kt = -dm(a[3 * c], b[3 * c], i, d.x) - dm(a[3 * c + 1], b[3 * c + 1], j, d.y) -
-                             dm(a[3 * c + 2], b[3 * c + 2], k, d.z) + uc[c] * y4;
-            const float vn = vo[c] - t[c] * kt;
-            v_out[p + c * n] = vn;
+            const float b[3] = {bx.y[3 * c], by.y[3 * c + 1], bz.y[3 * c + 2]};
+            const float kt = kty_of(a.y + 3 * c, b, i, j, k, d, uc[c], a.y[9]);
+            vn[c] = vo[c] - t[c] * kt;
             if (flags & kResid) {
-                const float r = fabsf((vo[c] - vn) / t[c] - kty[p + c * n] + kt);
+                const float r = fabsf((vo[c] - vn[c]) / t[c] - kty[p + (size_t)c * n] + kt);
                 pr = c == 0 ? r : pr + r;
             }
-            if (flags & kKeepKty) kty[p + c * n] = kt;
+            if (flags & kKeepKty) kty[p + (size_t)c * n] = kt;
         }
+        v_out[p] = make_float4(vn[0], vn[1], vn[2], 0.0f);
     }
     if (flags & kResid) add_resid(resid, pr);
+}
+
+// Constants of the dual step; lam2_lo: a bound just below lambda^2.
+struct DualPar {
+    float sigma1, hf, lambda, lam2_lo;
+    int huber;
+};
+
+// One flow component's dual (optical_flow.h:394-470): the ascent
+// yo + sigma1 (2 K v - K v_old), scaled by the Huber factor, projected onto the
+// lambda-ball.
+__device__ __forceinline__ void dual_channel(const float yo[3], const float kn[3], const float ko[3], const DualPar &q,
+                                             float yn[3]) {
+    float yt[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float t = yo[a] + q.sigma1 * (kn[a] + kn[a] - ko[a]);
+        yt[a] = q.huber ? t * q.hf : t;
+    }
+    // divisor = max(1, sqrt(s)/lambda) and y = yt/divisor.  Below lam2_lo
+    // (< lambda^2 with margin) sqrt(s) rounds below lambda, so the divisor is
+    // exactly 1 and y = yt exactly: skip the sqrt and the divisions.
+    const float ss = yt[0] * yt[0] + yt[1] * yt[1] + yt[2] * yt[2];
+    yn[0] = yt[0], yn[1] = yt[1], yn[2] = yt[2];
+    if (!(ss < q.lam2_lo)) {
+        const float div = smax(1.0f, sqrtf(ss) / q.lambda);
+        if (div != 1.0f) {
+            yn[0] = yt[0] / div;
+            yn[1] = yt[1] / div;
+            yn[2] = yt[2] / div;
+        }
+    }
 }
 
 // Dual step over every voxel (optical_flow.h:374-497): K v by forward
@@ -256,100 +315,166 @@ __global__ void __launch_bounds__(128) k_flow_primal(const Dims d, const FlowRoi
 // lambda-ball; y4 clamped to [-1, 1].  K v_old, which the reference stores
 // (10 floats per voxel), is recomputed here from v_old with the same float
 // operations, so it is the same value.
-__global__ void __launch_bounds__(128) k_flow_dual(const Dims d, const float *__restrict__ v,
-                                                   const float *__restrict__ v_old, const float *__restrict__ u,
-                                                   const float *__restrict__ sig2, const float *__restrict__ k4prev,
-                                                   float *__restrict__ y, float sigma1, float hf, float lambda,
-                                                   float lam2_lo, int huber, int flags, double *__restrict__ resid,
-                                                   const int *__restrict__ done) {
+__global__ void __launch_bounds__(128) k_flow_dual(const Dims d, const float4 *__restrict__ v,
+                                                   const float4 *__restrict__ v_old, const float4 *__restrict__ u,
+                                                   const float4 *__restrict__ steps, const float *__restrict__ k4prev,
+                                                   float *__restrict__ y, const DualPar q, int flags,
+                                                   double *__restrict__ resid, const int *__restrict__ done) {
     if (*done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
     float dr = 0.0f;
     if (i < d.x) {
-        const int sy = d.x, sz = d.x * d.y, n = sz * d.z;
-        const long long p = i + (long long)j * sy + (long long)k * sz;
-        const int ox = i < d.x - 1 ? 1 : 0, oy = j < d.y - 1 ? sy : 0, oz = k < d.z - 1 ? sz : 0;
+        const unsigned sy = d.x, sz = d.x * d.y, n = sz * d.z;
+        const unsigned p = i + j * sy + k * sz;
+        const unsigned ox = i < d.x - 1 ? 1 : 0, oy = j < d.y - 1 ? sy : 0, oz = k < d.z - 1 ? sz : 0;
         const bool zero_old = flags & kFirstOfLevel;
-        const float *vp = v + p, *op = v_old + p;
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         float vc[3], vx[3], vy[3], vz[3], oc[3], oxv[3], oyv[3], ozv[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const int off = c * n;
-            vc[c] = __ldg(vp + off);
-            vx[c] = __ldg(vp + off + ox);
-            vy[c] = __ldg(vp + off + oy);
-            vz[c] = __ldg(vp + off + oz);
-            if (!zero_old) {
-                oc[c] = __ldg(op + off);
-                oxv[c] = __ldg(op + off + ox);
-                oyv[c] = __ldg(op + off + oy);
-                ozv[c] = __ldg(op + off + oz);
-            }
-        }
-        float *yp = y + p;
-        float yo[10];
-#pragma unroll
-        for (int q = 0; q < 10; ++q) yo[q] = yp[q * n];
-        const float u1 = __ldg(u + p), u2 = __ldg(u + p + n), u3 = __ldg(u + p + 2 * n), ut = __ldg(u + p + 3 * n);
-        const float s2 = __ldg(sig2 + p);
+        spread(ld4(v + p), vc), spread(ld4(v + p + ox), vx), spread(ld4(v + p + oy), vy), spread(ld4(v + p + oz), vz);
+        spread(zero_old ? zero : ld4(v_old + p), oc), spread(zero_old ? zero : ld4(v_old + p + ox), oxv);
+        spread(zero_old ? zero : ld4(v_old + p + oy), oyv), spread(zero_old ? zero : ld4(v_old + p + oz), ozv);
+        const float4 *ya = reinterpret_cast<const float4 *>(y), *yb = ya + n;
+        const float4 y0 = ya[p], y1 = yb[p];
+        const float2 y2 = reinterpret_cast<const float2 *>(yb + n)[p];
+        const float yo[10] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w, y2.x, y2.y};
+        const float4 up = ld4(u + p);
+        const float s2 = ld4(steps + p).w;
+        float yn[9];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             // K v with unit step sizes (stepsizeD = 1: x * 1.0f == x, dropped)
             const float kn[3] = {dp(vc[c], vx[c], i, d.x), dp(vc[c], vy[c], j, d.y), dp(vc[c], vz[c], k, d.z)};
-            float ko[3] = {0.0f, 0.0f, 0.0f};
-            if (!zero_old) {
-                ko[0] = dp(oc[c], oxv[c], i, d.x);
-                ko[1] = dp(oc[c], oyv[c], j, d.y);
-                ko[2] = dp(oc[c], ozv[c], k, d.z);
-            }
-            float yt[3];
+            const float ko[3] = {dp(oc[c], oxv[c], i, d.x), dp(oc[c], oyv[c], j, d.y), dp(oc[c], ozv[c], k, d.z)};
+            dual_channel(yo + 3 * c, kn, ko, q, yn + 3 * c);
+            if (flags & kResid) {
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                const float t = yo[3 * c + a] + sigma1 * (kn[a] + kn[a] - ko[a]);
-                yt[a] = huber ? t * hf : t;
-            }
-            // divisor = max(1, sqrt(s)/lambda) and y = yt/divisor.  Below
-            // lam2_lo (< lambda^2 with margin) sqrt(s) rounds below lambda, so
-            // the divisor is exactly 1 and y = yt exactly: skip the sqrt and
-            // the divisions.
-            const float ss = yt[0] * yt[0] + yt[1] * yt[1] + yt[2] * yt[2];
-            float yn[3] = {yt[0], yt[1], yt[2]};
-            if (!(ss < lam2_lo)) {
-                const float div = smax(1.0f, sqrtf(ss) / lambda);
-                if (div != 1.0f) {
-                    yn[0] = yt[0] / div;
-                    yn[1] = yt[1] / div;
-                    yn[2] = yt[2] / div;
-                }
-            }
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                yp[(3 * c + a) * n] = yn[a];
-                if (flags & kResid) {
-                    const float r = fabsf((yo[3 * c + a] - yn[a]) / sigma1 - ko[a] + kn[a]);
+                for (int a = 0; a < 3; ++a) {
+                    const float r = fabsf((yo[3 * c + a] - yn[3 * c + a]) / q.sigma1 - ko[a] + kn[a]);
                     dr = (c == 0 && a == 0) ? r : dr + r;
                 }
             }
         }
-        const float k4 = u1 * vc[0] + u2 * vc[1] + u3 * vc[2];
+        const float k4 = up.x * vc[0] + up.y * vc[1] + up.z * vc[2];
         float k4o = 0.0f;
         if (flags & kFirstOfWarp) k4o = __ldg(k4prev + p);
-        else if (!zero_old) k4o = u1 * oc[0] + u2 * oc[1] + u3 * oc[2];
-        const float y4 = smax(-1.0f, smin(1.0f, yo[9] + s2 * (k4 + k4 - k4o + ut)));
-        yp[9 * n] = y4;
+        else if (!zero_old) k4o = up.x * oc[0] + up.y * oc[1] + up.z * oc[2];
+        const float y4 = smax(-1.0f, smin(1.0f, yo[9] + s2 * (k4 + k4 - k4o + up.w)));
+        store_dual(y, n, p, yn, y4);
         if (flags & kResid) dr = dr + fabsf((yo[9] - y4) / s2 - k4o + k4);
     }
     if (flags & kResid) add_resid(resid + 1, dr);
 }
 
-// End of a warp: the flow of the last iteration that ran lies in the second
-// buffer when that count is odd; bring it back to the first.
-__global__ void __launch_bounds__(256) k_flow_settle(long long n3, const int *__restrict__ iters,
-                                                     const float *__restrict__ v_b, float *__restrict__ v_a) {
-    if ((*iters & 1) == 0) return;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < n3; q += (long long)gridDim.x * blockDim.x)
-        v_a[q] = v_b[q];
+// The dual step of one iteration and the primal step of the next in one pass
+// (neither a residual iteration): y_in -> y_out and (v, v_old) -> v_next.  The
+// primal step at a voxel needs the new dual at the voxel and one voxel down each
+// axis.  A block owns 31 x STEP_Y columns and walks up z: lane 0 and row 0 are
+// the neighbouring columns' duals, formed here again (and not written); the
+// x neighbour's comes from the lane below, the y neighbour's through shared
+// memory, the z neighbour's from the step before.  The next plane's loads are in
+// flight during the exchange and the stores.  y and v_next have buffers of their
+// own: neighbouring blocks read the old ones.  The operations are the two
+// kernels', so are the bits.
+//
+// An iteration moves 160 bytes per voxel where the two kernels moved 212, in one
+// launch.  Per iteration, two planar kernels -> this, us: 54^3 14.7 -> 8.8, 83^3
+// 23.6 -> 21.5, 128^3 79.1 -> 76.0, 147 x 121 x 135 110.6 -> 88.3, 256^3 606 ->
+// 542 (4.9 TB/s).  Bound by the latency of a plane's chain (loads, duals,
+// exchange) at 20 warps per SM; so small blocks, whose barriers hold fewer warps
+// up, beat the smaller halo of larger ones (STEP_Y 8, two blocks: 80 us at
+// 128^3; 12: 80; 16: 92).  Measured and not kept: planar fields (42 loads and
+// their addresses a voxel: 82), planes through a shared-memory ring by
+// asynchronous copies (83), one component at a time in 72 registers (94).
+constexpr int STEP_Y = 4;
+__global__ void __launch_bounds__(32 * (STEP_Y + 1), 4)
+    k_flow_step(const Dims d, const FlowRoi roi, const float *__restrict__ y_in, float *__restrict__ y_out,
+                const float4 *__restrict__ v, const float4 *__restrict__ v_old, float4 *__restrict__ v_next,
+                const float4 *__restrict__ u, const float4 *__restrict__ steps, const float *__restrict__ k4prev,
+                float *__restrict__ kty, const DualPar q, int flags, int planes, const int *__restrict__ done) {
+    __shared__ float below[2][STEP_Y + 1][3][32];
+    if (*done) return;
+    const int lane = threadIdx.x, row = threadIdx.y;
+    const int i0 = (int)blockIdx.x * 31 + lane - 1, j0 = (int)blockIdx.y * STEP_Y + row - 1;
+    const bool own = lane > 0 && row > 0 && i0 < d.x && j0 < d.y;
+    const int i = min(max(i0, 0), d.x - 1), j = min(max(j0, 0), d.y - 1);
+    const unsigned sy = d.x, sz = d.x * d.y, n = sz * d.z;
+    const unsigned ox = i < d.x - 1 ? 1 : 0, oy = j < d.y - 1 ? sy : 0;
+    const int z0 = blockIdx.z * planes, z1 = min(z0 + planes, d.z);
+    const bool zero_old = flags & kFirstOfLevel;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int k = z0 > 0 ? z0 - 1 : 0;
+    unsigned p = i + j * sy + k * sz;
+    float4 vc = ld4(v + p), oc = zero_old ? zero : ld4(v_old + p), vx, vy, vz, oxv = zero, oyv = zero, ozv = zero, up, sp;
+    float pz[3] = {0.0f, 0.0f, 0.0f};
+    Dual yo;
+    // everything the dual step reads at offset o of plane kk but its own v and v_old
+    auto load = [&](int kk, unsigned o) {
+        const unsigned oz = kk < d.z - 1 ? sz : 0;
+        vx = ld4(v + o + ox), vy = ld4(v + o + oy), vz = ld4(v + o + oz);
+        if (!zero_old) oxv = ld4(v_old + o + ox), oyv = ld4(v_old + o + oy), ozv = ld4(v_old + o + oz);
+        yo = load_dual(y_in, n, o);
+        up = ld4(u + o);
+        sp = ld4(steps + o);
+    };
+    load(k, p);
+    for (int buf = 0; k < z1; ++k, p += sz, buf ^= 1) {
+        const bool mine = own && k >= z0;
+        const bool inside = mine && in_roi(roi, d, i, j, k);
+        float a[3], bx[3], by[3], bz[3], e[3], fx[3], fy[3], fz[3], yn[9], xm[3];
+        spread(vc, a), spread(vx, bx), spread(vy, by), spread(vz, bz);
+        spread(oc, e), spread(oxv, fx), spread(oyv, fy), spread(ozv, fz);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float kn[3] = {dp(a[c], bx[c], i, d.x), dp(a[c], by[c], j, d.y), dp(a[c], bz[c], k, d.z)};
+            const float ko[3] = {dp(e[c], fx[c], i, d.x), dp(e[c], fy[c], j, d.y), dp(e[c], fz[c], k, d.z)};
+            dual_channel(yo.y + 3 * c, kn, ko, q, yn + 3 * c);
+            xm[c] = __shfl_up_sync(0xffffffffu, yn[3 * c], 1);
+            below[buf][row][c][lane] = yn[3 * c + 1];
+        }
+        const float k4 = up.x * a[0] + up.y * a[1] + up.z * a[2];
+        float k4o = 0.0f;
+        if (flags & kFirstOfWarp) k4o = __ldg(k4prev + p);
+        else if (!zero_old) k4o = up.x * e[0] + up.y * e[1] + up.z * e[2];
+        const float y4 = smax(-1.0f, smin(1.0f, yo.y[9] + sp.w * (k4 + k4 - k4o + up.w)));
+        float uc[3], t[3];
+        spread(up, uc), spread(sp, t);
+        vc = vz, oc = ozv;
+        if (k + 1 < z1) load(k + 1, p + sz);  // the next plane's loads fly during the exchange and the stores
+        __syncthreads();  // (the other buffer is read before this plane's barrier, written after it)
+        if (mine) {
+            store_dual(y_out, n, p, yn, y4);
+            if (inside) {
+                float vn[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const float b[3] = {xm[c], below[buf][row - 1][c][lane], pz[c]};
+                    const float kt = kty_of(yn + 3 * c, b, i, j, k, d, uc[c], y4);
+                    vn[c] = a[c] - t[c] * kt;
+                    if (flags & kKeepKty) kty[p + (size_t)c * n] = kt;
+                }
+                v_next[p] = make_float4(vn[0], vn[1], vn[2], 0.0f);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) pz[c] = yn[3 * c + 2];
+    }
+}
+
+// End of a warp: the flow of the last iteration that ran lies in buffer
+// iters % 3; unpack it into the caller's planes, and bring it to the first
+// buffer for the next warp.
+__global__ void __launch_bounds__(256) k_flow_settle(unsigned n, const int *__restrict__ iters,
+                                                     const float4 *__restrict__ v_1, const float4 *__restrict__ v_2,
+                                                     float4 *__restrict__ v_0, float *__restrict__ V) {
+    const unsigned p = blockIdx.x * 256 + threadIdx.x;
+    if (p >= n) return;
+    const int at = *iters % 3;
+    const float4 r = at == 0 ? v_0[p] : ld4((at == 1 ? v_1 : v_2) + p);
+    if (at != 0) v_0[p] = r;
+    V[p] = r.x;
+    V[(size_t)n + p] = r.y;
+    V[(size_t)2 * n + p] = r.z;
 }
 
 // Stopping rule of optical_flow.h:306, 488-491: after a residual iteration
@@ -512,14 +637,17 @@ __global__ void __launch_bounds__(128) k_gradient(const Dims d, const float *__r
     g[2 * n + p] = (__ldg(img + zp) - __ldg(img + zm)) / 2;
 }
 
-// dst = src inside the ROI, nc planes (the write-back of optical_flow.h:503-533).
-__global__ void __launch_bounds__(128) k_copy_roi(const Dims d, int nc, const FlowRoi roi,
-                                                  const float *__restrict__ src, float *__restrict__ dst) {
+// The dual inside the ROI to the caller's planes (the write-back of
+// optical_flow.h:503-533).
+__global__ void __launch_bounds__(128) k_flow_unpack(const Dims d, const FlowRoi roi, const float *__restrict__ y,
+                                                     float *__restrict__ Y) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z % d.z, c = blockIdx.z / d.z;
-    if (i >= d.x || c >= nc || !in_roi(roi, d, i, j, k)) return;
-    const long long p = c * (long long)d.x * d.y * d.z + i + (long long)j * d.x + (long long)k * d.x * d.y;
-    dst[p] = src[p];
+    const int j = blockIdx.y, k = blockIdx.z;
+    if (i >= d.x || !in_roi(roi, d, i, j, k)) return;
+    const unsigned n = d.x * d.y * d.z, p = i + j * d.x + k * d.x * d.y;
+    const Dual q = load_dual(y, n, p);
+#pragma unroll
+    for (int c = 0; c < 10; ++c) Y[(size_t)c * n + p] = q.y[c];
 }
 
 inline dim3 vox_grid(const int *d, int zmul = 1) {
@@ -535,35 +663,71 @@ cudaError_t launch_warp_box(const int *dim, const float *box, const float *vel, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_flow_setup(const int *d, const FlowRoi &roi, const float *i2w, const float *i1, const float *v,
-                              float *u, float *tau, float *sig2, float *k4prev, cudaStream_t s) {
-    k_flow_setup<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, roi, i2w, i1, v, u, tau, sig2, k4prev);
+cudaError_t launch_flow_pack(long long n, const float *Y, const float *V, float *y, float4 *v0, float4 *v1, float4 *v2,
+                             cudaStream_t s) {
+    k_flow_pack<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((unsigned)n, Y, V, y, v0, v1, v2);
     return cudaGetLastError();
 }
 
-cudaError_t launch_flow_primal(const int *d, const FlowRoi &roi, const float *y, const float *u, const float *tau,
-                               const float *v_in, float *v_out, float *kty, int flags, double *resid, const int *done,
-                               cudaStream_t s) {
-    k_flow_primal<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, roi, y, u, tau, v_in, v_out, kty, flags, resid,
+cudaError_t launch_flow_setup(const int *d, const FlowRoi &roi, const float *i2w, const float *i1, const float *V,
+                              float4 *u, float4 *steps, float *k4prev, cudaStream_t s) {
+    k_flow_setup<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, roi, i2w, i1, V, u, steps, k4prev);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_flow_primal(const int *d, const FlowRoi &roi, const float *y, const float4 *u, const float4 *steps,
+                               const float4 *v_in, float4 *v_out, float *kty, int flags, double *resid,
+                               const int *done, cudaStream_t s) {
+    k_flow_primal<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, roi, y, u, steps, v_in, v_out, kty, flags, resid,
                                               done);
     return cudaGetLastError();
 }
 
-cudaError_t launch_flow_dual(const int *d, const float *v, const float *v_old, const float *u, const float *sig2,
-                             const float *k4prev, float *y, float sigma1, float hf, float lambda, int huber, int flags,
-                             double *resid, const int *done, cudaStream_t s) {
+namespace {
+DualPar dual_par(float sigma1, float hf, float lambda, int huber) {
     // lam2_lo = lambda^2 (1 - 2^-20) rounded down: s < lam2_lo gives sqrt(s) < lambda (1 - 2^-21), whose float
     // rounding stays below lambda, so sqrt(s)/lambda rounds to at most 1.
     const double l2 = (double)lambda * (double)lambda * (1.0 - 1.0 / 1048576.0);
     float lam2_lo = (float)l2;
     if ((double)lam2_lo > l2) lam2_lo = std::nextafter(lam2_lo, 0.0f);
-    k_flow_dual<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, v, v_old, u, sig2, k4prev, y, sigma1, hf, lambda,
-                                            lam2_lo, huber, flags, resid, done);
+    return DualPar{sigma1, hf, lambda, lam2_lo, huber};
+}
+}  // namespace
+
+cudaError_t launch_flow_dual(const int *d, const float4 *v, const float4 *v_old, const float4 *u, const float4 *steps,
+                             const float *k4prev, float *y, float sigma1, float hf, float lambda, int huber, int flags,
+                             double *resid, const int *done, cudaStream_t s) {
+    k_flow_dual<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, v, v_old, u, steps, k4prev, y,
+                                            dual_par(sigma1, hf, lambda, huber), flags, resid, done);
     return cudaGetLastError();
 }
 
-cudaError_t launch_flow_settle(long long n3, const int *iters, const float *v_b, float *v_a, cudaStream_t s) {
-    k_flow_settle<<<grid_stride_blocks(n3, 256), 256, 0, s>>>(n3, iters, v_b, v_a);
+cudaError_t launch_flow_step(const int *d, const FlowRoi &roi, const float *y_in, float *y_out, const float4 *v,
+                             const float4 *v_old, float4 *v_next, const float4 *u, const float4 *steps,
+                             const float *k4prev, float *kty, float sigma1, float hf, float lambda, int huber,
+                             int flags, const int *done, cudaStream_t s) {
+    const int gx = (d[0] + 30) / 31, gy = (d[1] + STEP_Y - 1) / STEP_Y;
+    // Runs along z: the count whose rounds of resident blocks (two per SM) walk
+    // the fewest planes, each run with about one and a half on top (the duals
+    // formed again below it, and its first loads).
+    const int resident = 4 * sm_count();
+    int planes = d[2];
+    long long best = -1;
+    for (int runs = 1; runs <= std::max(1, d[2] / 3); ++runs) {
+        const int pl = (d[2] + runs - 1) / runs;
+        const long long blocks = (long long)gx * gy * ((d[2] + pl - 1) / pl);
+        const long long cost = (blocks + resident - 1) / resident * (2 * pl + 3);
+        if (best < 0 || cost < best) best = cost, planes = pl;
+    }
+    k_flow_step<<<dim3(gx, gy, (d[2] + planes - 1) / planes), dim3(32, STEP_Y + 1), 0, s>>>(
+        Dims{d[0], d[1], d[2]}, roi, y_in, y_out, v, v_old, v_next, u, steps, k4prev, kty,
+        dual_par(sigma1, hf, lambda, huber), flags, planes, done);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_flow_settle(long long n, const int *iters, const float4 *v_1, const float4 *v_2, float4 *v_0,
+                               float *V, cudaStream_t s) {
+    k_flow_settle<<<(unsigned)((n + 255) / 256), 256, 0, s>>>((unsigned)n, iters, v_1, v_2, v_0, V);
     return cudaGetLastError();
 }
 
@@ -603,8 +767,8 @@ cudaError_t launch_gradient(const int *d, const float *img, float *g, cudaStream
     return cudaGetLastError();
 }
 
-cudaError_t launch_copy_roi(const int *d, int nc, const FlowRoi &roi, const float *src, float *dst, cudaStream_t s) {
-    k_copy_roi<<<vox_grid(d, nc), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, nc, roi, src, dst);
+cudaError_t launch_flow_unpack(const int *d, const FlowRoi &roi, const float *y, float *Y, cudaStream_t s) {
+    k_flow_unpack<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, roi, y, Y);
     return cudaGetLastError();
 }
 

@@ -62,8 +62,12 @@ struct stt_flow {
     std::vector<float *> pyr1, pyr2;           // the coarser levels of the pyramid
     float *vbuf[2] = {nullptr, nullptr};       // flow of the coarser levels
     float *ybuf[2] = {nullptr, nullptr};       // dual of every level
-    float *yw = nullptr, *vpp = nullptr, *kty = nullptr, *u = nullptr, *tau = nullptr, *sig2 = nullptr,
-          *i2w = nullptr, *k4prev = nullptr;
+    // the iterations' fields (k_flow.cu): the dual twice, the flow three times,
+    // the image gradient, the step sizes
+    float *yw[2] = {nullptr, nullptr};
+    float4 *vw[3] = {nullptr, nullptr, nullptr}, *u = nullptr, *steps = nullptr;
+    float *kty = nullptr, *i2w = nullptr, *k4prev = nullptr;
+    float *tmp = nullptr;  // a plane of scratch of the resizes
     int *tsrc = nullptr;
     double *tfrac = nullptr;
     double *resid = nullptr;
@@ -72,11 +76,11 @@ struct stt_flow {
     float *errs = nullptr;
     int n_stat = 0, stat_cap = 0;
     // The stop flag as the host last saw it: at every residual check the flag
-    // is copied into a slot of this pinned ring behind an event, so the host
-    // can stop enqueuing a warp whose iterations stopped (enqueue_level).
-    static constexpr int kRing = 8, kLookahead = 4;
+    // is copied to pinned memory behind an event, so the host can stop
+    // enqueuing a warp whose iterations stopped (enqueue_level).
+    static constexpr int kAhead = 16;
     int *done_host = nullptr;
-    cudaEvent_t ring_ev[kRing] = {};
+    cudaEvent_t seen = nullptr;
 
     stt_status fail(stt_status st, const std::string &m) {
         err = m;
@@ -99,8 +103,7 @@ struct stt_flow {
     }
     ~stt_flow() {
         for (void *q : allocs) cudaFree(q);
-        for (cudaEvent_t e : ring_ev)
-            if (e) cudaEventDestroy(e);
+        if (seen) cudaEventDestroy(seen);
         if (done_host) cudaFreeHost(done_host);
     }
 };
@@ -127,8 +130,7 @@ stt_status enqueue_blur(stt_flow *f, const int *d, int nc, float sigma, float *i
 }
 
 // get_resize(odim, nc, 5): one pass per axis whose extent changes, x then y
-// then z, one channel at a time, ping-ponging through f->i2w and f->sig2
-// (both free between levels).
+// then z, one channel at a time, ping-ponging through f->i2w and f->tmp.
 stt_status enqueue_resize(stt_flow *f, const int *di, int nc, const float *in, const int *dout, float *out,
                           cudaStream_t s) {
     int axes[3], na = 0;
@@ -163,7 +165,7 @@ stt_status enqueue_resize(stt_flow *f, const int *di, int nc, const float *in, c
                 ra.src = f->tsrc;
                 ra.frac = f->tfrac;
             }
-            float *dst = q == na - 1 ? out + ch * vol(dout) : (q % 2 == 0 ? f->i2w : f->sig2);
+            float *dst = q == na - 1 ? out + ch * vol(dout) : (q % 2 == 0 ? f->i2w : f->tmp);
             FLOW_CUDA(f, stt::launch_resize_axis(ra, src, dst, s), "k_resize_axis");
             src = dst;
         }
@@ -171,10 +173,13 @@ stt_status enqueue_resize(stt_flow *f, const int *di, int nc, const float *in, c
     return STT_OK;
 }
 
-// One L1Huber_OF call (optical_flow.h:83-623) on a level of size d.  The
-// flow alternates between V and f->vpp: iteration `it` reads buffer
-// (it-1)&1 and writes buffer it&1; k_flow_settle brings the last one back
-// into V at the end of every warp.
+// One L1Huber_OF call (optical_flow.h:83-623) on a level of size d.
+// Iteration `it` is a primal step (flow it-1 -> it) and a dual step; between
+// residual checks the dual step runs together with the next iteration's primal
+// step (k_flow_step).  The flow of iteration `it` lies in buffer it % 3;
+// k_flow_settle unpacks the last one into V at the end of every warp.  The
+// fused steps alternate two dual buffers, and an even number of them runs between
+// two checks, so the dual is in the first whenever a warp can stop.
 stt_status enqueue_level(stt_flow *f, const int *d, const float *box, const int *roi6, const float *i1,
                          const float *i2, float *V, float *Y, int stat0, cudaStream_t s) {
     const stt_flow_params &p = f->p;
@@ -182,22 +187,19 @@ stt_status enqueue_level(stt_flow *f, const int *d, const float *box, const int 
     const stt::FlowRoi roi{roi6[0], roi6[1], roi6[2], roi6[3], roi6[4], roi6[5]};
     const float sigma1 = std::min(1.0f / 3.0f, std::min(1.0f / 3.0f, 1.0f / 3.0f));
     const float hf = 1.0f / (1.0f + sigma1 * p.huber / p.lambda);
-    float *vb[2] = {V, f->vpp};
-    FLOW_CUDA(f, cudaMemcpyAsync(f->yw, Y, sizeof(float) * 10 * n, cudaMemcpyDeviceToDevice, s), "copy Y");
-    FLOW_CUDA(f, cudaMemcpyAsync(f->vpp, V, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, s), "copy V");
+    const int huber = p.norm == 4 ? 1 : 0;
+    float4 **vb = f->vw;
+    FLOW_CUDA(f, stt::launch_flow_pack(n, Y, V, f->yw[0], vb[0], vb[1], vb[2], s), "k_flow_pack");
     FLOW_CUDA(f, cudaMemsetAsync(f->kty, 0, sizeof(float) * 3 * n, s), "clear Kty");
     const bool runs = 1.0f > p.tol;  // err starts at 1 (optical_flow.h:305-306)
     const int last = p.max_iter + 1;
     bool any_dual = false;
-    // Once a warp's check has stopped it, the launches of its remaining
-    // iterations return at once, but each still costs its full grid (about
-    // 75 us per iteration at 256^3; with the reference's parameters the warps
-    // of a 256^3 multiscale solve stop after 400-1000 of their 3001
-    // iterations).  So after every check the stop flag is copied to pinned
-    // host memory behind an event; the host stays at most kLookahead checks
-    // ahead of the device, and when a copy that has landed shows the warp
-    // stopped, the rest of its iterations are not enqueued (they would have
-    // done nothing: the same results, and the same iteration counts, which
+    // Once a warp's check has stopped it, its remaining launches return at once
+    // but still cost a launch each.  So after every check the stop flag is
+    // copied to pinned host memory behind an event; kAhead iterations later
+    // (enough to keep the device busy meanwhile) the host waits for it, and when
+    // the warp stopped the rest of its iterations are not enqueued (they would
+    // have done nothing: the same results, and the same iteration counts, which
     // the check recorded when it stopped).  Not while the stream is being
     // captured: then every iteration is enqueued.
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -211,59 +213,60 @@ stt_status enqueue_level(stt_flow *f, const int *d, const float *box, const int 
         float *err_slot = f->errs + stat0 + w;
         FLOW_CUDA(f, stt::launch_flow_reset(f->done, f->resid, it_slot, err_slot, s), "k_flow_reset");
         FLOW_CUDA(f, stt::launch_warp_box(d, box, V, i2, 1, -1.0f, f->i2w, s), "k_warp_box");
-        FLOW_CUDA(f, stt::launch_flow_setup(d, roi, f->i2w, i1, V, f->u, f->tau, f->sig2, f->k4prev, s),
+        FLOW_CUDA(f, stt::launch_flow_setup(d, roi, f->i2w, i1, V, f->u, f->steps, f->k4prev, s),
                   "k_flow_setup");
         if (!runs) continue;
-        int pushed = 0, seen = 0;  // checks whose flag copy was enqueued / looked at
+        int fused0 = 0, fused1 = 0;  // iterations [fused0, fused1) of this block of 50 run fused
+        int ycur = 0, look = 0;      // the current dual; where the host looks at the stop flag next
+        bool primal_done = false;
         for (int it = 1; it <= last; ++it) {
-            int flags = (it % 50 == 0 ? 1 : 0) | ((it + 1) % 50 == 0 ? 2 : 0);
-            if (it == 1) flags |= any_dual ? 8 : 4;
-            const float *vin = vb[(it - 1) & 1];
-            float *vout = vb[it & 1];
-            FLOW_CUDA(f, stt::launch_flow_primal(d, roi, f->yw, f->u, f->tau, vin, vout, f->kty, flags, f->resid,
-                                                 f->done, s),
-                      "k_flow_primal");
-            FLOW_CUDA(f, stt::launch_flow_dual(d, vout, vin, f->u, f->sig2, f->k4prev, f->yw, sigma1, hf, p.lambda,
-                                               p.norm == 4 ? 1 : 0, flags, f->resid, f->done, s),
+            if (look && it > look) {
+                FLOW_CUDA(f, cudaEventSynchronize(f->seen), "cudaEventSynchronize");
+                if (*f->done_host) break;
+                look = 0;
+            }
+            // bit 0: residual; 1: keep K^T y for the next iteration's residual; 2, 3: first of the level, of the warp
+            const auto flags_of = [&](int k) { return (k % 50 == 0 ? 1 : 0) | ((k + 1) % 50 == 0 ? 2 : 0); };
+            const int first = it == 1 ? (any_dual ? 8 : 4) : 0;
+            const float4 *vin = vb[(it - 1) % 3];
+            float4 *vout = vb[it % 3];
+            if (it % 50 == 1) {  // its dual steps up to the one before the check's primal step, or the last
+                fused0 = it;
+                fused1 = std::min(it + 48, last);
+                if ((fused1 - fused0) & 1) ++fused0;
+            }
+            if (!primal_done)
+                FLOW_CUDA(f, stt::launch_flow_primal(d, roi, f->yw[ycur], f->u, f->steps, vin, vout, f->kty, flags_of(it),
+                                                     f->resid, f->done, s),
+                          "k_flow_primal");
+            primal_done = it >= fused0 && it < fused1;
+            if (primal_done) {
+                FLOW_CUDA(f, stt::launch_flow_step(d, roi, f->yw[ycur], f->yw[ycur ^ 1], vout, vin, vb[(it + 1) % 3], f->u,
+                                                   f->steps, f->k4prev, f->kty, sigma1, hf, p.lambda, huber,
+                                                   first | (flags_of(it + 1) & 2), f->done, s),
+                          "k_flow_step");
+                ycur ^= 1;
+                continue;
+            }
+            const int flags = flags_of(it) | first;
+            FLOW_CUDA(f, stt::launch_flow_dual(d, vout, vin, f->u, f->steps, f->k4prev, f->yw[ycur], sigma1, hf, p.lambda,
+                                               huber, flags, f->resid, f->done, s),
                       "k_flow_dual");
             if ((flags & 1) || it == last)
                 FLOW_CUDA(f, stt::launch_flow_check(f->resid, n, p.tol, it, flags & 1, it == last, f->done, it_slot,
                                                     err_slot, s),
                           "k_flow_check");
             if (poll && (flags & 1) && it < last) {
-                // at most kLookahead checks (kLookahead * 50 iterations) ahead of the
-                // device: past that, wait for the oldest copy, so that no more than
-                // those iterations are enqueued after the warp stopped
-                if (pushed - seen >= stt_flow::kLookahead) {
-                    FLOW_CUDA(f, cudaEventSynchronize(f->ring_ev[seen % stt_flow::kRing]), "cudaEventSynchronize");
-                    if (f->done_host[seen % stt_flow::kRing]) break;
-                    ++seen;
-                }
-                const int q = pushed++ % stt_flow::kRing;
-                FLOW_CUDA(f, cudaMemcpyAsync(f->done_host + q, f->done, sizeof(int), cudaMemcpyDeviceToHost, s),
+                FLOW_CUDA(f, cudaMemcpyAsync(f->done_host, f->done, sizeof(int), cudaMemcpyDeviceToHost, s),
                           "copy stop flag");
-                FLOW_CUDA(f, cudaEventRecord(f->ring_ev[q], s), "event record");
-                bool stopped = false;
-                while (seen < pushed) {
-                    const cudaError_t qe = cudaEventQuery(f->ring_ev[seen % stt_flow::kRing]);
-                    if (qe == cudaErrorNotReady) {
-                        cudaGetLastError();  // (not an error: the copy has not landed yet)
-                        break;
-                    }
-                    FLOW_CUDA(f, qe, "cudaEventQuery");
-                    if (f->done_host[seen % stt_flow::kRing]) {
-                        stopped = true;
-                        break;
-                    }
-                    ++seen;
-                }
-                if (stopped) break;
+                FLOW_CUDA(f, cudaEventRecord(f->seen, s), "event record");
+                look = it + stt_flow::kAhead;
             }
         }
         any_dual = true;
-        FLOW_CUDA(f, stt::launch_flow_settle(3 * n, it_slot, f->vpp, V, s), "k_flow_settle");
+        FLOW_CUDA(f, stt::launch_flow_settle(n, it_slot, vb[1], vb[2], vb[0], V, s), "k_flow_settle");
     }
-    FLOW_CUDA(f, stt::launch_copy_roi(d, 10, roi, f->yw, Y, s), "k_copy_roi");
+    FLOW_CUDA(f, stt::launch_flow_unpack(d, roi, f->yw[0], Y, s), "k_flow_unpack");
     return STT_OK;
 }
 
@@ -336,13 +339,13 @@ stt_status stt_flow_create(int device, const int *dims, const stt_flow_params *p
         A(&f->vbuf[b], 3 * coarse_max);
         A(&f->ybuf[b], 10 * n);
     }
-    A(&f->yw, 10 * n);
-    A(&f->vpp, 3 * n);
+    for (int b = 0; b < 2; ++b) A(&f->yw[b], 10 * n);
+    for (int b = 0; b < 3; ++b) A(&f->vw[b], n);
     A(&f->k4prev, n);
     A(&f->kty, 3 * n);
-    A(&f->u, 4 * n);
-    A(&f->tau, 3 * n);
-    A(&f->sig2, n);
+    A(&f->u, n);
+    A(&f->steps, n);
+    A(&f->tmp, n);
     A(&f->i2w, n);
     A(&f->tsrc, kTableCap);
     A(&f->tfrac, kTableCap);
@@ -351,17 +354,15 @@ stt_status stt_flow_create(int device, const int *dims, const stt_flow_params *p
     f->stat_cap = std::max(1, (int)f->lev.size() * std::max(1, p->n_warps));
     A(&f->iters, f->stat_cap);
     A(&f->errs, f->stat_cap);
-    if (st == STT_OK && cudaHostAlloc((void **)&f->done_host, stt_flow::kRing * sizeof(int), cudaHostAllocDefault) !=
-                            cudaSuccess) {
+    if (st == STT_OK && cudaHostAlloc((void **)&f->done_host, sizeof(int), cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         f->done_host = nullptr;
-        st = f->fail(STT_ERR_NOMEM, "cudaHostAlloc of the stop-flag ring failed");
+        st = f->fail(STT_ERR_NOMEM, "cudaHostAlloc of the stop flag failed");
     }
-    for (int q = 0; q < stt_flow::kRing && st == STT_OK; ++q)
-        if (cudaEventCreateWithFlags(&f->ring_ev[q], cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            st = f->fail(STT_ERR_CUDA, "event create");
-        }
+    if (st == STT_OK && cudaEventCreateWithFlags(&f->seen, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        st = f->fail(STT_ERR_CUDA, "event create");
+    }
     if (st != STT_OK) {
         std::string m = f->err;
         delete f;

@@ -294,15 +294,26 @@ struct ResizeAxis {
 
 cudaError_t launch_warp_box(const int *dim, const float *box, const float *vel, const float *src, int nc,
                             float dt, float *out, cudaStream_t s);
-cudaError_t launch_flow_setup(const int *d, const FlowRoi &roi, const float *i2w, const float *i1,
-                              const float *v, float *u, float *tau, float *sig2, float *k4prev, cudaStream_t s);
-cudaError_t launch_flow_primal(const int *d, const FlowRoi &roi, const float *y, const float *u,
-                               const float *tau, const float *v_in, float *v_out, float *kty, int flags,
-                               double *resid, const int *done, cudaStream_t s);
-cudaError_t launch_flow_dual(const int *d, const float *v, const float *v_old, const float *u, const float *sig2,
-                             const float *k4prev, float *y, float sigma1, float hf, float lambda, int huber,
-                             int flags, double *resid, const int *done, cudaStream_t s);
-cudaError_t launch_flow_settle(long long n3, const int *iters, const float *v_b, float *v_a, cudaStream_t s);
+// The iterations' fields (float4 per voxel: v, u, steps; y packed): see FlowVec in
+// k_flow.cu.  Y and V are the caller's planes.
+cudaError_t launch_flow_pack(long long n, const float *Y, const float *V, float *y, float4 *v0, float4 *v1, float4 *v2,
+                             cudaStream_t s);
+cudaError_t launch_flow_setup(const int *d, const FlowRoi &roi, const float *i2w, const float *i1, const float *V,
+                              float4 *u, float4 *steps, float *k4prev, cudaStream_t s);
+cudaError_t launch_flow_primal(const int *d, const FlowRoi &roi, const float *y, const float4 *u, const float4 *steps,
+                               const float4 *v_in, float4 *v_out, float *kty, int flags, double *resid,
+                               const int *done, cudaStream_t s);
+cudaError_t launch_flow_dual(const int *d, const float4 *v, const float4 *v_old, const float4 *u, const float4 *steps,
+                             const float *k4prev, float *y, float sigma1, float hf, float lambda, int huber, int flags,
+                             double *resid, const int *done, cudaStream_t s);
+// The dual step of an iteration and the primal step of the next in one pass
+// (k_flow_step); y_out and v_next are buffers of their own.
+cudaError_t launch_flow_step(const int *d, const FlowRoi &roi, const float *y_in, float *y_out, const float4 *v,
+                             const float4 *v_old, float4 *v_next, const float4 *u, const float4 *steps,
+                             const float *k4prev, float *kty, float sigma1, float hf, float lambda, int huber,
+                             int flags, const int *done, cudaStream_t s);
+cudaError_t launch_flow_settle(long long n, const int *iters, const float4 *v_1, const float4 *v_2, float4 *v_0,
+                               float *V, cudaStream_t s);
 cudaError_t launch_flow_check(double *resid, long long n, float tol, int it, int is_resid, int is_last,
                               int *done, int *iters, float *err, cudaStream_t s);
 cudaError_t launch_flow_reset(int *done, double *resid, int *iters, float *err, cudaStream_t s);
@@ -311,8 +322,7 @@ cudaError_t launch_deriche(const int *d, int nc, int axis, const DericheCoef &c,
 cudaError_t launch_resize_table(int old_n, int new_n, int *src, double *frac, cudaStream_t s);
 cudaError_t launch_resize_axis(const ResizeAxis &ra, const float *in, float *out, cudaStream_t s);
 cudaError_t launch_gradient(const int *d, const float *img, float *g, cudaStream_t s);
-cudaError_t launch_copy_roi(const int *d, int nc, const FlowRoi &roi, const float *src, float *dst,
-                            cudaStream_t s);
+cudaError_t launch_flow_unpack(const int *d, const FlowRoi &roi, const float *y, float *Y, cudaStream_t s);
 
 // `status` (may be null: then a per-device word read by warp_poll_status) is
 // set when the staged kernel's bounded wait for its velocity box gave up.
