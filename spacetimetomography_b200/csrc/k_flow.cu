@@ -702,6 +702,21 @@ cudaError_t launch_flow_dual(const int *d, const float4 *v, const float4 *v_old,
     return cudaGetLastError();
 }
 
+// Whether the steps between residual checks run fused.  The two kernels update
+// the dual in place, so they hold 120 bytes per voxel where k_flow_step holds
+// 160: for the sizes in between, the two kernels' fields still stay in the L2
+// (126 MB) from one iteration to the next and the fused kernel's don't.  Two
+// kernels / fused, us per iteration: 80^3 (160 n = 0.62 of the L2) 19.0 / 17.6,
+// 90^3 (0.88) 23.9 / 29.6, 96^3 (1.07) 30.0 / 37.0, 97 x 96 x 99 (1.11) 34.0 / 38.2,
+// 104^3 (1.36) 44.4 / 46.2, 110^3 (1.60) 52.1 / 50.0, 124^3 (2.30) 71.0 / 65.9,
+// 256^3 578 / 542.
+bool flow_fuses(long long voxels) {
+    int dev = 0, l2 = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, dev) != cudaSuccess) cudaGetLastError();
+    return voxels * 160 < l2 * 3LL / 4 || voxels * 160 > l2 * 3LL / 2;
+}
+
 cudaError_t launch_flow_step(const int *d, const FlowRoi &roi, const float *y_in, float *y_out, const float4 *v,
                              const float4 *v_old, float4 *v_next, const float4 *u, const float4 *steps,
                              const float *k4prev, float *kty, float sigma1, float hf, float lambda, int huber,

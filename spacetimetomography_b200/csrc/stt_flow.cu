@@ -176,7 +176,7 @@ stt_status enqueue_resize(stt_flow *f, const int *di, int nc, const float *in, c
 // One L1Huber_OF call (optical_flow.h:83-623) on a level of size d.
 // Iteration `it` is a primal step (flow it-1 -> it) and a dual step; between
 // residual checks the dual step runs together with the next iteration's primal
-// step (k_flow_step).  The flow of iteration `it` lies in buffer it % 3;
+// step (k_flow_step; not for the volumes of flow_fuses).  The flow of iteration `it` lies in buffer it % 3;
 // k_flow_settle unpacks the last one into V at the end of every warp.  The
 // fused steps alternate two dual buffers, and an even number of them runs between
 // two checks, so the dual is in the first whenever a warp can stop.
@@ -194,6 +194,7 @@ stt_status enqueue_level(stt_flow *f, const int *d, const float *box, const int 
     const bool runs = 1.0f > p.tol;  // err starts at 1 (optical_flow.h:305-306)
     const int last = p.max_iter + 1;
     bool any_dual = false;
+    const bool fuse = stt::flow_fuses(n);
     // Once a warp's check has stopped it, its remaining launches return at once
     // but still cost a launch each.  So after every check the stop flag is
     // copied to pinned host memory behind an event; kAhead iterations later
@@ -239,7 +240,7 @@ stt_status enqueue_level(stt_flow *f, const int *d, const float *box, const int 
                 FLOW_CUDA(f, stt::launch_flow_primal(d, roi, f->yw[ycur], f->u, f->steps, vin, vout, f->kty, flags_of(it),
                                                      f->resid, f->done, s),
                           "k_flow_primal");
-            primal_done = it >= fused0 && it < fused1;
+            primal_done = fuse && it >= fused0 && it < fused1;
             if (primal_done) {
                 FLOW_CUDA(f, stt::launch_flow_step(d, roi, f->yw[ycur], f->yw[ycur ^ 1], vout, vin, vb[(it + 1) % 3], f->u,
                                                    f->steps, f->k4prev, f->kty, sigma1, hf, p.lambda, huber,

@@ -306,6 +306,8 @@ cudaError_t launch_flow_primal(const int *d, const FlowRoi &roi, const float *y,
 cudaError_t launch_flow_dual(const int *d, const float4 *v, const float4 *v_old, const float4 *u, const float4 *steps,
                              const float *k4prev, float *y, float sigma1, float hf, float lambda, int huber, int flags,
                              double *resid, const int *done, cudaStream_t s);
+// Whether a level of that many voxels takes launch_flow_step between residual checks.
+bool flow_fuses(long long voxels);
 // The dual step of an iteration and the primal step of the next in one pass
 // (k_flow_step); y_out and v_next are buffers of their own.
 cudaError_t launch_flow_step(const int *d, const FlowRoi &roi, const float *y_in, float *y_out, const float4 *v,

@@ -50,3 +50,9 @@ def test_iteration_counts_around_the_checks(cuda, last):
 def test_a_warp_that_stops_on_its_residual(cuda):
     its = _run((12, 10, 40), (0, 0, 0, 0, 0, 0), max_iter=400, n_warps=3, tol=0.9, seed=5)
     assert all(k % 50 == 0 and k < 401 for k in its), its
+
+
+@pytest.mark.parametrize("shape", [(85, 88, 99), (90, 90, 90), (106, 104, 105), (109, 110, 111)])
+def test_volumes_around_the_l2(cuda, shape):
+    """Both sides of the sizes whose dual and primal steps run as two kernels."""
+    _run(shape, (2, 1, 3, 1, 2, 4), max_iter=6, n_warps=1, seed=shape[0])
