@@ -42,9 +42,15 @@ template <typename T>
 __device__ __forceinline__ void roi_apply_at(int i, int j, int k, int nx, int ny, int nz, const int *cut,
                                              const int *pdcut, T *vol, const T *xprev, T *xbar) {
     const size_t p = i + (size_t)j * nx + (size_t)k * nx * ny;
-    const float v = ld_stored(vol + p) * roi_value(i, j, k, nx, ny, nz, cut);  // (a product by 0 or 1: exact)
-    st_stored(vol + p, v);
-    if (xbar && !roi_out(i, j, k, nx, ny, nz, pdcut)) st_stored(xbar + p, 2.0f * v - ld_voxel(xprev + p));
+    const bool kept = roi_value(i, j, k, nx, ny, nz, cut) != 0.0f;
+    const bool relax = xbar && !roi_out(i, j, k, nx, ny, nz, pdcut);
+    if (kept && !relax) return;  // times one: the voxel stays as it is
+    float v = ld_stored(vol + p);
+    if (!kept) {
+        v *= 0.0f;  // (the reference's product: a NaN stays one, a negative voxel becomes -0)
+        st_stored(vol + p, v);
+    }
+    if (relax) st_stored(xbar + p, 2.0f * v - ld_voxel(xprev + p));
 }
 
 // A load of an FP32 array: through the read-only path, or (RW) a plain load
