@@ -151,7 +151,8 @@ typedef struct stt_tuning {
     int from_cache;  /* stt_autotune: the choice came from the cache (nothing timed) */
     float fp_us[12], slab_us[8], bp_us[8];
     int ray_variant;  /* the ray-driven backprojection's scatter (kernel 3 of stt_tuning_variant_name);
-                         untuned: the shared-memory slab box from 2^26 voxels on, else global atomics */
+                         untuned: global atomics, or the shared-memory slab box from 2^26 voxels on
+                         where the detector rows are 0.75 voxels apart or more */
     float ray_us[2];
     unsigned staged_bins_bf16;  /* staged_bins for a BF16-stored volume (stt_solve_cfg.storage,
                                    stt_sart_sweep_typed): its gathers and boxes move half the bytes */

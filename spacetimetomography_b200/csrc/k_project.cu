@@ -1,6 +1,5 @@
-// k_project.cu -- ray-driven kernels: forward projection, forward projection
-// fused with the SART correction, the ray-driven backprojection scatter and
-// the exact adjoint A^T.
+// k_project.cu -- the forward projection, and the forward projection fused with
+// the SART correction.
 //
 // One thread per detector pixel.  A 128-thread block covers 32x4 pixels: each
 // warp is 32 consecutive detector columns of one row, so at every step its 32
@@ -136,95 +135,6 @@ __global__ void __launch_bounds__(32 * NW) k_fp_corr(const GeomDev g, const View
         L = raylen_state ? raylen_state[pix] : 0.0f;
     }
     corr[pix] = __fdiv_rn(__fsub_rn(ld_voxel(b + pix), sum), __fadd_rn(L, 1.0f));
-}
-
-// BP-mode march (SingleScalarVolume.core.h:128-143, UpdateContributionSum
-// :73-84): every sample scatters (c*w_k, w_k) into the interleaved
-// accumulator of its 8 clamped corners with one vector atomic each.
-__global__ void __launch_bounds__(128) k_bp_ray_scatter(const GeomDev g,
-                                                        const ViewRec *__restrict__ views,
-                                                        const ViewSel sel,
-                                                        const float *__restrict__ corr,
-                                                        float2 *__restrict__ acc) {
-    int i, j;
-    if (!tile_pixel(g, i, j)) return;
-    int local;
-    const int view = sel_view(sel, local);
-    Ray r;
-    make_ray(g, views[view], i, j, r);
-    if (!(r.tnear < r.tfar)) return;
-    const float c = __ldg(corr + i + (size_t)j * g.W);
-    march(g, r, [&](const float p[3]) {
-        Taps t;
-        make_taps(g, p, t);
-        float w[8];
-        tri_weights(t, w);
-        scatter_corners(acc, t, c, w);
-    });
-}
-
-// Exact adjoint of k_fp: vol_bar[corner] += sd * w_k * y for every sample,
-// the entry sample twice, clamped corners collapsing as in the forward pass.
-__global__ void __launch_bounds__(128) k_fp_adjoint(const GeomDev g, const ViewRec *__restrict__ views,
-                                                    int view0, const float *__restrict__ proj_bar,
-                                                    float *__restrict__ vol_bar) {
-    int i, j;
-    if (!tile_pixel(g, i, j)) return;
-    const int v = blockIdx.z;
-    const float y = __ldg(proj_bar + (size_t)v * g.W * g.H + i + (size_t)j * g.W);
-    if (y == 0.0f) return;
-    Ray r;
-    make_ray(g, views[view0 + v], i, j, r);
-    if (!(r.tnear < r.tfar)) return;
-    const float ys = y * g.sd;
-    march(g, r, [&](const float p[3]) {
-        Taps t;
-        make_taps(g, p, t);
-        float w[8];
-        tri_weights(t, w);
-        // x-neighbour corners inside the volume whose first address is 8-byte
-        // aligned (the caller's vol_bar may start anywhere on 4 bytes): one
-        // vector atomic (the same terms)
-#pragma unroll
-        for (int m = 0; m < 8; m += 2) {
-            const long long idx = tap_index(t, m);
-            if (t.dx == 1 && !(reinterpret_cast<uintptr_t>(vol_bar + idx) & 7)) {
-                atomicAdd(reinterpret_cast<float2 *>(vol_bar + idx), make_float2(ys * w[m], ys * w[m + 1]));
-            } else {
-                atomicAdd(vol_bar + idx, ys * w[m]);
-                atomicAdd(vol_bar + idx + t.dx, ys * w[m + 1]);
-            }
-        }
-    });
-}
-
-// Ray-BP normalisation (ST_Tomography.cpp:746-762): vol += contrib/weight,
-// clamped with the reference macros so 0/0 = NaN becomes 0; the accumulator
-// is reset for the next view (TypicalRayProducer::Initial, TypicalRayProducer.cpp:91-95).
-template <typename T>
-__global__ void k_bp_ray_update(long long n, float2 *__restrict__ acc, T *__restrict__ vol, float gmax) {
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x) {
-        float2 a = acc[k];
-        float v = ld_stored(vol + k) + __fdiv_rn(a.x, a.y);
-        st_stored(vol + k, rmax(rmin(gmax, v), 0.0f));
-        acc[k] = make_float2(0.0f, 0.0f);
-    }
-}
-
-// Adds the scatter accumulators to caller arrays and clears them: the raw
-// contributions and weights of the reference's backprojection mode
-// (SingleScalarVolume.core.h:128-143, read back through
-// TypicalRayProducer::GetContributions / GetTotalWeight).
-__global__ void k_acc_split(long long n, float2 *__restrict__ acc, float *__restrict__ contrib,
-                            float *__restrict__ wsum) {
-    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n;
-         k += (long long)gridDim.x * blockDim.x) {
-        const float2 a = acc[k];
-        contrib[k] += a.x;
-        wsum[k] += a.y;
-        acc[k] = make_float2(0.0f, 0.0f);
-    }
 }
 
 // Stand-alone SART correction (ST_Tomography.cpp:667-676) for the unfused
@@ -732,56 +642,6 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigne
     else
         k_fp_corr<long long, 32, 4, FP_GROUP, false, U, U><<<ray_grid(g, 1), 128, 0, s>>>(
             g, views, vol, vol_t, sel, b_stack, raylen_state, corr, skip, FpTex{});
-    return cudaGetLastError();
-}
-
-const char *ray_variant_name(int v) {
-    static const char *names[kRayVariants] = {"global vector atomic per corner", "shared-memory box per slab"};
-    return v >= 0 && v < kRayVariants ? names[v] : "?";
-}
-
-int default_ray_variant(const GeomDev &g) { return (long long)g.nx * g.ny * g.nz >= (1LL << 26) ? 1 : 0; }
-
-// The scatter of the ray-driven backprojection: ray variant 1 (the slab box,
-// below 2^31 voxels) or 0 (a global vector atomic per corner).
-static cudaError_t bp_ray_scatter_any(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                                      float2 *acc, cudaStream_t s, int ray_variant) {
-    if (ray_variant < 0) ray_variant = default_ray_variant(g);
-    if (ray_variant == 1 && small_volume(g)) return launch_bp_ray_scatter_slab(g, views, sel, corr, acc, s);
-    k_bp_ray_scatter<<<ray_grid(g, 1), 128, 0, s>>>(g, views, sel, corr, acc);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_bp_ray(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                          float2 *acc, float *vol, float gmax, cudaStream_t s, int ray_variant) {
-    cudaError_t e = bp_ray_scatter_any(g, views, sel, corr, acc, s, ray_variant);
-    if (e != cudaSuccess) return e;
-    const long long n = (long long)g.nx * g.ny * g.nz;
-    k_bp_ray_update<float><<<grid_stride_blocks(n, 256), 256, 0, s>>>(n, acc, vol, gmax);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_bp_ray(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                          float2 *acc, unsigned short *vol, float gmax, cudaStream_t s, int ray_variant) {
-    cudaError_t e = bp_ray_scatter_any(g, views, sel, corr, acc, s, ray_variant);
-    if (e != cudaSuccess) return e;
-    const long long n = (long long)g.nx * g.ny * g.nz;
-    k_bp_ray_update<unsigned short><<<grid_stride_blocks(n, 256), 256, 0, s>>>(n, acc, vol, gmax);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_bp_ray_scatter(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
-                                  float2 *acc, float *contrib, float *wsum, cudaStream_t s, int ray_variant) {
-    cudaError_t e = bp_ray_scatter_any(g, views, sel, corr, acc, s, ray_variant);
-    if (e != cudaSuccess) return e;
-    const long long n = (long long)g.nx * g.ny * g.nz;
-    k_acc_split<<<grid_stride_blocks(n, 256), 256, 0, s>>>(n, acc, contrib, wsum);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fp_adjoint(const GeomDev &g, const ViewRec *views, int view0, int nviews,
-                              const float *proj_bar, float *vol_bar, cudaStream_t s) {
-    k_fp_adjoint<<<ray_grid(g, nviews), 128, 0, s>>>(g, views, view0, proj_bar, vol_bar);
     return cudaGetLastError();
 }
 

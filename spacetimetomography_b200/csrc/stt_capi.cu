@@ -281,6 +281,7 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g) {
     d.cx = (float)((g->W - 1) * 0.5);
     d.cy = (float)((g->H - 1) * 0.5);
     d.sdd_ds = (float)(g->sdd / g->ds);
+    d.row_pitch = (float)(g->ds * g->sid / g->sdd / g->sy);
     // detector rows per voxel where the volume comes nearest to the source (sid exceeds the reach, checked above)
     d.bp_len = stt::bp_default_len(g->sdd / g->ds * g->sy / (g->sid - std::sqrt(hx * hx + hz * hz) - off));
     ctx->sp[0] = g->sx;

@@ -56,6 +56,7 @@ struct GeomDev {
     float sd;          // sample distance |spacing| (ST_Tomography.cpp:300), FP32
     float cx, cy;      // (W-1)/2, (H-1)/2
     float sdd_ds;      // sdd / ds
+    float row_pitch;   // voxels (along y) between neighbouring detector rows' rays at the isocentre
     int bp_len;        // column length of the voxel backprojection's default variant (bp_default_len)
 };
 

@@ -30,8 +30,8 @@ int grid_stride_blocks(long long n, int threads);
 //   bp:   the column length of the voxel backprojection and the blocks per SM
 //         it is compiled for (bp_variant_name);
 //   ray:  the scatter of the ray-driven backprojection (ray_variant_name):
-//         0 one global vector atomic per corner, 1 a shared-memory box per
-//         slab (volumes below 2^31 voxels).  Its sums differ in float order
+//         0 global vector atomics, neighbouring rows merged, 1 a shared-memory
+//         box per slab (volumes below 2^31 voxels).  Its sums differ in float order
 //         only (as any two atomic runs do), not in their terms.
 // Which views the slab kernel projects is the per-view ViewRec::staged flag.
 constexpr int kFpVariants = 12, kSlabVariants = 8, kBpVariants = 5, kRayVariants = 2;
@@ -43,8 +43,7 @@ const char *fp_variant_name(int v);
 const char *slab_variant_name(int v);
 const char *bp_variant_name(int v);
 const char *ray_variant_name(int v);
-// The scatter an untuned context uses: the slab box from 2^26 voxels on (at
-// 512^3 it is the faster form; at 256^3 and below the global scatter is).
+// The scatter an untuned context uses (k_scatter.cu has the measurements).
 int default_ray_variant(const GeomDev &g);
 
 // The projection of nviews views: corners through the textures of `tex` where
