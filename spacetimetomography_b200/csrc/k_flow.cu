@@ -249,6 +249,8 @@ __global__ void __launch_bounds__(128) k_flow_primal(const Dims d, const FlowRoi
                                                      const float4 *__restrict__ v_in, float4 *__restrict__ v_out,
                                                      float *__restrict__ kty, int flags, double *__restrict__ resid,
                                                      const int *__restrict__ done) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     if (*done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
@@ -320,6 +322,8 @@ __global__ void __launch_bounds__(128) k_flow_dual(const Dims d, const float4 *_
                                                    const float4 *__restrict__ steps, const float *__restrict__ k4prev,
                                                    float *__restrict__ y, const DualPar q, int flags,
                                                    double *__restrict__ resid, const int *__restrict__ done) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     if (*done) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
@@ -378,14 +382,19 @@ __global__ void __launch_bounds__(128) k_flow_dual(const Dims d, const float4 *_
 // kernels', so are the bits.
 //
 // An iteration moves 160 bytes per voxel where the two kernels moved 212, in one
-// launch.  Per iteration, two planar kernels -> this, us: 54^3 14.7 -> 8.8, 83^3
-// 23.6 -> 21.5, 128^3 79.1 -> 76.0, 147 x 121 x 135 110.6 -> 88.3, 256^3 606 ->
-// 542 (4.9 TB/s).  Bound by the latency of a plane's chain (loads, duals,
-// exchange) at 20 warps per SM; so small blocks, whose barriers hold fewer warps
-// up, beat the smaller halo of larger ones (STEP_Y 8, two blocks: 80 us at
-// 128^3; 12: 80; 16: 92).  Measured and not kept: planar fields (42 loads and
-// their addresses a voxel: 82), planes through a shared-memory ring by
-// asynchronous copies (83), one component at a time in 72 registers (94).
+// launch.  The next step's blocks come up while this one's last ones finish
+// (launch_chained; they are let up two planes before a block's end: from its
+// start they take the places that the last round's blocks spread over, 256^3 538
+// -> 555).  Per iteration, two planar kernels -> this -> chained, us: 54^3 14.7 ->
+// 8.8, 48^3 10.7 -> 8.7 -> 6.9, 80^3 23.5 -> 17.6 -> 16.5, 128^3 79.1 -> 76.0 ->
+// 70.7, 147 x 121 x 135 110.6 -> 88.9 -> 81.9, 256^3 606 -> 538 -> 528 (5.1 TB/s).
+// Bound by the latency of a plane's chain (loads, duals, exchange) at 20 warps
+// per SM; so small blocks, whose barriers hold fewer warps up, beat the smaller
+// halo of larger ones (unchained, STEP_Y 8, two blocks: 80 us at 128^3; 12: 80;
+// 16: 92).  Measured and not kept: planar fields (42 loads and their addresses a
+// voxel: 82), planes through a shared-memory ring by asynchronous copies (83),
+// one component at a time in 72 registers (94), the steps formed from u instead
+// of read (four divisions: 79).
 constexpr int STEP_Y = 4;
 __global__ void __launch_bounds__(32 * (STEP_Y + 1), 4)
     k_flow_step(const Dims d, const FlowRoi roi, const float *__restrict__ y_in, float *__restrict__ y_out,
@@ -393,6 +402,7 @@ __global__ void __launch_bounds__(32 * (STEP_Y + 1), 4)
                 const float4 *__restrict__ u, const float4 *__restrict__ steps, const float *__restrict__ k4prev,
                 float *__restrict__ kty, const DualPar q, int flags, int planes, const int *__restrict__ done) {
     __shared__ float below[2][STEP_Y + 1][3][32];
+    cudaGridDependencySynchronize();
     if (*done) return;
     const int lane = threadIdx.x, row = threadIdx.y;
     const int i0 = (int)blockIdx.x * 31 + lane - 1, j0 = (int)blockIdx.y * STEP_Y + row - 1;
@@ -419,6 +429,7 @@ __global__ void __launch_bounds__(32 * (STEP_Y + 1), 4)
     };
     load(k, p);
     for (int buf = 0; k < z1; ++k, p += sz, buf ^= 1) {
+        if (k + 2 >= z1) cudaTriggerProgrammaticLaunchCompletion();
         const bool mine = own && k >= z0;
         const bool inside = mine && in_roi(roi, d, i, j, k);
         float a[3], bx[3], by[3], bz[3], e[3], fx[3], fy[3], fz[3], yn[9], xm[3];
@@ -678,9 +689,8 @@ cudaError_t launch_flow_setup(const int *d, const FlowRoi &roi, const float *i2w
 cudaError_t launch_flow_primal(const int *d, const FlowRoi &roi, const float *y, const float4 *u, const float4 *steps,
                                const float4 *v_in, float4 *v_out, float *kty, int flags, double *resid,
                                const int *done, cudaStream_t s) {
-    k_flow_primal<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, roi, y, u, steps, v_in, v_out, kty, flags, resid,
-                                              done);
-    return cudaGetLastError();
+    return launch_chained(k_flow_primal, vox_grid(d), 128, s, Dims{d[0], d[1], d[2]}, roi, y, u, steps, v_in, v_out,
+                          kty, flags, resid, done);
 }
 
 namespace {
@@ -697,19 +707,18 @@ DualPar dual_par(float sigma1, float hf, float lambda, int huber) {
 cudaError_t launch_flow_dual(const int *d, const float4 *v, const float4 *v_old, const float4 *u, const float4 *steps,
                              const float *k4prev, float *y, float sigma1, float hf, float lambda, int huber, int flags,
                              double *resid, const int *done, cudaStream_t s) {
-    k_flow_dual<<<vox_grid(d), 128, 0, s>>>(Dims{d[0], d[1], d[2]}, v, v_old, u, steps, k4prev, y,
-                                            dual_par(sigma1, hf, lambda, huber), flags, resid, done);
-    return cudaGetLastError();
+    return launch_chained(k_flow_dual, vox_grid(d), 128, s, Dims{d[0], d[1], d[2]}, v, v_old, u, steps, k4prev, y,
+                          dual_par(sigma1, hf, lambda, huber), flags, resid, done);
 }
 
 // Whether the steps between residual checks run fused.  The two kernels update
 // the dual in place, so they hold 120 bytes per voxel where k_flow_step holds
 // 160: for the sizes in between, the two kernels' fields still stay in the L2
 // (126 MB) from one iteration to the next and the fused kernel's don't.  Two
-// kernels / fused, us per iteration: 80^3 (160 n = 0.62 of the L2) 19.0 / 17.6,
-// 90^3 (0.88) 23.9 / 29.6, 96^3 (1.07) 30.0 / 37.0, 97 x 96 x 99 (1.11) 34.0 / 38.2,
-// 104^3 (1.36) 44.4 / 46.2, 110^3 (1.60) 52.1 / 50.0, 124^3 (2.30) 71.0 / 65.9,
-// 256^3 578 / 542.
+// kernels / fused, us per iteration: 72^3 (160 n = 0.45 of the L2) 14.7 / 13.6,
+// 80^3 (0.62) 17.7 / 16.5, 90^3 (0.88) 23.1 / 25.8, 96^3 (1.07) 28.0 / 32.7, 97 x 96
+// x 99 (1.11) 30.9 / 34.1, 104^3 (1.36) 40.5 / 41.5, 110^3 (1.60) 48.2 / 45.6,
+// 124^3 (2.30) 67.0 / 60.4, 256^3 569 / 528.
 bool flow_fuses(long long voxels) {
     int dev = 0, l2 = 0;
     cudaGetDevice(&dev);
@@ -734,10 +743,9 @@ cudaError_t launch_flow_step(const int *d, const FlowRoi &roi, const float *y_in
         const long long cost = (blocks + resident - 1) / resident * (2 * pl + 3);
         if (best < 0 || cost < best) best = cost, planes = pl;
     }
-    k_flow_step<<<dim3(gx, gy, (d[2] + planes - 1) / planes), dim3(32, STEP_Y + 1), 0, s>>>(
-        Dims{d[0], d[1], d[2]}, roi, y_in, y_out, v, v_old, v_next, u, steps, k4prev, kty,
-        dual_par(sigma1, hf, lambda, huber), flags, planes, done);
-    return cudaGetLastError();
+    return launch_chained(k_flow_step, dim3(gx, gy, (d[2] + planes - 1) / planes), dim3(32, STEP_Y + 1), s,
+                          Dims{d[0], d[1], d[2]}, roi, y_in, y_out, v, v_old, v_next, u, steps, k4prev, kty,
+                          dual_par(sigma1, hf, lambda, huber), flags, planes, done);
 }
 
 cudaError_t launch_flow_settle(long long n, const int *iters, const float4 *v_1, const float4 *v_2, float4 *v_0,

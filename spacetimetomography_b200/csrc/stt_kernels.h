@@ -15,6 +15,25 @@ struct PdParams {
     int cut[8];
 };
 
+// A launch that may start before the kernel ahead of it in the stream has
+// finished: its blocks take the places that kernel's last blocks leave, and wait
+// in cudaGridDependencySynchronize(), which the kernel calls before it touches
+// anything another kernel writes or reads, until it has.  A kernel that calls
+// cudaTriggerProgrammaticLaunchCompletion() lets its successor come up early.
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t s, Args &&...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 // Multiprocessor count of the current device (cached per device).
 int sm_count();
 int grid_stride_blocks(long long n, int threads);
