@@ -46,92 +46,134 @@ __device__ __forceinline__ float cimg_cr(float p, float c, float n, float a, flo
     return c + 0.5f * (d * (-p + n) + d * d * (2 * p - 5 * c + 4 * n - a) + d * d * d * (-p + 3 * c - 3 * n + a));
 }
 
-__device__ __forceinline__ void cimg_taps(float f, int dim, int t[4], float &d) {
-    const float nf = f < 0.0f ? 0.0f : (f > (float)(dim - 1) ? (float)(dim - 1) : f);
-    const int x = (int)nf;
-    d = nf - (float)x;
-    t[0] = x - 1 < 0 ? 0 : x - 1;
-    t[1] = x;
-    t[2] = d > 0.0f ? x + 1 : x;
-    t[3] = x + 2 >= dim ? dim - 1 : x + 2;
+// Two of them in the packed FP32x2 instructions, each lane rounded as cimg_cr: a
+// product is rounded on its own before it is added.  The compiler contracts packed
+// products and sums whatever -fmad says, so a product is a fused multiply-add of a
+// negative zero that it does not know (nz); doubling, quadrupling and halving are
+// exact, so those products may stay fused.
+__device__ __forceinline__ float2 cimg_cr2(float2 p, float2 c, float2 n, float2 a, float d, float nz) {
+    const auto k = [](float x) { return make_float2(x, x); };
+    const auto mul = [&](float x, float2 y) { return __ffma2_rn(k(x), y, k(nz)); };
+    const auto sub = [&](float2 x, float2 y) { return __fadd2_rn(x, make_float2(-y.x, -y.y)); };
+    const float2 c5 = mul(-5.0f, c);
+    const float2 l = mul(d, sub(n, p));
+    const float2 q = mul(d * d, sub(__ffma2_rn(k(4.0f), n, __ffma2_rn(k(2.0f), p, c5)), a));
+    const float2 e = mul(d * d * d, __fadd2_rn(sub(sub(mul(3.0f, c), p), mul(3.0f, n)), a));
+    return __ffma2_rn(k(0.5f), __fadd2_rn(__fadd2_rn(l, q), e), c);
 }
 
-// warping::sample_image: world point -> cell grid (aabb [0, box]), clamped to
-// [1, dim-2], cubic value clamped to the min/max of the cell's 8 corners.
-__device__ float sample_box(const float *__restrict__ img, const Dims &d, const float box[3], const float p[3]) {
+// A world point's cell: the grid coordinate clamped to [1, dim-2], so taps x-1,
+// x, x+1 are inside the image; CImg takes x for the tap x+1 where the fraction
+// is zero, and the last voxel for x+2 past it.
+struct BoxCell {
+    int o[3];     // x, y, z of the first tap
+    float d[3];   // fractions
+    int last[3];  // the fourth tap, counted from the first: 3, or 2 at the upper edge
+};
+
+__device__ __forceinline__ void box_cell(const Dims &d, const float box[3], const float p[3], BoxCell &c) {
     const int D[3] = {d.x, d.y, d.z};
-    float g[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const float gw = (float)D[a] * (p[a] - 0.0f) / (box[a] - 0.0f);
-        float q = (float)((double)gw - 0.5);
+        float q = (float)D[a] * (p[a] - 0.0f) / (box[a] - 0.0f) - 0.5f;
         const float hi = (float)(D[a] - 2), lo = 1.0f;
         q = (q < hi) ? q : hi;
         q = (lo < q) ? q : lo;
-        g[a] = q;
+        const int x = (int)q;
+        c.d[a] = q - (float)x;
+        c.o[a] = x - 1;
+        c.last[a] = x + 2 >= D[a] ? 2 : 3;
     }
-    const long long sy = d.x, sz = (long long)d.x * d.y;
-    const int ix = (int)g[0], iy = (int)g[1], iz = (int)g[2];
-    const float *c0 = img + ix + iy * sy + iz * sz;
-    float mn = __ldg(c0), mx = mn;
-    const long long off[7] = {1, 1 + sy, sy, sz, 1 + sz, 1 + sy + sz, sy + sz};
+}
+
+// warping::sample_image: the cubic value clamped to the min/max of the cell's 8
+// corners, which are taps of the stencil.  Rows go in pairs of planes.
+__device__ __forceinline__ float sample_box(const float *__restrict__ img, const Dims &d, const BoxCell &q, float nz) {
+    const int sy = d.x, sz = d.x * d.y;
+    const int at = q.o[0] + q.o[1] * sy + q.o[2] * sz;
+    const float dx = q.d[0], dy = q.d[1], dz = q.d[2];
+    float zv[4], corner[8];
+#pragma unroll
+    for (int c = 0; c < 4; c += 2) {
+        float2 yv[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int row = at + (b < 3 ? b : q.last[1]) * sy;
+            const float *r0 = img + (row + c * sz), *r1 = img + (row + (c == 0 ? 1 : q.last[2]) * sz);
+            const float2 t0 = make_float2(__ldg(r0), __ldg(r1)), t1 = make_float2(__ldg(r0 + 1), __ldg(r1 + 1));
+            float2 t2 = make_float2(__ldg(r0 + 2), __ldg(r1 + 2));
+            const float2 t3 = make_float2(__ldg(r0 + q.last[0]), __ldg(r1 + q.last[0]));
+            if (b == 1 || b == 2) {  // planes 1 and 2 hold the corners: (x, y, z) at x + 2 y + 4 z
+                const int m = 2 * (b - 1) + (c == 0 ? 0 : 4);
+                corner[m] = c == 0 ? t1.y : t1.x;
+                corner[m + 1] = c == 0 ? t2.y : t2.x;
+            }
+            if (!(dx > 0.0f)) t2 = t1;
+            yv[b] = cimg_cr2(t0, t1, t2, t3, dx, nz);
+        }
+        if (!(dy > 0.0f)) yv[2] = yv[1];
+        const float2 z = cimg_cr2(yv[0], yv[1], yv[2], yv[3], dy, nz);
+        zv[c] = z.x, zv[c + 1] = z.y;
+    }
+    if (!(dz > 0.0f)) zv[2] = zv[1];
+    const float val = cimg_cr(zv[0], zv[1], zv[2], zv[3], dz);
+    constexpr int order[7] = {1, 3, 2, 4, 5, 7, 6};  // (the reference's, warping.h:71-80)
+    float mn = corner[0], mx = mn;
 #pragma unroll
     for (int k = 0; k < 7; ++k) {
-        const float v = __ldg(c0 + off[k]);
+        const float v = corner[order[k]];
         mn = (v < mn) ? v : mn;
         mx = (mx < v) ? v : mx;
     }
-    int tx[4], ty[4], tz[4];
-    float dx, dy, dz;
-    cimg_taps(g[0], d.x, tx, dx);
-    cimg_taps(g[1], d.y, ty, dy);
-    cimg_taps(g[2], d.z, tz, dz);
-    float zv[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        float yv[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const float *row = img + ty[b] * sy + tz[c] * sz;
-            yv[b] = cimg_cr(__ldg(row + tx[0]), __ldg(row + tx[1]), __ldg(row + tx[2]), __ldg(row + tx[3]), dx);
-        }
-        zv[c] = cimg_cr(yv[0], yv[1], yv[2], yv[3], dy);
-    }
-    const float val = cimg_cr(zv[0], zv[1], zv[2], zv[3], dz);
     const float inner = (val < mx) ? val : mx;
     return (mn < inner) ? inner : mn;
 }
 
 // warping::warp: trace back from each cell centre with -dt (two-step
-// semi-Lagrangian, warping.h:100-114), sample every source channel there.
-__global__ void __launch_bounds__(128) k_warp_box(const Dims d, const float bx, const float by, const float bz,
-                                                  const float *__restrict__ vel, const float *__restrict__ src, int nc,
-                                                  float dt, float *__restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= d.x) return;
+// semi-Lagrangian, warping.h:100-114), sample every source channel there.  Seven
+// samples of 64 taps and 21 uncontracted cubics a voxel: bound by issue.  So the
+// three channels of a velocity share a cell, the corners of the clamp are taps, and
+// ten of a sample's cubics are packed pairs.  One source channel, a cell and 21
+// scalar cubics per sample in 64-bit offsets, blocks of 128 x 1 -> this, us: 54^3 126
+// -> 53, 128^3 628 -> 300, 147 x 121 x 135 1289 -> 438, 256^3 5301 -> 2228 (scalar
+// cubics 128^3 414; blocks of 32 x 4 in 168 registers 304, in 96 or 80 313).
+constexpr int BOX_X = 32, BOX_Y = 8;
+__global__ void __launch_bounds__(BOX_X *BOX_Y, 2)
+    k_warp_box(const Dims d, const float bx, const float by, const float bz, const float *__restrict__ vel,
+               const float *__restrict__ src, int nc, float dt, float *__restrict__ out, float nz) {
+    const int i = blockIdx.x * BOX_X + threadIdx.x;
+    const int j = blockIdx.y * BOX_Y + threadIdx.y, k = blockIdx.z;
+    if (i >= d.x || j >= d.y) return;
     const long long n = (long long)d.x * d.y * d.z;
     const float box[3] = {bx, by, bz};
     const int ijk[3] = {i, j, k};
     const int D[3] = {d.x, d.y, d.z};
     float p[3], v[3], p2[3], q[3];
+    BoxCell cell;
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
-        p[a] = (float)(0 + ((double)(float)ijk[a] + 0.5) * (double)(box[a] - 0) / (double)(float)D[a]);
+    for (int a = 0; a < 3; ++a) {
+        if (box[a] == (float)D[a])
+            p[a] = (float)ijk[a] + 0.5f;  // (exactly what the division gives)
+        else
+            p[a] = (float)(0 + ((double)(float)ijk[a] + 0.5) * (double)(box[a] - 0) / (double)(float)D[a]);
+    }
     const float h = -dt;
+    box_cell(d, box, p, cell);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) v[c] = sample_box(vel + c * n, d, box, p);
+    for (int c = 0; c < 3; ++c) v[c] = sample_box(vel + c * n, d, cell, nz);
 #pragma unroll
     for (int c = 0; c < 3; ++c) p2[c] = p[c] + h * v[c];
+    box_cell(d, box, p2, cell);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) v[c] = sample_box(vel + c * n, d, box, p2);
+    for (int c = 0; c < 3; ++c) v[c] = sample_box(vel + c * n, d, cell, nz);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const float p0 = p2[c] - h * v[c];
-        q[c] = p2[c] + (float)(0.5 * (double)(p[c] - p0));
+        q[c] = p2[c] + 0.5f * (p[c] - p0);
     }
+    box_cell(d, box, q, cell);
     const long long o = i + (long long)j * d.x + (long long)k * d.x * d.y;
-    for (int c = 0; c < nc; ++c) out[o + c * n] = sample_box(src + c * n, d, box, q);
+    for (int c = 0; c < nc; ++c) out[o + c * n] = sample_box(src + c * n, d, cell, nz);
 }
 
 // ---- per-warp setup (optical_flow.h:257-297) ---------------------------------
@@ -669,8 +711,9 @@ inline dim3 vox_grid(const int *d, int zmul = 1) {
 
 cudaError_t launch_warp_box(const int *dim, const float *box, const float *vel, const float *src, int nc, float dt,
                             float *out, cudaStream_t s) {
-    k_warp_box<<<vox_grid(dim), 128, 0, s>>>(Dims{dim[0], dim[1], dim[2]}, box[0], box[1], box[2], vel, src, nc, dt,
-                                             out);
+    const dim3 grid((dim[0] + BOX_X - 1) / BOX_X, (dim[1] + BOX_Y - 1) / BOX_Y, dim[2]);
+    k_warp_box<<<grid, dim3(BOX_X, BOX_Y), 0, s>>>(Dims{dim[0], dim[1], dim[2]}, box[0], box[1], box[2], vel, src, nc, dt,
+                                             out, -0.0f);
     return cudaGetLastError();
 }
 
