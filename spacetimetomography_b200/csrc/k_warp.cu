@@ -165,95 +165,158 @@ __global__ void __launch_bounds__(WARP_BX *WARP_BY) k_warp_staged(const Dim3i d,
 }
 
 // ---- VJP ---------------------------------------------------------------
-// For one clamped sample: which branch the clamp took and, when unclamped,
-// the spatial gradient of the Catmull-Rom value (zero along an axis whose
-// grid coordinate was clamped to [1, dim-2]).
+// One axis of a sample's stencil: the taps x-1, x, x+1, x+2 counted from the
+// first (the last one held at the image's edge, where its weight is 0), their
+// weights and the weights' slopes.  An axis whose coordinate was clamped to
+// [1, dim-2] has no slope.
+struct AxisD {
+    int lo, last;
+    float w[4], dw[4];
+};
+
+__device__ __forceinline__ void axis_d(float p, int dim, AxisD &a) {
+    bool clamped;
+    const float g = to_grid(p, dim, &clamped);
+    const int x = (int)g;
+    const float d = g - (float)x, d2 = d * d;
+    cr_weights(d, a.w);
+    a.dw[0] = 0.5f * (-1.0f + 4.0f * d - 3.0f * d2);
+    a.dw[1] = 0.5f * (-10.0f * d + 9.0f * d2);
+    a.dw[2] = 0.5f * (1.0f + 8.0f * d - 9.0f * d2);
+    a.dw[3] = 0.5f * (-2.0f * d + 3.0f * d2);
+    if (!(d > 0.0f)) a.dw[1] = a.dw[2], a.dw[2] = 0.0f;  // (on a node CImg's tap x+1 is x; dw[1] is 0 there)
+    if (clamped)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) a.dw[k] = 0.0f;
+    a.lo = x - 1;
+    a.last = x + 2 < dim ? 3 : 2;
+}
+
+struct CellD {
+    AxisD x, y, z;
+    int at;  // the first tap
+};
+
+__device__ __forceinline__ void cell_d(const Dim3i d, const float p[3], CellD &c) {
+    axis_d(p[0], d.x, c.x);
+    axis_d(p[1], d.y, c.y);
+    axis_d(p[2], d.z, c.z);
+    c.at = c.x.lo + c.y.lo * d.x + c.z.lo * d.x * d.y;
+}
+
+// One clamped sample: its value, which branch the clamp took (corner: the
+// voxel it took, or -1) and, where it did not, the value's spatial gradient.
 struct SampleD {
     float value;
-    int branch;        // 0 interior, 1 clamped to max corner, 2 clamped to min corner
-    long long corner;  // arg-max / arg-min corner index when branch != 0
+    int corner;
     float grad[3];
 };
 
-__device__ __forceinline__ void cr_dweights(float d, float w[4]) {
-    float d2 = d * d;
-    w[0] = 0.5f * (-1.0f + 4.0f * d - 3.0f * d2);
-    w[1] = 0.5f * (-10.0f * d + 9.0f * d2);
-    w[2] = 0.5f * (1.0f + 8.0f * d - 9.0f * d2);
-    w[3] = 0.5f * (-2.0f * d + 3.0f * d2);
-}
-
-__device__ __forceinline__ void sample_d(const float *__restrict__ img, const Stencil &s,
-                                         const bool clamped[3], SampleD &r) {
-    float dwx[4], dwy[4], dwz[4];
-    cr_dweights(s.dx, dwx);
-    cr_dweights(s.dy, dwy);
-    cr_dweights(s.dz, dwz);
+__device__ __forceinline__ void sample_d(const Dim3i d, const float *__restrict__ img, const CellD &s, SampleD &r) {
     // Separable sums in the forward sampler's order (x taps, then rows, then
     // planes): per row its value and x-slope, per plane its value and x- and
     // y-slopes, then the sample's value and gradient.
-    float val = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f;
-#pragma unroll 1
+    const int sy = d.x, sz = d.x * d.y;
+    float val = 0.0f, gx = 0.0f, gy = 0.0f, gz = 0.0f, corner[8];
+#pragma unroll
     for (int c = 0; c < 4; ++c) {
         float pv = 0.0f, px = 0.0f, py = 0.0f;
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const float *row = img + s.yo[b] + s.zo[c];
-            const float t0 = __ldg(row + s.xo[0]), t1 = __ldg(row + s.xo[1]), t2 = __ldg(row + s.xo[2]),
-                        t3 = __ldg(row + s.xo[3]);
-            const float xv = s.wx[0] * t0 + s.wx[1] * t1 + s.wx[2] * t2 + s.wx[3] * t3;
-            const float xd = dwx[0] * t0 + dwx[1] * t1 + dwx[2] * t2 + dwx[3] * t3;
-            pv += s.wy[b] * xv;
-            px += s.wy[b] * xd;
-            py += dwy[b] * xv;
-        }
-        val += s.wz[c] * pv;
-        gx += s.wz[c] * px;
-        gy += s.wz[c] * py;
-        gz += dwz[c] * pv;
-    }
-    long long imn = s.c0, imx = s.c0;
-    float mn = __ldg(img + s.c0), mx = mn;
-    const int off[7] = {s.sx1, s.sx1 + s.sy1, s.sy1, s.sz1, s.sx1 + s.sz1, s.sx1 + s.sy1 + s.sz1,
-                        s.sy1 + s.sz1};
-#pragma unroll
-    for (int k = 0; k < 7; ++k) {
-        float v = __ldg(img + s.c0 + off[k]);
-        if (v < mn) { mn = v; imn = s.c0 + off[k]; }
-        if (mx < v) { mx = v; imx = s.c0 + off[k]; }
-    }
-    r.grad[0] = r.grad[1] = r.grad[2] = 0.0f;
-    if (val > mx) {
-        r.value = mx; r.branch = 1; r.corner = imx;
-    } else if (val < mn) {
-        r.value = mn; r.branch = 2; r.corner = imn;
-    } else {
-        r.value = val; r.branch = 0; r.corner = -1;
-        r.grad[0] = clamped[0] ? 0.0f : gx;
-        r.grad[1] = clamped[1] ? 0.0f : gy;
-        r.grad[2] = clamped[2] ? 0.0f : gz;
-    }
-}
-
-__device__ __forceinline__ void scatter_sample(float *__restrict__ bar, const Stencil &s,
-                                               const SampleD &r, float g) {
-    if (g == 0.0f) return;
-    if (r.branch != 0) {
-        atomicAdd(bar + r.corner, g);
-        return;
-    }
-#pragma unroll 1
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            float wbc = g * s.wy[b] * s.wz[c];
-            float *row = bar + s.yo[b] + s.zo[c];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                float w = s.wx[a] * wbc;
-                if (w != 0.0f) atomicAdd(row + s.xo[a], w);
+            const float *row = img + (s.at + (b < 3 ? b : s.y.last) * sy + (c < 3 ? c : s.z.last) * sz);
+            const float t0 = __ldg(row), t1 = __ldg(row + 1), t2 = __ldg(row + 2), t3 = __ldg(row + s.x.last);
+            const float xv = __fmaf_rn(s.x.w[3], t3, __fmaf_rn(s.x.w[2], t2, __fmaf_rn(s.x.w[0], t0, __fmul_rn(s.x.w[1], t1))));
+            const float xd = s.x.dw[0] * t0 + s.x.dw[1] * t1 + s.x.dw[2] * t2 + s.x.dw[3] * t3;
+            pv = __fmaf_rn(s.y.w[b], xv, pv);
+            px += s.y.w[b] * xd;
+            py += s.y.dw[b] * xv;
+            if ((b == 1 || b == 2) && (c == 1 || c == 2)) {
+                corner[2 * (b - 1) + 4 * (c - 1)] = t1;
+                corner[2 * (b - 1) + 4 * (c - 1) + 1] = t2;
             }
         }
+        val = __fmaf_rn(s.z.w[c], pv, val);
+        gx += s.z.w[c] * px;
+        gy += s.z.w[c] * py;
+        gz += s.z.dw[c] * pv;
+    }
+    constexpr int order[7] = {1, 3, 2, 4, 5, 7, 6};  // (of equal corners the first in the reference's order)
+    int imn = 0, imx = 0;
+    float mn = corner[0], mx = mn;
+#pragma unroll
+    for (int k = 0; k < 7; ++k) {
+        const float v = corner[order[k]];
+        if (v < mn) mn = v, imn = order[k];
+        if (mx < v) mx = v, imx = order[k];
+    }
+    const bool above = val > mx, below = !above && val < mn, in = !above && !below;
+    const int m = above ? imx : imn;
+    const float inner = (val < mx) ? val : mx;
+    r.value = (mn < inner) ? inner : mn;
+    r.corner = in ? -1 : s.at + 1 + (m & 1) + (1 + (m >> 1 & 1)) * sy + (1 + (m >> 2)) * sz;
+    r.grad[0] = in ? gx : 0.0f;
+    r.grad[1] = in ? gy : 0.0f;
+    r.grad[2] = in ? gz : 0.0f;
+}
+
+// Which neighbours in the warp have the same cell one voxel on: left: the lane
+// below samples the cell at x-1, right: the lane above the one at x+1.
+struct Links {
+    bool left, right;
+};
+
+__device__ __forceinline__ Links links_of(const CellD &s, const SampleD &r, bool live) {
+    const int lane = threadIdx.x & 31;
+    const int key = live && r.corner < 0 ? s.at : INT_MIN;
+    // (cells of a row of voxels: at is one more exactly where x is, and y and z are the same: x+1 <= dim-2)
+    const int below = __shfl_up_sync(0xffffffffu, key, 1), above = __shfl_down_sync(0xffffffffu, key, 1);
+    Links l;
+    l.left = lane > 0 && key != INT_MIN && below == key - 1;
+    l.right = lane < 31 && key != INT_MIN && above == key + 1;
+    return l;
+}
+
+// Adds g times a sample's weights to bar.  Every lane of the warp calls this.
+// Lanes are neighbours along x, and so mostly are their cells: of the four taps
+// of a row, three fall on voxels that neighbouring lanes add to as well.  Those go
+// to the neighbour by shuffle, and a lane adds its own voxel's sum; the taps past
+// the ends of a run of linked lanes are added on their own, one per lane and
+// instruction.  (An atomic instruction costs the SM 4.7 cycles however few of its
+// lanes are live, 7.4 for 32 adjacent floats, 11 for 32 in four rows; four a row
+// without the merge.)
+__device__ __forceinline__ void scatter_sample(const Dim3i d, float *__restrict__ bar, const CellD &s, const SampleD &r,
+                                               float g, bool live) {
+    live = live && g != 0.0f;
+    if (!__any_sync(0xffffffffu, live)) return;
+    if (live && r.corner >= 0) atomicAdd(bar + r.corner, g);
+    const Links l = links_of(s, r, live);
+    const bool mine = live && r.corner < 0;
+    const bool ends = !l.left || !l.right, alone = !l.left && !l.right;
+    const int sy = d.x, sz = d.x * d.y;
+    float wx[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) wx[a] = mine ? g * s.x.w[a] : 0.0f;
+#pragma unroll 1
+    for (int c = 0; c < 4; ++c) {
+        const float wz = c == 0 ? s.z.w[0] : c == 1 ? s.z.w[1] : c == 2 ? s.z.w[2] : s.z.w[3];
+        const int plane = s.at + (c < 3 ? c : s.z.last) * sz;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float f = s.y.w[b] * wz;
+            const float w0 = wx[0] * f, w1 = wx[1] * f, w2 = wx[2] * f, w3 = wx[3] * f;
+            const float u3 = __shfl_up_sync(0xffffffffu, w3, 1);
+            const float e2 = w2 + (l.left ? u3 : 0.0f);  // what lies at x+1: mine and the left neighbour's last
+            const float u2 = __shfl_up_sync(0xffffffffu, e2, 1), d0 = __shfl_down_sync(0xffffffffu, w0, 1);
+            const float e1 = w1 + (l.left ? u2 : 0.0f) + (l.right ? d0 : 0.0f);
+            float *row = bar + (plane + (b < 3 ? b : s.y.last) * sy);
+            if (e1 != 0.0f) atomicAdd(row + 1, e1);
+            // what no neighbour takes: the first tap of a run, the last two of its end
+            const float out = l.left ? w3 : w0;
+            if (ends && out != 0.0f) atomicAdd(row + (l.left ? s.x.last : 0), out);
+            if (!l.right && e2 != 0.0f) atomicAdd(row + 2, e2);
+            if (alone && w3 != 0.0f) atomicAdd(row + s.x.last, w3);
+        }
+    }
 }
 
 // q = p + (h/2) v(p) + (h/2) v(p2), p2 = p + h v(p).  Reverse mode:
@@ -261,58 +324,67 @@ __device__ __forceinline__ void scatter_sample(float *__restrict__ bar, const St
 //   q_bar -> v2_bar = (h/2) q_bar;  p2_bar = q_bar/2 + J_v(p2)^T v2_bar
 //   v1_bar = (h/2) q_bar' ... folded: v1_bar = h * p2_bar (p2 = p + h v1)
 // The centre read v(p) is an exact node value, so its adjoint is a single add.
-__global__ void __launch_bounds__(128) k_warp_vjp(const Dim3i d, const float *__restrict__ vel,
-                                                  const float *__restrict__ src, int nc, float dt,
-                                                  const float *__restrict__ out_bar,
-                                                  float *__restrict__ src_bar,
-                                                  float *__restrict__ vel_bar) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y, k = blockIdx.z;
-    if (i >= d.x) return;
-    const size_t n = (size_t)d.x * d.y * d.z;
+// One pass over the velocity taps gives the trace and the gradients, which only
+// the reverse step uses.  Per voxel 256 taps, and 64 row sums of 2 to 3 atomic
+// instructions, which bound it.  us, every tap an atomic, the velocity sampled
+// again for its gradients, rows of 128 voxels -> this: 60 x 50 x 55 121 -> 79,
+// 112 x 128 x 96 629 -> 401 (motion of 8 voxels: 793 -> 512), 256^3 6281 -> 4062.
+// Five blocks per SM (96 registers): four 414, three 481, six 416 at 112 x 128 x 96.
+__global__ void __launch_bounds__(WARP_BX *WARP_BY, 5) k_warp_vjp(const Dim3i d, const float *__restrict__ vel,
+                                                               const float *__restrict__ src, int nc, float dt,
+                                                               const float *__restrict__ out_bar,
+                                                               float *__restrict__ src_bar,
+                                                               float *__restrict__ vel_bar) {
+    const int i = blockIdx.x * WARP_BX + threadIdx.x;
+    const int j = blockIdx.y * WARP_BY + threadIdx.y, k = blockIdx.z;
+    const bool live = i < d.x && j < d.y;
+    const int n = d.x * d.y * d.z;
     const float h = -dt;
-    float q[3], p2[3], v1[3], v2[3];
-    trace(d, vel, n, i, j, k, h, q, p2, v1, v2);
-    bool cq[3];
-    float gq[3] = {to_grid(q[0], d.x, &cq[0]), to_grid(q[1], d.y, &cq[1]), to_grid(q[2], d.z, &cq[2])};
-    Stencil sq;
-    make_stencil(d, gq, sq);
+    // cell centre (warping.h:25-29) and the velocity there (an exact node read)
+    const float p[3] = {(float)i + 0.5f, (float)j + 0.5f, (float)k + 0.5f};
+    const int ci = min(max(i, 1), d.x - 2), cj = min(max(j, 1), d.y - 2), ck = min(max(k, 1), d.z - 2);
+    const int centre = ci + cj * d.x + ck * d.x * d.y;
+    float p2[3], q[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) p2[a] = __fadd_rn(p[a], __fmul_rn(h, __ldg(vel + (size_t)a * n + centre)));
+    CellD s2, sq;
+    cell_d(d, p2, s2);
+    SampleD v2[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        sample_d(d, vel + (size_t)a * n, s2, v2[a]);
+        const float p0 = __fsub_rn(p2[a], __fmul_rn(h, v2[a].value));
+        q[a] = __fadd_rn(p2[a], __fmul_rn(0.5f, __fsub_rn(p[a], p0)));
+    }
+    cell_d(d, q, sq);
     const size_t o = i + (size_t)j * d.x + (size_t)k * d.x * d.y;
     float qbar[3] = {0.0f, 0.0f, 0.0f};
     for (int c = 0; c < nc; ++c) {
-        const float ob = __ldg(out_bar + o + c * n);
-        if (ob == 0.0f) continue;
+        const float ob = live ? __ldg(out_bar + o + (size_t)c * n) : 0.0f;
         SampleD r;
-        sample_d(src + c * n, sq, cq, r);
-        if (src_bar) scatter_sample(src_bar + c * n, sq, r, ob);
-        qbar[0] += ob * r.grad[0];
-        qbar[1] += ob * r.grad[1];
-        qbar[2] += ob * r.grad[2];
+        r.corner = -1;
+        if (ob != 0.0f) {
+            sample_d(d, src + (size_t)c * n, sq, r);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) qbar[a] += ob * r.grad[a];
+        }
+        if (src_bar) scatter_sample(d, src_bar + (size_t)c * n, sq, r, ob, live);
     }
     if (!vel_bar) return;
-    if (qbar[0] == 0.0f && qbar[1] == 0.0f && qbar[2] == 0.0f) return;
-    bool c2[3];
-    float g2[3] = {to_grid(p2[0], d.x, &c2[0]), to_grid(p2[1], d.y, &c2[1]), to_grid(p2[2], d.z, &c2[2])};
-    Stencil s2;
-    make_stencil(d, g2, s2);
-    float v2bar[3], p2bar[3] = {0.5f * qbar[0], 0.5f * qbar[1], 0.5f * qbar[2]};
+    const bool moves = qbar[0] != 0.0f || qbar[1] != 0.0f || qbar[2] != 0.0f;
+    float p2bar[3] = {0.5f * qbar[0], 0.5f * qbar[1], 0.5f * qbar[2]};
 #pragma unroll
-    for (int a = 0; a < 3; ++a) v2bar[a] = 0.5f * h * qbar[a];
-#pragma unroll 1
     for (int a = 0; a < 3; ++a) {
-        SampleD r;
-        sample_d(vel + a * n, s2, c2, r);
-        scatter_sample(vel_bar + a * n, s2, r, v2bar[a]);
-        p2bar[0] += v2bar[a] * r.grad[0];
-        p2bar[1] += v2bar[a] * r.grad[1];
-        p2bar[2] += v2bar[a] * r.grad[2];
+        const float v2bar = 0.5f * h * qbar[a];
+        scatter_sample(d, vel_bar + (size_t)a * n, s2, v2[a], v2bar, moves);
+#pragma unroll
+        for (int e = 0; e < 3; ++e) p2bar[e] += v2bar * v2[a].grad[e];
     }
-    const int ci = min(max(i, 1), d.x - 2), cj = min(max(j, 1), d.y - 2), ck = min(max(k, 1), d.z - 2);
-    const size_t cc = ci + (size_t)cj * d.x + (size_t)ck * d.x * d.y;
+    if (!moves) return;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        float g = h * p2bar[a];
-        if (g != 0.0f) atomicAdd(vel_bar + a * n + cc, g);
+        const float g = h * p2bar[a];
+        if (g != 0.0f) atomicAdd(vel_bar + (size_t)a * n + centre, g);
     }
 }
 
@@ -359,8 +431,8 @@ cudaError_t launch_warp(const int *dim, const float *vel, const unsigned short *
 cudaError_t launch_warp_vjp(const int *dim, const float *vel, const float *src, int nc, float dt,
                             const float *out_bar, float *src_bar, float *vel_bar, cudaStream_t s) {
     Dim3i d{dim[0], dim[1], dim[2]};
-    k_warp_vjp<<<dim3((d.x + 127) / 128, d.y, d.z), 128, 0, s>>>(d, vel, src, nc, dt, out_bar,
-                                                                  src_bar, vel_bar);
+    const dim3 grid((d.x + WARP_BX - 1) / WARP_BX, (d.y + WARP_BY - 1) / WARP_BY, d.z), block(WARP_BX, WARP_BY);
+    k_warp_vjp<<<grid, block, 0, s>>>(d, vel, src, nc, dt, out_bar, src_bar, vel_bar);
     return cudaGetLastError();
 }
 
