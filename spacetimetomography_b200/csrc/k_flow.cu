@@ -219,11 +219,13 @@ __global__ void __launch_bounds__(128) k_flow_setup(const Dims d, const FlowRoi 
 struct Dual {
     float y[10];
 };
-__device__ __forceinline__ float4 ld4(const float4 *p) { return __ldg(p); }
+// Chained launches overlap the one ahead: cached loads that are ordered after the
+// wait, not the read-only path.
+__device__ __forceinline__ float4 ld4(const float4 *p) { return __ldca(p); }
 __device__ __forceinline__ Dual load_dual(const float *y, unsigned n, unsigned p) {
     const float4 *ya = reinterpret_cast<const float4 *>(y), *yb = ya + n;
     const float4 a = ld4(ya + p), b = ld4(yb + p);
-    const float2 c = __ldg(reinterpret_cast<const float2 *>(yb + n) + p);
+    const float2 c = __ldca(reinterpret_cast<const float2 *>(yb + n) + p);
     return Dual{{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y}};
 }
 __device__ __forceinline__ void store_dual(float *y, unsigned n, unsigned p, const float yn[9], float y4) {
@@ -293,7 +295,7 @@ __global__ void __launch_bounds__(128) k_flow_primal(const Dims d, const FlowRoi
                                                      const int *__restrict__ done) {
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
-    if (*done) return;
+    if (__ldca(done)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
     float pr = 0.0f;
@@ -311,7 +313,7 @@ __global__ void __launch_bounds__(128) k_flow_primal(const Dims d, const FlowRoi
             const float kt = kty_of(a.y + 3 * c, b, i, j, k, d, uc[c], a.y[9]);
             vn[c] = vo[c] - t[c] * kt;
             if (flags & kResid) {
-                const float r = fabsf((vo[c] - vn[c]) / t[c] - kty[p + (size_t)c * n] + kt);
+                const float r = fabsf((vo[c] - vn[c]) / t[c] - __ldca(kty + p + (size_t)c * n) + kt);
                 pr = c == 0 ? r : pr + r;
             }
             if (flags & kKeepKty) kty[p + (size_t)c * n] = kt;
@@ -366,7 +368,7 @@ __global__ void __launch_bounds__(128) k_flow_dual(const Dims d, const float4 *_
                                                    double *__restrict__ resid, const int *__restrict__ done) {
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
-    if (*done) return;
+    if (__ldca(done)) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int j = blockIdx.y, k = blockIdx.z;
     float dr = 0.0f;
@@ -381,8 +383,8 @@ __global__ void __launch_bounds__(128) k_flow_dual(const Dims d, const float4 *_
         spread(zero_old ? zero : ld4(v_old + p), oc), spread(zero_old ? zero : ld4(v_old + p + ox), oxv);
         spread(zero_old ? zero : ld4(v_old + p + oy), oyv), spread(zero_old ? zero : ld4(v_old + p + oz), ozv);
         const float4 *ya = reinterpret_cast<const float4 *>(y), *yb = ya + n;
-        const float4 y0 = ya[p], y1 = yb[p];
-        const float2 y2 = reinterpret_cast<const float2 *>(yb + n)[p];
+        const float4 y0 = ld4(ya + p), y1 = ld4(yb + p);
+        const float2 y2 = __ldca(reinterpret_cast<const float2 *>(yb + n) + p);
         const float yo[10] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w, y2.x, y2.y};
         const float4 up = ld4(u + p);
         const float s2 = ld4(steps + p).w;
@@ -403,7 +405,7 @@ __global__ void __launch_bounds__(128) k_flow_dual(const Dims d, const float4 *_
         }
         const float k4 = up.x * vc[0] + up.y * vc[1] + up.z * vc[2];
         float k4o = 0.0f;
-        if (flags & kFirstOfWarp) k4o = __ldg(k4prev + p);
+        if (flags & kFirstOfWarp) k4o = __ldca(k4prev + p);
         else if (!zero_old) k4o = up.x * oc[0] + up.y * oc[1] + up.z * oc[2];
         const float y4 = smax(-1.0f, smin(1.0f, yo[9] + s2 * (k4 + k4 - k4o + up.w)));
         store_dual(y, n, p, yn, y4);
@@ -445,7 +447,7 @@ __global__ void __launch_bounds__(32 * (STEP_Y + 1), 4)
                 float *__restrict__ kty, const DualPar q, int flags, int planes, const int *__restrict__ done) {
     __shared__ float below[2][STEP_Y + 1][3][32];
     cudaGridDependencySynchronize();
-    if (*done) return;
+    if (__ldca(done)) return;
     const int lane = threadIdx.x, row = threadIdx.y;
     const int i0 = (int)blockIdx.x * 31 + lane - 1, j0 = (int)blockIdx.y * STEP_Y + row - 1;
     const bool own = lane > 0 && row > 0 && i0 < d.x && j0 < d.y;
@@ -487,7 +489,7 @@ __global__ void __launch_bounds__(32 * (STEP_Y + 1), 4)
         }
         const float k4 = up.x * a[0] + up.y * a[1] + up.z * a[2];
         float k4o = 0.0f;
-        if (flags & kFirstOfWarp) k4o = __ldg(k4prev + p);
+        if (flags & kFirstOfWarp) k4o = __ldca(k4prev + p);
         else if (!zero_old) k4o = up.x * e[0] + up.y * e[1] + up.z * e[2];
         const float y4 = smax(-1.0f, smin(1.0f, yo.y[9] + sp.w * (k4 + k4 - k4o + up.w)));
         float uc[3], t[3];

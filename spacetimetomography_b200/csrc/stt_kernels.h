@@ -18,7 +18,9 @@ struct PdParams {
 // A launch that may start before the kernel ahead of it in the stream has
 // finished: its blocks take the places that kernel's last blocks leave, and wait
 // in cudaGridDependencySynchronize(), which the kernel calls before it touches
-// anything another kernel writes or reads, until it has.  A kernel that calls
+// anything another kernel writes or reads, until it has.  What that kernel writes is
+// read after the wait and not through the read-only or texture path, whose data may
+// not change while a grid runs.  A kernel that calls
 // cudaTriggerProgrammaticLaunchCompletion() lets its successor come up early.
 template <typename... Params, typename... Args>
 cudaError_t launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, cudaStream_t s, Args &&...args) {
