@@ -196,6 +196,7 @@ __global__ void __launch_bounds__(32 * SPLIT_P) k_fp_split(const GeomDev g, cons
     int count;
     const float sum = fp_ray_sum_split<SPLIT_P, SPLIT_G>(
         g, [=](int, const FpCell &c, float w[8]) { fp_corners_tex<T>(t, nx, c, w); }, r, hit, part, lane, vals, count);
+    cudaTriggerProgrammaticLaunchCompletion();
     if (part == 0 && pixel) out.write(g, i + (size_t)j * g.W, hit, r.tfar - r.tnear, sum, count);
 }
 

@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(32 * NW) k_fp_corr(const GeomDev g, const View
     } else {
         L = raylen_state ? raylen_state[pix] : 0.0f;
     }
+    cudaTriggerProgrammaticLaunchCompletion();
     corr[pix] = __fdiv_rn(__fsub_rn(ld_voxel(b + pix), sum), __fadd_rn(L, 1.0f));
 }
 

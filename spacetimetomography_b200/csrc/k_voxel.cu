@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, con
                                                             T *__restrict__ mirror, size_t mpitch) {
     __shared__ float table[BP_ROWS * 4 * BP_PITCH];
     constexpr int RS = 4 * BP_PITCH;  // one row of every column
+    cudaGridDependencySynchronize();  // (a chained launch)
     int local;
     const ViewRec &v = views[sel_view(sel, local)];
     const int y0 = blockIdx.y * K, y1 = min(y0 + K, g.ny);
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, con
             unsigned o = (unsigned)(c.r0 * g.W + px - 1);  // (W H < 2^31)
 #pragma unroll 4
             for (int i = 0; i < c.nr; ++i, o += g.W) {
-                const float t[4] = {__ldg(corr + o), __ldg(corr + o + 1), __ldg(corr + o + 2), __ldg(corr + o + 3)};
+                const float t[4] = {__ldca(corr + o), __ldca(corr + o + 1), __ldca(corr + o + 2), __ldca(corr + o + 3)};
                 row[RS * i] = bp_row(t, wx);
             }
         }
@@ -292,13 +293,15 @@ namespace {
 template <int K, int OCC, typename T>
 cudaError_t bp_cols(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr, T *vol, float alpha,
                     float gmax, cudaStream_t s, T *mirror) {
+    // Chained to the projection that writes corr: 128 views of 128^2 at 128^3 3.46
+    // -> 3.21 ms.  (The projection is not chained to this: it reads the volume
+    // through the texture path.)
     const dim3 grid((g.nx + 31) / 32, (g.ny + K - 1) / K, (g.nz + 3) / 4);
     if (mirror)
-        k_bp_voxel_cols<K, OCC, T, true><<<grid, 128, 0, s>>>(g, views, sel, corr, vol, alpha, gmax, mirror,
-                                                              fp_mirror_pitch((size_t)g.nx * g.ny));
-    else
-        k_bp_voxel_cols<K, OCC, T, false><<<grid, 128, 0, s>>>(g, views, sel, corr, vol, alpha, gmax, mirror, 0);
-    return cudaGetLastError();
+        return launch_chained(k_bp_voxel_cols<K, OCC, T, true>, grid, 128, s, g, views, sel, corr, vol, alpha, gmax, mirror,
+                              fp_mirror_pitch((size_t)g.nx * g.ny));
+    return launch_chained(k_bp_voxel_cols<K, OCC, T, false>, grid, 128, s, g, views, sel, corr, vol, alpha, gmax, mirror,
+                          (size_t)0);
 }
 
 template <typename T>

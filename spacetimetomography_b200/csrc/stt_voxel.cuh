@@ -200,7 +200,7 @@ struct BpRowsLdg {
     __device__ __forceinline__ void operator()(int px, int pyr, float r[4]) const {
         const float *c = corr + (size_t)pyr * W + (px - 1);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) r[a] = __ldg(c + a);
+        for (int a = 0; a < 4; ++a) r[a] = __ldca(c + a);
     }
 };
 // From the correction array with plain loads (written by the same launch).
