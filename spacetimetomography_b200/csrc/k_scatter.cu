@@ -226,13 +226,19 @@ __device__ __forceinline__ void scatter_column(const GeomDev &g, const ViewRec &
 }
 
 // Rays a thread: enough to merge where rows lie close, as long as the launch
-// still fills the GPU (the measurements above, and 128^3 / 128^2, rows 1.2 voxels
-// apart: one ray a thread 47/59/51 us, two 99/126/73).
+// still fills the GPU.  Backprojection of one view with 1 / 2 / 4, us, mean of six
+// views: rows 0.6 voxels apart 65,536 rays 130/129/193, 102,400 226/208/256,
+// 147,456 363/289/308, 200,704 575/439/417; 0.9 apart 65,536 205/203/287, 90,000
+// 319/304/381; 1.2 apart (128^2 at 128^3) 52/99.  The adjoint of dense residuals the same:
+// one view of 65,536 rays 0.9 apart 172/176/235, four 515/410/430; of residuals with
+// empty surroundings, whose zeros a ray a thread skips: one view 72/123/209, twelve
+// 283/300/334 (402/392 where the volume is not in the L2), four 0.6 apart
+// 625/538/478.
 int merged_rays(const GeomDev &g, int nviews) {
     const long long rays = (long long)g.W * g.H * nviews;
     if (!((long long)g.nx * g.nz < (1LL << 31))) return 1;  // (32-bit cell keys)
-    if (g.row_pitch < CLOSE_ROWS && rays >= 150000) return 4;
-    if (g.row_pitch < 1.05f && rays >= 60000) return 2;
+    if (g.row_pitch < CLOSE_ROWS && rays >= 180000) return 4;
+    if (g.row_pitch < 1.05f && rays >= 90000) return 2;
     return 1;
 }
 

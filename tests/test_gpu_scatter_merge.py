@@ -18,10 +18,11 @@ import oracle_bind as ob
 pytestmark = pytest.mark.gpu
 
 CASES = [  # dims, detector, pixel, spacing, offset: rows per voxel and rays choose how many merge; in patches
-    ((40, 36, 44), (403, 389), 0.25, 1.0, (0.0, 0.0, 0.0), False),   # four rays a thread
-    ((24, 50, 17), (391, 401), 0.33, 1.3, (1.5, -2.0, 0.7), False),  # four, a ragged last column of rows
-    ((33, 20, 31), (253, 241), 1.5, 1.0, (0.3, 0.1, -0.4), False),   # two; most rays miss
+    ((40, 36, 44), (403, 389), 0.25, 1.0, (0.0, 0.0, 0.0), False),   # two rays a thread, the adjoint four
+    ((24, 50, 17), (391, 401), 0.33, 1.3, (1.5, -2.0, 0.7), False),  # the same, a ragged last column of rows
+    ((33, 20, 31), (253, 241), 1.5, 1.0, (0.3, 0.1, -0.4), False),   # one, the adjoint two; most rays miss
     ((2, 2, 2), (390, 386), 0.02, 1.0, (0.0, 0.0, 0.0), True),   # every cell on a face
+    ((40, 36, 44), (431, 421), 0.23, 1.0, (0.2, 0.0, -0.3), False),  # four
 ]
 ANGLES = np.array([0.0, 0.6, np.pi / 2, 3.9])
 
