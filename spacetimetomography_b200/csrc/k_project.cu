@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(128) k_fp(const GeomDev g, const ViewRec *__re
         if constexpr (TX)
             sum = fp_ray_sum_tex<8, true, T>(g, tex, r, &count);
         else
-            sum = fp_ray_sum<I>(g, vr, vol, vol_t, r, &count);
+            sum = fp_ray_sum<I, sizeof(T) == 4 ? 2 : FP_GROUP>(g, vr, vol, vol_t, r, &count);  // (FP_DEFAULT_LOADS)
     }
     const size_t o = (size_t)v * g.W * g.H + i + (size_t)j * g.W;
     proj[o] = sum;

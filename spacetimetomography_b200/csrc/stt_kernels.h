@@ -156,6 +156,14 @@ cudaError_t launch_fp_corr_split(const GeomDev &g, const ViewRec *views, const V
 // 192^3 / 256^2 45/93/66 -> 31/36/30, 256^3 / 512^2 124/213/176 -> 118/122/116
 // (the times before include the z-fastest copy of the views along x).
 constexpr int FP_DEFAULT_TEX = 10;
+// And where no texture binds (slices past the texture width): loads with two
+// samples in flight.  Both forms have 64 registers, so the warps are as many; four
+// samples' 32 loads a thread only lengthen the bursts that share the L1.
+// Views at 0 and 90 degrees, us, four in flight -> two: 128^3 / 128^2 31/47 -> 26/37,
+// 256^3 / 512^2 118/171 -> 108/160, 400^3 / 800^2 459/614 -> 406/531, 512^3 / 1024^2
+// 895/1177 -> 793/1008 (the oblique views are staged, 1230); a BF16 volume's loads
+// gain nothing (765/964 -> 771/953) and keep four.
+constexpr int FP_DEFAULT_LOADS = 5;
 // Forward projection of one view fused with the SART correction.  With usable
 // slab maps, staged views run in the slab-staged kernel and the others in the
 // gather kernel (both are launched; each leaves the other's views alone).

@@ -191,7 +191,7 @@ const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, unsigned short **mirro
 FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds) {
     if (ctx->tuned) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), ctx->staged_bins != 0};
     if (tex_binds) return {FP_DEFAULT_TEX, true, false};
-    return {0, false, ctx->staged_bins != 0};
+    return {FP_DEFAULT_LOADS, false, ctx->staged_bins != 0};
 }
 
 FpChoice fp_choice(const stt_ctx *ctx, const unsigned short *, bool tex_binds) {
