@@ -540,7 +540,7 @@ void destroy_fp_tex(FpTex &t) {
 cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t,
                            const ViewSel &sel, const float *b_stack, float *raylen_state, float *corr,
                            cudaStream_t s, const FpSlabMaps *maps, int *status,
-                           int fp_variant, const FpTex *tex) {
+                           int fp_variant, const FpTex *tex, int chains) {
     const int skip = maps && maps->ok && maps->esize == 4 && (!vol_t || maps->has_z);
     // a texture variant without a usable texture runs the load-based variant of the same shape
     if (is_tex_fp_variant(fp_variant) && !(tex && tex->ok && tex->esize == 4)) fp_variant = fp_variant == 10 ? 4 : 8;
@@ -555,7 +555,7 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *
                                                             skip, FpTex{});
         return cudaGetLastError();
     }
-    if (is_tex_fp_variant(fp_variant) && (long long)g.W * g.H <= FP_SPLIT_RAYS)
+    if (is_tex_fp_variant(fp_variant) && (long long)g.W * g.H <= fp_split_rays(chains))
         return launch_fp_corr_split(g, views, sel, b_stack, raylen_state, corr, s, tx, skip);
     switch (fp_variant) {
     case 1: fp_corr_variant<32, 2, 4>(g, views, vol, vol_t, sel, b_stack, raylen_state, corr, s, skip); break;
@@ -620,7 +620,7 @@ cudaError_t launch_correction(long long n, const unsigned short *b, const float 
 cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigned short *vol,
                            const unsigned short *vol_t, const ViewSel &sel, const unsigned short *b_stack,
                            float *raylen_state, float *corr, cudaStream_t s,
-                           const FpSlabMaps *maps, int *status, int fp_variant16, const FpTex *tex) {
+                           const FpSlabMaps *maps, int *status, int fp_variant16, const FpTex *tex, int chains) {
     typedef unsigned short U;
     const int skip = maps && maps->ok && maps->esize == 2 && (!vol_t || maps->has_z);
     if (skip) {
@@ -630,7 +630,7 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigne
     }
     if (fp_variant16 == 1 && tex && tex->ok && tex->esize == 2 && small_volume(g)) {
         const FpTex tx = *tex;
-        if ((long long)g.W * g.H <= FP_SPLIT_RAYS)
+        if ((long long)g.W * g.H <= fp_split_rays(chains))
             return launch_fp_corr_split(g, views, sel, b_stack, raylen_state, corr, s, tx, skip);
         constexpr int WX = 8, NW = 4, TH = (32 / WX) * NW;
         k_fp_corr<int, WX, NW, 8, true, U, U, true><<<dim3((g.W + WX - 1) / WX, (g.H + TH - 1) / TH, 1), 32 * NW, 0, s>>>(

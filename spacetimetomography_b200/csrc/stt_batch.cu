@@ -52,6 +52,7 @@ struct stt_batch {
 
 extern "C" stt_status stt_internal_set_error(stt_ctx *ctx, stt_status st, const char *msg);
 extern "C" stt_status stt_internal_solver_presweep(stt_solver *s, void *stream);
+extern "C" void stt_internal_solver_chains(stt_solver *s, int chains);
 extern "C" int stt_internal_solver_jobs(const stt_solver *s, void *jobs);
 extern "C" void stt_internal_solver_end_iteration(stt_solver *s);
 
@@ -342,6 +343,7 @@ stt_status stt_batch_create(const stt_instance *instances, int n, int mode, stt_
         if (e != cudaSuccess) return bail(STT_ERR_CUDA, std::string("instance set-up: ") + cudaGetErrorString(e));
         stt_status st = make_solver(in, persistent);
         if (st) return bail(st, "instance " + std::to_string(i) + ": " + stt_last_error(I.ctx));
+        stt_internal_solver_chains(in.solver, n);
     }
     if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
         return bail(STT_ERR_CUDA, "event create");

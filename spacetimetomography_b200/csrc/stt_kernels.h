@@ -142,6 +142,16 @@ void destroy_fp_tex(FpTex &t);
 // Projections of at most this many rays in one launch share each ray between
 // the 4 warps of a block when their corners come from a texture (k_fp_split.cu).
 constexpr long long FP_SPLIT_RAYS = 24576;
+// Of `chains` sequences of views that run side by side (a solver's frames, a
+// batch's instances) each gets a share of the GPU, which the steps that the warps
+// repeat waste: eight cubes of 65 to 124 voxels, views of 80^2 to 160^2, all split
+// 3.47 ms, up to 8192 rays 3.05, none 3.13; but three of 70^2 to 141^2 1.41, 1.58,
+// 1.78; five of 51^2 to 102^2 0.98, 0.99, 1.14.
+constexpr long long FP_SPLIT_SHARED_RAYS = 65536;
+inline long long fp_split_rays(int chains) {
+    const long long share = FP_SPLIT_SHARED_RAYS / (chains > 1 ? chains : 1);
+    return share < FP_SPLIT_RAYS ? share : FP_SPLIT_RAYS;
+}
 cudaError_t launch_fp_split(const GeomDev &g, const ViewRec *views, int view0, int nviews, float *proj, float *raylen,
                             float *weight, cudaStream_t s, const FpTex &tex);
 cudaError_t launch_fp_corr_split(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *b_stack,
@@ -173,10 +183,8 @@ constexpr int FP_DEFAULT_LOADS = 5;
 cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t,
                            const ViewSel &sel, const float *b_stack, float *raylen_state, float *corr,
                            cudaStream_t s, const FpSlabMaps *maps = nullptr,
-                           int *status = nullptr, int fp_variant = 0, const FpTex *tex = nullptr);
-cudaError_t launch_fp_corr_split(const GeomDev &g, const ViewRec *views, const float *vol, const float *vol_t,
-                                 const ViewSel &sel, const float *b_stack, float *raylen_state, float *corr,
-                                 cudaStream_t s, const FpTex *tex, int form);
+                           int *status = nullptr, int fp_variant = 0, const FpTex *tex = nullptr,
+                           int chains = 1);
 cudaError_t launch_transpose(const GeomDev &g, const float *in, float *out, cudaStream_t s);
 cudaError_t launch_fp(const GeomDev &g, const ViewRec *views, const unsigned short *vol, const unsigned short *vol_t,
                       int view0, int nviews, float *proj, float *raylen, float *weight, cudaStream_t s,
@@ -209,7 +217,7 @@ cudaError_t launch_fp_corr(const GeomDev &g, const ViewRec *views, const unsigne
                            const unsigned short *vol_t, const ViewSel &sel, const unsigned short *b_stack,
                            float *raylen_state, float *corr, cudaStream_t s,
                            const FpSlabMaps *maps = nullptr, int *status = nullptr, int fp_variant16 = 0,
-                           const FpTex *tex = nullptr);
+                           const FpTex *tex = nullptr, int chains = 1);
 cudaError_t launch_correction(long long n, const unsigned short *b, const float *ax, const float *raylen,
                               float *corr, cudaStream_t s);
 cudaError_t launch_correction(long long n, const float *b, const float *ax, const float *raylen,

@@ -91,6 +91,7 @@ struct stt_solver {
     int *status = nullptr;     // raised by a bounded device-side wait that gave up
     unsigned long long host_iter = 0;
     std::vector<cudaStream_t> streams;
+    int chains = 1;            // view sequences that run beside one another: the frames here, or a batch's instances
     std::vector<cudaEvent_t> ev_dual, ev_done;
     cudaEvent_t ev_fork = nullptr;
     cudaGraph_t graph = nullptr;
@@ -207,7 +208,7 @@ int fp_corr(stt_solver *s, int f, const float *vol, const float *volt, const stt
             float *rl, float *corr, cudaStream_t cs, cudaError_t &e) {
     const stt::FpSlabMaps *maps = s->fpmaps.empty() ? nullptr : &s->fpmaps[f];
     e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status, s->fp.variant,
-                            s->fp.tex ? &s->fptex[f] : nullptr);
+                            s->fp.tex ? &s->fptex[f] : nullptr, s->chains);
     return (maps && maps->ok) ? 2 : 1;  // slab-staged + gather kernels, or gather only
 }
 
@@ -215,7 +216,7 @@ int fp_corr(stt_solver *s, int f, const unsigned short *vol, const unsigned shor
             const unsigned short *stack, float *rl, float *corr, cudaStream_t cs, cudaError_t &e) {
     const stt::FpSlabMaps *maps = s->fpmaps.empty() ? nullptr : &s->fpmaps[f];
     e = stt::launch_fp_corr(*s->g, s->views, vol, volt, sel, stack, rl, corr, cs, maps, s->status, s->fp.variant,
-                            s->fp.tex ? &s->fptex[f] : nullptr);
+                            s->fp.tex ? &s->fptex[f] : nullptr, s->chains);
     return (maps && maps->ok) ? 2 : 1;
 }
 
@@ -671,6 +672,7 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
     if (ce == cudaSuccess) ce = cudaMemset(s->counter, 0, sizeof(unsigned long long));
     if (ce == cudaSuccess) ce = cudaMemset(s->status, 0, sizeof(int));
     if (ce == cudaSuccess && s->acc) ce = cudaMemset(s->acc, 0, (size_t)F * s->n * sizeof(float2));
+    s->chains = s->cfg.mode == STT_SOLVE_PLAIN ? 1 : F;
     s->streams.resize(F);
     s->ev_dual.resize(F);
     s->ev_done.resize(F);
@@ -865,6 +867,9 @@ stt_status stt_solver_destroy(stt_solver *s) {
     delete s;
     return STT_OK;
 }
+
+// How many instances of a batch run beside this solver's frame (stt_batch.cu).
+void stt_internal_solver_chains(stt_solver *s, int chains) { s->chains = chains; }
 
 // Hooks of the batch's persistent form (stt_batch.cu), for a solver created
 // with STT_SOLVE_PERSISTENT: one iteration's steps before the sweep, joined
