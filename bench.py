@@ -512,12 +512,12 @@ def flow_bench(args, dev, stream, rank: int) -> dict:
     achieved = FLOW_BYTES_PER_VOXEL * N ** 3 / t_it / 1e9
     out = {"workload": f"L1Huber_OF level, {N}^3, ROI cut {cut}, {iters} iterations, 1 warp",
            "ms_per_iteration": 1000.0 * t_it, "gvoxel_iter_per_s": N ** 3 / t_it / 1e9,
-           "roofline": {"bound": "hbm", "kernel": "k_flow_primal + k_flow_dual", "achieved": achieved,
+           "roofline": {"bound": "hbm", "kernel": "k_flow_step", "achieved": achieved,
                         "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_source": peak_kind,
                         "algorithmic_bytes_per_voxel": FLOW_BYTES_PER_VOXEL,
-                        "moved_bytes_per_voxel": 212,
-                        "note": "moved per iteration: primal reads y 10, u 3, tau 3, v 3 and writes v 3 (ROI); "
-                                "dual reads v 3, v_old 3, u 4, sigma2 1, y 10 and writes y 10"}}
+                        "moved_bytes_per_voxel": 160,
+                        "note": "moved per iteration: reads y 10, v 4, v_old 4, u 4, steps 4 and writes y 10, v 4 "
+                                "(the vectors are padded to 16 bytes)"}}
     # the whole multiscale solve between the same frames with the reference's
     # parameters (tol 0.1, 3000 iterations, 3 warps, 3 scales, the ROI cut):
     # the warps stop on their residuals
