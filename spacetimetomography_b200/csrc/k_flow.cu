@@ -87,10 +87,12 @@ __device__ __forceinline__ void box_cell(const Dims &d, const float box[3], cons
 }
 
 // warping::sample_image: the cubic value clamped to the min/max of the cell's 8
-// corners, which are taps of the stencil.  Rows go in pairs of planes.
+// corners, which are taps of the stencil.  Rows go in pairs of planes.  I: the
+// offsets inside a plane of voxels (int below 2^31 of them, else long long).
+template <typename I>
 __device__ __forceinline__ float sample_box(const float *__restrict__ img, const Dims &d, const BoxCell &q, float nz) {
-    const int sy = d.x, sz = d.x * d.y;
-    const int at = q.o[0] + q.o[1] * sy + q.o[2] * sz;
+    const I sy = d.x, sz = (I)d.x * d.y;
+    const I at = q.o[0] + q.o[1] * sy + q.o[2] * sz;
     const float dx = q.d[0], dy = q.d[1], dz = q.d[2];
     float zv[4], corner[8];
 #pragma unroll
@@ -98,7 +100,7 @@ __device__ __forceinline__ float sample_box(const float *__restrict__ img, const
         float2 yv[4];
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
-            const int row = at + (b < 3 ? b : q.last[1]) * sy;
+            const I row = at + (b < 3 ? b : q.last[1]) * sy;
             const float *r0 = img + (row + c * sz), *r1 = img + (row + (c == 0 ? 1 : q.last[2]) * sz);
             const float2 t0 = make_float2(__ldg(r0), __ldg(r1)), t1 = make_float2(__ldg(r0 + 1), __ldg(r1 + 1));
             float2 t2 = make_float2(__ldg(r0 + 2), __ldg(r1 + 2));
@@ -138,6 +140,7 @@ __device__ __forceinline__ float sample_box(const float *__restrict__ img, const
 // -> 53, 128^3 628 -> 300, 147 x 121 x 135 1289 -> 438, 256^3 5301 -> 2228 (scalar
 // cubics 128^3 414; blocks of 32 x 4 in 168 registers 304, in 96 or 80 313).
 constexpr int BOX_X = 32, BOX_Y = 8;
+template <typename I>
 __global__ void __launch_bounds__(BOX_X *BOX_Y, 2)
     k_warp_box(const Dims d, const float bx, const float by, const float bz, const float *__restrict__ vel,
                const float *__restrict__ src, int nc, float dt, float *__restrict__ out, float nz) {
@@ -160,12 +163,12 @@ __global__ void __launch_bounds__(BOX_X *BOX_Y, 2)
     const float h = -dt;
     box_cell(d, box, p, cell);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) v[c] = sample_box(vel + c * n, d, cell, nz);
+    for (int c = 0; c < 3; ++c) v[c] = sample_box<I>(vel + c * n, d, cell, nz);
 #pragma unroll
     for (int c = 0; c < 3; ++c) p2[c] = p[c] + h * v[c];
     box_cell(d, box, p2, cell);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) v[c] = sample_box(vel + c * n, d, cell, nz);
+    for (int c = 0; c < 3; ++c) v[c] = sample_box<I>(vel + c * n, d, cell, nz);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const float p0 = p2[c] - h * v[c];
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(BOX_X *BOX_Y, 2)
     }
     box_cell(d, box, q, cell);
     const long long o = i + (long long)j * d.x + (long long)k * d.x * d.y;
-    for (int c = 0; c < nc; ++c) out[o + c * n] = sample_box(src + c * n, d, cell, nz);
+    for (int c = 0; c < nc; ++c) out[o + c * n] = sample_box<I>(src + c * n, d, cell, nz);
 }
 
 // ---- per-warp setup (optical_flow.h:257-297) ---------------------------------
@@ -714,8 +717,9 @@ inline dim3 vox_grid(const int *d, int zmul = 1) {
 cudaError_t launch_warp_box(const int *dim, const float *box, const float *vel, const float *src, int nc, float dt,
                             float *out, cudaStream_t s) {
     const dim3 grid((dim[0] + BOX_X - 1) / BOX_X, (dim[1] + BOX_Y - 1) / BOX_Y, dim[2]);
-    k_warp_box<<<grid, dim3(BOX_X, BOX_Y), 0, s>>>(Dims{dim[0], dim[1], dim[2]}, box[0], box[1], box[2], vel, src, nc, dt,
-                                             out, -0.0f);
+    const auto kernel = (long long)dim[0] * dim[1] * dim[2] < (1LL << 31) ? k_warp_box<int> : k_warp_box<long long>;
+    kernel<<<grid, dim3(BOX_X, BOX_Y), 0, s>>>(Dims{dim[0], dim[1], dim[2]}, box[0], box[1], box[2], vel, src, nc, dt,
+                                               out, -0.0f);
     return cudaGetLastError();
 }
 
