@@ -82,10 +82,10 @@ __global__ void __launch_bounds__(128, OCC) k_bp_voxel_cols(const GeomDev g, con
             float wx[4];
             bp_weights(upx - (float)px, wx);
             float *row = table + zl * BP_PITCH + xl;
-            unsigned o = (unsigned)(c.r0 * g.W + px - 1);  // (W H < 2^31)
+            const float *d = corr + (size_t)c.r0 * g.W + (px - 1);  // (a detector may have more than 2^32 pixels)
 #pragma unroll 4
-            for (int i = 0; i < c.nr; ++i, o += g.W) {
-                const float t[4] = {__ldca(corr + o), __ldca(corr + o + 1), __ldca(corr + o + 2), __ldca(corr + o + 3)};
+            for (int i = 0; i < c.nr; ++i, d += g.W) {
+                const float t[4] = {__ldca(d), __ldca(d + 1), __ldca(d + 2), __ldca(d + 3)};
                 row[RS * i] = bp_row(t, wx);
             }
         }
