@@ -13,8 +13,13 @@
  *   - `stream` is a cudaStream_t passed as void*; NULL is the legacy default
  *     stream.  Calls only enqueue work; nothing synchronises unless stated.
  *   - A context is used by one host thread at a time; different contexts may
- *     be used concurrently.  A context owns its geometry tables and the scratch
- *     accumulators of the ray-driven backprojector.
+ *     be used concurrently.  A context owns its geometry tables and scratch: the
+ *     accumulators of the ray-driven backprojector, the correction image of
+ *     stt_sart_sweep and stt_sart_view, the power iteration's images, the z-fastest
+ *     copy that projections without a texture make for views along x, and the
+ *     mirror of a volume whose slices a texture cannot step over.  Calls that use
+ *     the same scratch must not overlap on different streams, but for the mirror,
+ *     whose users wait for one another on the device.
  *
  * Reference interfaces replaced (paths relative to the reference project root
  * gmzang/SpaceTimeTomography, S/ = SpaceTimeTomography/):

@@ -141,9 +141,11 @@ stt_status stt_destroy(stt_ctx *ctx) {
     cudaFree(ctx->pwd);
     cudaFree(ctx->status);
     for (auto &e : ctx->fp_tex) stt::destroy_fp_tex(e.tex);
-    for (auto &m : ctx->mirror) {
+    for (auto &m : ctx->mirror) ctx->retired.push_back(m);
+    for (auto &m : ctx->retired) {
         stt::destroy_fp_tex(m.tex);
         cudaFree(m.p);
+        if (m.read) cudaEventDestroy(m.read);
     }
     delete ctx;
     return STT_OK;
@@ -332,16 +334,24 @@ static stt_status check_views(stt_ctx *ctx, int view0, int nviews) {
 }  // extern "C"
 
 // Where a call's projections fetch their corners: the volume's own texture, a
-// mirror's (made from the volume here; `mirror` set), or loads (tex null).
+// mirror's (made from the volume here; `mirror` set, the call's until the source
+// goes out of scope), or loads (tex null).
 template <typename T>
 struct FpSource {
     const stt::FpTex *tex = nullptr;
     T *mirror = nullptr;
+    stt_ctx *ctx;
+    cudaStream_t s;
+    FpSource(stt_ctx *ctx, cudaStream_t s) : ctx(ctx), s(s) {}
+    FpSource(const FpSource &) = delete;
+    FpSource &operator=(const FpSource &) = delete;
+    ~FpSource() {
+        if (mirror) stt::ctx_mirror_done(ctx, sizeof(T), s);
+    }
 };
 
 template <typename T>
 static stt_status fp_source(stt_ctx *ctx, const T *vol, cudaStream_t s, FpSource<T> &src) {
-    src = FpSource<T>{};
     if ((src.tex = stt::ctx_fp_tex(ctx, vol, s))) return STT_OK;
     if (!(src.tex = stt::ctx_mirror_tex(ctx, s, &src.mirror))) return STT_OK;
     STT_CUDA(ctx, stt::launch_mirror(ctx->g, vol, src.mirror, s), "k_mirror launch");
@@ -353,7 +363,7 @@ static stt_status fp_source(stt_ctx *ctx, const T *vol, cudaStream_t s, FpSource
 template <typename T>
 static stt_status project(stt_ctx *ctx, const T *vol, float *proj, float *raylen, float *weight, int view0, int nviews,
                           cudaStream_t s) {
-    FpSource<T> src;
+    FpSource<T> src(ctx, s);
     stt_status st = fp_source(ctx, vol, s, src);
     if (st) return st;
     const T *volt = nullptr;
@@ -367,7 +377,6 @@ static stt_status project(stt_ctx *ctx, const T *vol, float *proj, float *raylen
 // form is one.
 template <typename T>
 static stt_status corr_source(stt_ctx *ctx, const T *vol, cudaStream_t s, FpSource<T> &src) {
-    src = FpSource<T>{};
     return stt::fp_choice(ctx, vol, true).tex ? fp_source(ctx, vol, s, src) : STT_OK;
 }
 
@@ -418,7 +427,7 @@ stt_status stt_fp_correction(stt_ctx *ctx, const float *vol, const float *b, flo
     if (!vol || !b || !corr) return fail(ctx, STT_ERR_INVALID, "null vol, b or corr");
     if ((st = check_views(ctx, view, 1))) return st;
     if ((st = set_device(ctx))) return st;
-    FpSource<float> src;
+    FpSource<float> src(ctx, S(stream));
     if ((st = corr_source(ctx, vol, S(stream), src))) return st;
     return project_corr(ctx, vol, src, stt::ViewSel{view, nullptr, 0, view}, b, raylen_state, corr, S(stream));
 }
@@ -609,7 +618,7 @@ static stt_status sart_sweep_t(stt_ctx *ctx, T *vol, const T *proj_stack, const 
     const size_t npix = (size_t)ctx->g.W * ctx->g.H;
     if ((st = ensure(ctx, ctx->corr, ctx->corr_n, npix, "correction image"))) return st;
     if (bp_mode == 1 && (st = ensure_acc(ctx, s))) return st;
-    FpSource<T> src;
+    FpSource<T> src(ctx, s);
     if (nperm > 0 && (st = corr_source(ctx, static_cast<const T *>(vol), s, src))) return st;
     for (int i = 0; i < nperm; ++i) {
         const stt::ViewSel sel{view_offset + perm[i], nullptr, 0, view_offset};

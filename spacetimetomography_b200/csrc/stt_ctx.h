@@ -55,13 +55,20 @@ struct stt_ctx {
     static constexpr int kFpTexCache = 32;
     std::vector<FpTexEntry> fp_tex;
     // The mirror of a volume no texture binds (launch_mirror), by storage:
-    // [0] FP32, [1] BF16.  Written anew by every call that projects from it.
+    // [0] FP32, [1] BF16.  Written anew by every call that projects from it, on
+    // whatever stream, so a call first waits for `read`, recorded behind the last
+    // reader of the call before (as an external event in a stream capture, so a
+    // replay takes its place in the order).  One that a capture uses is kept until
+    // stt_destroy (`retired`), for the replays.
     struct Mirror {
         void *p = nullptr;
+        cudaEvent_t read = nullptr;
+        bool captured = false;
         size_t bytes = 0;
         int nx = 0, ny = 0, nz = 0;
         stt::FpTex tex;
     } mirror[2];
+    std::vector<Mirror> retired;
 };
 
 namespace stt {
@@ -78,9 +85,12 @@ stt_status apply_staged_bins(stt_ctx *ctx);
 const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol, cudaStream_t s);
 const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s);
 // The texture of the context's mirror for volumes of this storage, and the
-// mirror (allocated on first use; nullptr as above, or without memory).
+// mirror (allocated on first use; nullptr as above, or without memory), which `s`
+// may write from here on.  The caller ends its use with ctx_mirror_done once its
+// last reader is enqueued.
 const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, float **mirror);
 const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, unsigned short **mirror);
+void ctx_mirror_done(stt_ctx *ctx, size_t esize, cudaStream_t s);
 // How the correction projector runs on volumes of one storage: a tuned context's
 // choices; untuned, tld4 corners and no view staged where the textures bind
 // (FP_DEFAULT_TEX), else load variant 0 with the oblique views staged.

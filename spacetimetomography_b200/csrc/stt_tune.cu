@@ -150,11 +150,15 @@ template <typename T>
 const FpTex *mirror_tex(stt_ctx *ctx, cudaStream_t s, T **mirror) {
     const GeomDev &g = ctx->g;
     stt_ctx::Mirror &m = ctx->mirror[sizeof(T) == 2];
+    const bool cap = capturing(s);
     if (m.nx != g.nx || m.ny != g.ny || m.nz != g.nz) {
         const size_t pitch = fp_mirror_pitch((size_t)g.nx * g.ny), bytes = pitch * g.nz * sizeof(T);
         // (a base as aligned as cudaMalloc's: whether the mirror's own texture would bind)
-        if (capturing(s) || !fp_tex_fits(g, reinterpret_cast<const void *>((uintptr_t)4096), (int)sizeof(T), pitch))
-            return nullptr;
+        if (cap || !fp_tex_fits(g, reinterpret_cast<const void *>((uintptr_t)4096), (int)sizeof(T), pitch)) return nullptr;
+        if (m.captured) {
+            ctx->retired.push_back(m);
+            m = stt_ctx::Mirror{};
+        }
         // another size: launches enqueued earlier (on any stream) may still gather
         // from the old texture, so the device drains before it goes
         if (m.p && cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
@@ -175,6 +179,16 @@ const FpTex *mirror_tex(stt_ctx *ctx, cudaStream_t s, T **mirror) {
         make_fp_tex(g, static_cast<const T *>(m.p), m.tex, pitch);
     }
     if (!m.tex.ok) return nullptr;
+    if (!m.read && (cap || cudaEventCreateWithFlags(&m.read, cudaEventDisableTiming) != cudaSuccess)) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    // (an event never recorded waits for nothing)
+    if (cudaStreamWaitEvent(s, m.read, cap ? cudaEventWaitExternal : cudaEventWaitDefault) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    m.captured |= cap;
     *mirror = static_cast<T *>(m.p);
     return &m.tex;
 }
@@ -187,6 +201,13 @@ const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s)
 const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, float **mirror) { return mirror_tex(ctx, s, mirror); }
 
 const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, unsigned short **mirror) { return mirror_tex(ctx, s, mirror); }
+
+void ctx_mirror_done(stt_ctx *ctx, size_t esize, cudaStream_t s) {
+    const unsigned flag = capturing(s) ? cudaEventRecordExternal : cudaEventRecordDefault;
+    if (cudaEventRecordWithFlags(ctx->mirror[esize == 2].read, s, flag) == cudaSuccess) return;
+    cudaGetLastError();  // nothing to wait for: the device drains instead
+    if (cudaDeviceSynchronize() != cudaSuccess) cudaGetLastError();
+}
 
 FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds) {
     if (ctx->tuned) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), ctx->staged_bins != 0};
