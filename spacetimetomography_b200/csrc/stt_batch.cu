@@ -52,7 +52,8 @@ struct stt_batch {
 
 extern "C" stt_status stt_internal_set_error(stt_ctx *ctx, stt_status st, const char *msg);
 extern "C" stt_status stt_internal_solver_presweep(stt_solver *s, void *stream);
-extern "C" void stt_internal_solver_chains(stt_solver *s, int chains);
+extern "C" void stt_internal_solver_set_chains(stt_solver *s, int chains);
+extern "C" int stt_internal_solver_chains(const stt_solver *s);
 extern "C" int stt_internal_solver_jobs(const stt_solver *s, void *jobs);
 extern "C" void stt_internal_solver_end_iteration(stt_solver *s);
 
@@ -172,8 +173,8 @@ cudaError_t init_state(stt_batch::Inst &in) {
 }
 
 // (Re)creates the instance's one-frame solver with its context's current
-// launch choices.
-stt_status make_solver(stt_batch::Inst &in, bool persistent = false) {
+// launch choices, as one of the batch's instances that run side by side.
+stt_status make_solver(stt_batch *b, stt_batch::Inst &in) {
     if (in.solver) {
         stt_solver_destroy(in.solver);
         in.solver = nullptr;
@@ -195,7 +196,7 @@ stt_status make_solver(stt_batch::Inst &in, bool persistent = false) {
     cfg.seed = I.seed;
     cfg.autotune = I.autotune;
     cfg.storage = I.storage;
-    cfg.mode = persistent ? STT_SOLVE_PERSISTENT : STT_SOLVE_STREAMS;
+    cfg.mode = b->mode == STT_SOLVE_PERSISTENT ? STT_SOLVE_PERSISTENT : STT_SOLVE_STREAMS;
     stt_pd_state state{};  // (BF16 storage: the primal pointers address BF16 arrays)
     state.vol = reinterpret_cast<float *>(vol);
     state.xbar = reinterpret_cast<float *>(xbar);
@@ -205,7 +206,9 @@ stt_status make_solver(stt_batch::Inst &in, bool persistent = false) {
     state.ybc = ybc;
     state.flow = flow;
     state.proj = I.proj;
-    return stt_solver_create(I.ctx, &cfg, &state, &in.solver);
+    const stt_status st = stt_solver_create(I.ctx, &cfg, &state, &in.solver);
+    if (!st) stt_internal_solver_set_chains(in.solver, (int)b->inst.size());
+    return st;
 }
 
 void drop_graph(stt_batch *b) {
@@ -277,7 +280,7 @@ stt_status choose_staging(stt_batch *b) {
         st = stt_set_tuning(b->inst[i].ctx, &t);
     }
     for (size_t i = 0; i < n && !st; ++i)
-        if ((st = make_solver(b->inst[i]))) bfail(b, st, "instance " + std::to_string(i) + ": solver");
+        if ((st = make_solver(b, b->inst[i]))) bfail(b, st, "instance " + std::to_string(i) + ": solver");
     for (size_t i = 0; i < n && !st; ++i)
         if (init_state(b->inst[i]) != cudaSuccess) st = bfail(b, STT_ERR_CUDA, "state reset");
     if (!st) st = time_iteration(b, b->ms_gather);
@@ -288,7 +291,7 @@ stt_status choose_staging(stt_batch *b) {
         for (size_t i = 0; i < n && !st; ++i) st = stt_set_tuning(b->inst[i].ctx, &saved[i]);
     // fresh solvers (iteration counters at 0, no sticky ray lengths) and states
     for (size_t i = 0; i < n && !st; ++i)
-        if ((st = make_solver(b->inst[i]))) bfail(b, st, "instance " + std::to_string(i) + ": solver");
+        if ((st = make_solver(b, b->inst[i]))) bfail(b, st, "instance " + std::to_string(i) + ": solver");
     for (size_t i = 0; i < n && !st; ++i)
         if (init_state(b->inst[i]) != cudaSuccess) st = bfail(b, STT_ERR_CUDA, "state reset");
     return st;
@@ -341,9 +344,8 @@ stt_status stt_batch_create(const stt_instance *instances, int n, int mode, stt_
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&in.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&in.done, cudaEventDisableTiming);
         if (e != cudaSuccess) return bail(STT_ERR_CUDA, std::string("instance set-up: ") + cudaGetErrorString(e));
-        stt_status st = make_solver(in, persistent);
+        stt_status st = make_solver(b, in);
         if (st) return bail(st, "instance " + std::to_string(i) + ": " + stt_last_error(I.ctx));
-        stt_internal_solver_chains(in.solver, n);
     }
     if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess)
         return bail(STT_ERR_CUDA, "event create");
@@ -451,6 +453,11 @@ stt_status stt_batch_staging(const stt_batch *b, int *timed, int *all_gather, fl
     if (ms_split) *ms_split = b->ms_split;
     if (ms_gather) *ms_gather = b->ms_gather;
     return STT_OK;
+}
+
+// The chains that instance i's solver counts (tests).
+int stt_internal_batch_chains(const stt_batch *b, int i) {
+    return b && i >= 0 && i < (int)b->inst.size() ? stt_internal_solver_chains(b->inst[i].solver) : -1;
 }
 
 const char *stt_batch_last_error(const stt_batch *b) { return b ? b->err.c_str() : "null batch"; }

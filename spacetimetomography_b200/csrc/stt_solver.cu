@@ -869,7 +869,8 @@ stt_status stt_solver_destroy(stt_solver *s) {
 }
 
 // How many instances of a batch run beside this solver's frame (stt_batch.cu).
-void stt_internal_solver_chains(stt_solver *s, int chains) { s->chains = chains; }
+void stt_internal_solver_set_chains(stt_solver *s, int chains) { s->chains = chains; }
+int stt_internal_solver_chains(const stt_solver *s) { return s->chains; }
 
 // Hooks of the batch's persistent form (stt_batch.cu), for a solver created
 // with STT_SOLVE_PERSISTENT: one iteration's steps before the sweep, joined
