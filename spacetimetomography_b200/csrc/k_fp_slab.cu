@@ -376,10 +376,15 @@ const char *slab_variant_name(int v) {
     return v >= 0 && v < kSlabVariants ? names[v] : "?";
 }
 
+bool fp_slab_fits(const GeomDev &g, int esize, bool copy) {
+    return (long long)g.nx * g.ny * g.nz < (1LL << 31) &&  // 32-bit fallback offsets
+           (size_t)g.nx * esize % 16 == 0 && !(copy && (size_t)g.nz * esize % 16);
+}
+
 static bool make_maps(const GeomDev &g, const void *vol, const void *vol_t, size_t esize, FpSlabMaps &m,
                       int variant) {
     m = FpSlabMaps{};
-    if ((long long)g.nx * g.ny * g.nz >= (1LL << 31)) return false;  // 32-bit fallback offsets
+    if (!fp_slab_fits(g, (int)esize, vol_t != nullptr)) return false;
     if (variant < 0 || variant >= kSlabVariants) return false;
     cuuint32_t box[3];
     switch (variant & 3) {  // variants 4..7: the boxes of 0..3 with packed sample pairs

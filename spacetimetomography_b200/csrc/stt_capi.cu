@@ -391,7 +391,7 @@ static stt_status project_corr(stt_ctx *ctx, const T *vol, const FpSource<T> &sr
     if (stt::fp_needs_copy(c, v, (sizeof(T) == 2 ? v.staged16 : v.staged) != 0))
         if (stt_status st = make_copy(ctx, vol, s, &volt)) return st;
     stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
-    if (c.stage) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
+    if (c.stage[v.layout]) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
     STT_CUDA(ctx, stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, raylen, corr, s, &maps, ctx->status,
                                       c.variant, c.tex ? src.tex : nullptr),
              "k_fp_corr launch");

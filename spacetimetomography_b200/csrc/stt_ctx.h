@@ -97,12 +97,14 @@ void ctx_mirror_done(stt_ctx *ctx, size_t esize, cudaStream_t s);
 struct FpChoice {
     int variant;  // launch_fp_corr's fp_variant (FP32) or fp_variant16 (BF16)
     bool tex;     // its corners come from the volume's texture
-    bool stage;   // some view class goes to the slab-staged projector
+    // Some view class goes to the slab-staged projector, by ViewRec::layout (its boxes
+    // cover the volume for layout 0, and the z-fastest copy too for layout 1).
+    bool stage[2];
 };
 FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds);
 FpChoice fp_choice(const stt_ctx *ctx, const unsigned short *, bool tex_binds);
 // Whether a view gathers from the z-fastest copy under that choice.
 inline bool fp_needs_copy(const FpChoice &c, const ViewRec &v, bool staged) {
-    return v.layout == 1 && (!c.tex || (c.stage && staged));
+    return v.layout == 1 && (!c.tex || (c.stage[1] && staged));
 }
 }  // namespace stt

@@ -91,6 +91,9 @@ bool make_fp_slab_maps(const GeomDev &g, const float *vol, const float *vol_t, F
 // BF16 storage: the scalar boxes (variant & 3); x and z extents multiples of 8.
 bool make_fp_slab_maps(const GeomDev &g, const unsigned short *vol, const unsigned short *vol_t, FpSlabMaps &m,
                        int variant = 0);
+// Whether the maps' extents admit volumes of this size (esize bytes per voxel), and
+// with `copy` their z-fastest copies too.
+bool fp_slab_fits(const GeomDev &g, int esize, bool copy);
 // A 4D FP32 tensor map over nc planar volumes (x fastest, then y, z, plane)
 // with the given box (x, y, z, plane); false where TMA cannot address them
 // (nx not a multiple of 4, ptr not 16-byte aligned, box row not 16 bytes).

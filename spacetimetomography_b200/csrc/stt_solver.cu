@@ -623,7 +623,7 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
         s->fp = choice(binds);
     }
     // the z-fastest copies, where a view may gather from one
-    if (!per_view_kernels || !s->fp.tex || s->fp.stage) {
+    if (!per_view_kernels || !s->fp.tex || s->fp.stage[1]) {
         unsigned char *vt = nullptr;
         if ((e = alloc(s, vt, (size_t)F * s->n * (f32 ? 4 : 2), "transposed volumes"))) {
             stt_solver_destroy(s);
@@ -632,7 +632,7 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
         s->volt = vt;
     }
     // no views staged (one gather launch per view): no maps
-    if (per_view_kernels && s->fp.stage) {
+    if (per_view_kernels && s->fp.stage[1]) {
         s->fpmaps.resize(F);
         for (int f = 0; f < F; ++f) {  // where the maps do not apply, ok stays 0 and every view gathers
             if (f32)

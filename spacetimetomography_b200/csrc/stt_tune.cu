@@ -210,15 +210,17 @@ void ctx_mirror_done(stt_ctx *ctx, size_t esize, cudaStream_t s) {
 }
 
 FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds) {
-    if (ctx->tuned) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), ctx->staged_bins != 0};
-    if (tex_binds) return {FP_DEFAULT_TEX, true, false};
-    return {FP_DEFAULT_LOADS, false, ctx->staged_bins != 0};
+    const bool s0 = ctx->staged_bins != 0 && fp_slab_fits(ctx->g, 4, false), s1 = s0 && fp_slab_fits(ctx->g, 4, true);
+    if (ctx->tuned) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), {s0, s1}};
+    if (tex_binds) return {FP_DEFAULT_TEX, true, {false, false}};
+    return {FP_DEFAULT_LOADS, false, {s0, s1}};
 }
 
 FpChoice fp_choice(const stt_ctx *ctx, const unsigned short *, bool tex_binds) {
-    if (ctx->tuned) return {ctx->tuning.fp16, tex_binds && ctx->tuning.fp16 == 1, ctx->staged_bins16 != 0};
-    if (tex_binds) return {1, true, false};
-    return {0, false, ctx->staged_bins16 != 0};
+    const bool s0 = ctx->staged_bins16 != 0 && fp_slab_fits(ctx->g, 2, false), s1 = s0 && fp_slab_fits(ctx->g, 2, true);
+    if (ctx->tuned) return {ctx->tuning.fp16, tex_binds && ctx->tuning.fp16 == 1, {s0, s1}};
+    if (tex_binds) return {1, true, {false, false}};
+    return {0, false, {s0, s1}};
 }
 
 }  // namespace stt
@@ -440,15 +442,11 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
             gather_all += (double)count[b] * tg[t.fp_variant][b];
         }
         if (split >= gather_all) t.staged_bins = 0;
-    } else {
-        t.staged_bins = 0x1E0u;  // irrelevant: without slab maps every view gathers
-    }
+    }  // else none is staged: without slab maps every view gathers
     // BF16 storage: per class the gather kernel's two forms (loads, and tld4
     // gathers of 16-bit textures where they bind) and the slab kernel's BF16
     // box (the box just chosen); a BF16 volume's gathers move half the bytes,
     // so the faster projector can differ from the FP32 choice
-    t.staged_bins_bf16 = 0x1E0u;  // irrelevant where the BF16 maps do not apply
-    t.fp_variant_bf16 = 0;
     {
         if ((e = cudaMalloc(&sc.vol16, n * sizeof(unsigned short))) ||
             (e = cudaMalloc(&sc.volt16, n * sizeof(unsigned short))) ||
@@ -508,7 +506,6 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
             if (tot < best16) best16 = tot, t.fp_variant_bf16 = fv;
         }
         if (maps16) {
-            t.staged_bins_bf16 = 0;
             double split = 0.0, gather_all = 0.0;
             for (int b = 0; b < 9; ++b) {
                 if (rep[b] < 0) {
