@@ -143,12 +143,14 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g);
  * synchronises `stream` and rewrites the context's view table, so call it
  * (and stt_set_tuning) while no launch of this context is in flight; launches
  * enqueued after it use the choice (a context that is not tuned gathers every
- * view with tld4 where the volume binds, else uses load variant 0 and stages the
- * classes from 25 degrees on), and a solver uses the choice current when
+ * view with tld4 where the volume binds, else with load variant 5, BF16 with form
+ * 0, and stages the classes from 25 degrees on), and a solver uses the choice current when
  * it is created (stt_solve_cfg.autotune runs the tuner then).  out (may be
  * NULL) receives the choice and the timings (microseconds per launch, 0 where
- * a variant was not timed).  stt_get_tuning reads the current choice;
- * stt_set_tuning sets one (a variant out of range is STT_ERR_INVALID). */
+ * a variant was not timed).  stt_get_tuning reads the current choice, of an
+ * untuned context what it runs (tld4 and no class staged where volumes of this size
+ * bind); stt_set_tuning sets one (a variant out of range is STT_ERR_INVALID).
+ * Setting what was read changes nothing, also where an array does not bind. */
 typedef struct stt_tuning {
     int fp_variant, slab_variant, bp_variant;
     unsigned staged_bins;

@@ -532,6 +532,11 @@ bool fp_tex_fits(const GeomDev &g, const void *vol, int esize, size_t pitch) {
     return small_volume(g) && tex_limits(l) && slices_fit(l, vol, slice, g.nz, (pitch ? (long long)pitch : slice) * esize);
 }
 
+bool fp_tex_admits(const GeomDev &g, int esize) {
+    const void *aligned = reinterpret_cast<const void *>((uintptr_t)4096);  // (as cudaMalloc's)
+    return fp_tex_fits(g, aligned, esize) || fp_tex_fits(g, aligned, esize, fp_mirror_pitch((size_t)g.nx * g.ny));
+}
+
 void destroy_fp_tex(FpTex &t) {
     if (t.x) cudaDestroyTextureObject((cudaTextureObject_t)t.x);
     t = FpTex{};

@@ -258,6 +258,7 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g) {
     ctx->geom.angles_rad = nullptr;
     ctx->tuning = stt::Tuning{};
     ctx->staged_bins = ctx->staged_bins16 = 0x1E0u;
+    ctx->fp_default = ctx->fp16_default = true;
     ctx->tuned = false;
     ctx->report = stt_tuning{};
     if (g->n_views > 0) {
@@ -290,6 +291,8 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g) {
     ctx->sp[1] = g->sy;
     ctx->sp[2] = g->sz;
     ctx->tuning.ray = stt::default_ray_variant(d);  // (depends on the volume size just set)
+    ctx->tex_admits = stt::fp_tex_admits(d, sizeof(float));
+    ctx->tex_admits16 = stt::fp_tex_admits(d, sizeof(unsigned short));
     ctx->has_geom = true;
     return STT_OK;
 }

@@ -41,6 +41,12 @@ struct stt_ctx {
     stt::Tuning tuning{};
     unsigned staged_bins = 0x1E0u;
     unsigned staged_bins16 = 0x1E0u;  // the same for a BF16-stored volume (ViewRec::staged16)
+    // The projector's default choices: texture gathers of every view where a
+    // volume of this size can bind (itself or through a mirror), and loads with the
+    // oblique views staged where the one at hand does not.  Also what
+    // stt_set_tuning keeps when it is given the pair that default_fp reports.
+    bool fp_default = true, fp16_default = true;
+    bool tex_admits = false, tex_admits16 = false;
     bool tuned = false;
     stt_tuning report{};
     // Texture objects of the tld4 gather forms for the arrays the entry points
@@ -91,9 +97,18 @@ const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s)
 const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, float **mirror);
 const FpTex *ctx_mirror_tex(stt_ctx *ctx, cudaStream_t s, unsigned short **mirror);
 void ctx_mirror_done(stt_ctx *ctx, size_t esize, cudaStream_t s);
-// How the correction projector runs on volumes of one storage: a tuned context's
-// choices; untuned, tld4 corners and no view staged where the textures bind
-// (FP_DEFAULT_TEX), else load variant 0 with the oblique views staged.
+// The default pair of gather variant and staged classes, as it is reported.
+struct FpDefault {
+    int variant;
+    unsigned staged_bins;
+};
+inline FpDefault default_fp(const stt_ctx *c) {
+    return c->tex_admits ? FpDefault{FP_DEFAULT_TEX, 0u} : FpDefault{FP_DEFAULT_LOADS, 0x1E0u};
+}
+inline FpDefault default_fp16(const stt_ctx *c) { return c->tex_admits16 ? FpDefault{1, 0u} : FpDefault{0, 0x1E0u}; }
+// How the correction projector runs on volumes of one storage: the choices set; by
+// default tld4 corners and no view staged where the textures bind (FP_DEFAULT_TEX),
+// else loads (FP_DEFAULT_LOADS; BF16 form 0) with the oblique views staged.
 struct FpChoice {
     int variant;  // launch_fp_corr's fp_variant (FP32) or fp_variant16 (BF16)
     bool tex;     // its corners come from the volume's texture

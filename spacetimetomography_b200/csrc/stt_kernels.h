@@ -141,6 +141,8 @@ cudaError_t launch_mirror(const GeomDev &g, const unsigned short *vol, unsigned 
 // Whether make_fp_tex admits `vol` (esize bytes per voxel) on this device
 // (checks the limits only; creates nothing).
 bool fp_tex_fits(const GeomDev &g, const void *vol, int esize, size_t pitch = 0);
+// Whether one of this size can bind: at an aligned base, or its mirror.
+bool fp_tex_admits(const GeomDev &g, int esize);
 void destroy_fp_tex(FpTex &t);
 // Projections of at most this many rays in one launch share each ray between
 // the 4 warps of a block when their corners come from a texture (k_fp_split.cu).

@@ -211,14 +211,14 @@ void ctx_mirror_done(stt_ctx *ctx, size_t esize, cudaStream_t s) {
 
 FpChoice fp_choice(const stt_ctx *ctx, const float *, bool tex_binds) {
     const bool s0 = ctx->staged_bins != 0 && fp_slab_fits(ctx->g, 4, false), s1 = s0 && fp_slab_fits(ctx->g, 4, true);
-    if (ctx->tuned) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), {s0, s1}};
+    if (!ctx->fp_default) return {ctx->tuning.fp, tex_binds && is_tex_fp_variant(ctx->tuning.fp), {s0, s1}};
     if (tex_binds) return {FP_DEFAULT_TEX, true, {false, false}};
     return {FP_DEFAULT_LOADS, false, {s0, s1}};
 }
 
 FpChoice fp_choice(const stt_ctx *ctx, const unsigned short *, bool tex_binds) {
     const bool s0 = ctx->staged_bins16 != 0 && fp_slab_fits(ctx->g, 2, false), s1 = s0 && fp_slab_fits(ctx->g, 2, true);
-    if (ctx->tuned) return {ctx->tuning.fp16, tex_binds && ctx->tuning.fp16 == 1, {s0, s1}};
+    if (!ctx->fp16_default) return {ctx->tuning.fp16, tex_binds && ctx->tuning.fp16 == 1, {s0, s1}};
     if (tex_binds) return {1, true, {false, false}};
     return {0, false, {s0, s1}};
 }
@@ -240,13 +240,14 @@ stt_status stt_get_tuning(const stt_ctx *ctx, stt_tuning *out) {
     if (!ctx || !out) return STT_ERR_INVALID;
     if (!ctx->has_geom) return STT_ERR_STATE;
     *out = ctx->report;
-    out->fp_variant = ctx->tuning.fp;
+    const stt::FpDefault d = stt::default_fp(ctx), d16 = stt::default_fp16(ctx);
+    out->fp_variant = ctx->fp_default ? d.variant : ctx->tuning.fp;
     out->slab_variant = ctx->tuning.slab;
     out->bp_variant = ctx->tuning.bp;
     out->ray_variant = ctx->tuning.ray;
-    out->fp_variant_bf16 = ctx->tuning.fp16;
-    out->staged_bins = ctx->staged_bins;
-    out->staged_bins_bf16 = ctx->staged_bins16;
+    out->fp_variant_bf16 = ctx->fp16_default ? d16.variant : ctx->tuning.fp16;
+    out->staged_bins = ctx->fp_default ? d.staged_bins : ctx->staged_bins;
+    out->staged_bins_bf16 = ctx->fp16_default ? d16.staged_bins : ctx->staged_bins16;
     out->tuned = ctx->tuned ? 1 : 0;
     return STT_OK;
 }
@@ -271,11 +272,17 @@ stt_status stt_set_tuning(stt_ctx *ctx, const stt_tuning *t) {
     ctx->tuning.bp = t->bp_variant;
     ctx->tuning.ray = t->ray_variant;
     ctx->tuning.fp16 = t->fp_variant_bf16;
-    ctx->staged_bins = t->staged_bins;
-    ctx->staged_bins16 = t->staged_bins_bf16;
-    ctx->tuned = true;
+    // the default pairs keep their other half, the loads with staged views
+    const stt::FpDefault d = stt::default_fp(ctx), d16 = stt::default_fp16(ctx);
+    ctx->fp_default = t->fp_variant == d.variant && t->staged_bins == d.staged_bins;
+    ctx->fp16_default = t->fp_variant_bf16 == d16.variant && t->staged_bins_bf16 == d16.staged_bins;
+    ctx->staged_bins = ctx->fp_default ? 0x1E0u : t->staged_bins;
+    ctx->staged_bins16 = ctx->fp16_default ? 0x1E0u : t->staged_bins_bf16;
+    // what stt_get_tuning read from an untuned context leaves it untuned
+    ctx->tuned = t->tuned || !ctx->fp_default || !ctx->fp16_default || t->slab_variant != 0 || t->bp_variant != 0 ||
+                 t->ray_variant != stt::default_ray_variant(ctx->g);
     ctx->report = *t;
-    ctx->report.tuned = 1;
+    ctx->report.tuned = ctx->tuned;
     return stt::apply_staged_bins(ctx);
 }
 
@@ -300,7 +307,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
         auto it = g_cache.find(key);
         if (it != g_cache.end()) {
             stt_tuning t = it->second;
-            t.from_cache = 1;
+            t.from_cache = t.tuned = 1;
             stt_status st = stt_set_tuning(ctx, &t);
             if (st) return st;
             if (out) *out = ctx->report;
@@ -572,6 +579,7 @@ stt_status stt_autotune(stt_ctx *ctx, stt_tuning *out, void *stream) {
         }
     }
     if ((e = cudaStreamSynchronize(s))) return fail(e, "synchronize");
+    t.tuned = 1;
     stt_status st = stt_set_tuning(ctx, &t);
     if (st) return st;
     {
