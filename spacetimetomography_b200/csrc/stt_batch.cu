@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "stt.h"
+#include "stt_ctx.h"
 #include "stt_internal.cuh"
 #include "stt_kernels.h"
 
@@ -254,47 +255,69 @@ stt_status time_iteration(stt_batch *b, float &ms) {
     return st;
 }
 
-// Which views the slab-staged projector takes is tuned per instance on an
-// otherwise idle GPU.  In a batch, the instances' views run side by side, and
-// there every view gathering (one launch per view, no 37 KB of shared memory
-// per block) can be faster: measured on the 64 uneven instances of the batch
-// workload, 409 against 466 ms per iteration (BF16 storage 400 against 444).
-// So a batch whose instances ask for tuning times one batched iteration both
-// ways and keeps the faster; the states are re-initialised and the solvers
-// re-created afterwards, so the solve starts as if untimed.
-stt_status choose_staging(stt_batch *b) {
-    const size_t n = b->inst.size();
-    std::vector<stt_tuning> saved(n);
-    bool any = false;
-    for (size_t i = 0; i < n; ++i) {
-        stt_status st = stt_get_tuning(b->inst[i].ctx, &saved[i]);
-        if (st) return bfail(b, st, "instance " + std::to_string(i) + ": stt_get_tuning");
-        any |= (b->inst[i].cfg.storage == STT_DTYPE_BF16 ? saved[i].staged_bins_bf16 : saved[i].staged_bins) != 0;
-    }
-    if (!any) return STT_OK;  // every view gathers already
-    stt_status st = time_iteration(b, b->ms_split);
-    for (size_t i = 0; i < n && !st; ++i) {  // the mask of the instance's own storage
-        stt_tuning t = saved[i];
-        if (b->inst[i].cfg.storage == STT_DTYPE_BF16) t.staged_bins_bf16 = 0;
-        else t.staged_bins = 0;
-        st = stt_set_tuning(b->inst[i].ctx, &t);
-    }
-    for (size_t i = 0; i < n && !st; ++i)
+// The launch choices of every instance, and the solvers and states made anew with
+// them, as if nothing had run.
+stt_status apply_choices(stt_batch *b, const std::vector<stt_tuning> &set) {
+    stt_status st = STT_OK;
+    for (size_t i = 0; i < set.size() && !st; ++i)
+        if ((st = stt_set_tuning(b->inst[i].ctx, &set[i]))) bfail(b, st, "instance " + std::to_string(i) + ": stt_set_tuning");
+    for (size_t i = 0; i < set.size() && !st; ++i)
         if ((st = make_solver(b, b->inst[i]))) bfail(b, st, "instance " + std::to_string(i) + ": solver");
-    for (size_t i = 0; i < n && !st; ++i)
-        if (init_state(b->inst[i]) != cudaSuccess) st = bfail(b, STT_ERR_CUDA, "state reset");
-    if (!st) st = time_iteration(b, b->ms_gather);
-    if (st) return st;
-    b->staging_timed = 1;
-    b->all_gather = b->ms_gather < b->ms_split;
-    if (!b->all_gather)
-        for (size_t i = 0; i < n && !st; ++i) st = stt_set_tuning(b->inst[i].ctx, &saved[i]);
-    // fresh solvers (iteration counters at 0, no sticky ray lengths) and states
-    for (size_t i = 0; i < n && !st; ++i)
-        if ((st = make_solver(b, b->inst[i]))) bfail(b, st, "instance " + std::to_string(i) + ": solver");
-    for (size_t i = 0; i < n && !st; ++i)
+    for (size_t i = 0; i < set.size() && !st; ++i)
         if (init_state(b->inst[i]) != cudaSuccess) st = bfail(b, STT_ERR_CUDA, "state reset");
     return st;
+}
+
+// The choices are tuned per instance on an otherwise idle GPU.  In a batch the
+// instances' views run side by side, and there others can be faster: every view
+// gathering (one launch per view, no 37 KB of shared memory per block), or the
+// untuned choices as a whole.  So a batch whose instances ask for tuning times one
+// batched iteration of each set and keeps the fastest; the solve then starts as if
+// untimed.  64 uneven instances, ms per iteration: tuned 273.7, untuned 261.5.
+stt_status choose_tuning(stt_batch *b) {
+    const size_t n = b->inst.size();
+    std::vector<stt_tuning> best(n);
+    bool any = false;
+    for (size_t i = 0; i < n; ++i) {
+        stt_status st = stt_get_tuning(b->inst[i].ctx, &best[i]);
+        if (st) return bfail(b, st, "instance " + std::to_string(i) + ": stt_get_tuning");
+        any |= (b->inst[i].cfg.storage == STT_DTYPE_BF16 ? best[i].staged_bins_bf16 : best[i].staged_bins) != 0;
+    }
+    std::vector<stt_tuning> untuned = best, gather = best;
+    bool differs = false;
+    for (size_t i = 0; i < n; ++i) {
+        const stt_ctx *c = b->inst[i].ctx;
+        if (b->inst[i].cfg.storage == STT_DTYPE_BF16) gather[i].staged_bins_bf16 = 0;  // the mask of its own storage
+        else gather[i].staged_bins = 0;
+        if (!b->inst[i].cfg.autotune) continue;
+        stt_tuning &t = untuned[i];
+        const stt::FpDefault d = stt::default_fp(c), d16 = stt::default_fp16(c);
+        t.fp_variant = d.variant, t.staged_bins = d.staged_bins;
+        t.fp_variant_bf16 = d16.variant, t.staged_bins_bf16 = d16.staged_bins;
+        t.slab_variant = t.bp_variant = 0;
+        t.ray_variant = stt::default_ray_variant(c->g);
+        const stt_tuning &q = best[i];
+        differs |= t.fp_variant != q.fp_variant || t.staged_bins != q.staged_bins || t.bp_variant != q.bp_variant ||
+                   t.fp_variant_bf16 != q.fp_variant_bf16 || t.staged_bins_bf16 != q.staged_bins_bf16 ||
+                   t.ray_variant != q.ray_variant;
+    }
+    if (!any && !differs) return STT_OK;
+    float ms = 0.0f;
+    stt_status st = time_iteration(b, ms);
+    const std::vector<stt_tuning> *keep = &best;
+    if (!st && any) {
+        b->ms_split = ms;
+        if (!(st = apply_choices(b, gather))) st = time_iteration(b, b->ms_gather);
+        b->staging_timed = 1;
+        b->all_gather = b->ms_gather < b->ms_split;
+        if (b->all_gather) keep = &gather, ms = b->ms_gather;
+    }
+    if (!st && differs) {
+        float t = 0.0f;
+        if (!(st = apply_choices(b, untuned))) st = time_iteration(b, t);
+        if (t < ms) keep = &untuned;
+    }
+    return st ? st : apply_choices(b, *keep);
 }
 
 }  // namespace
@@ -352,8 +375,8 @@ stt_status stt_batch_create(const stt_instance *instances, int n, int mode, stt_
     bool tune = false;
     for (int i = 0; i < n; ++i) tune |= instances[i].autotune != 0;
     if (tune && !persistent) {  // (the persistent sweep has one projector: nothing to choose)
-        const stt_status st = choose_staging(b);
-        if (st) return bail(st, "batch staging choice: " + b->err);
+        const stt_status st = choose_tuning(b);
+        if (st) return bail(st, "batch tuning: " + b->err);
     }
     if (persistent) {
         const stt_status st = build_sweep(b);
