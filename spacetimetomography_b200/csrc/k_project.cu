@@ -362,6 +362,35 @@ int grid_stride_blocks(long long n, int threads) {
     return (int)(b < cap ? (b < 1 ? 1 : b) : cap);
 }
 
+FpFrom fp_from(long long voxels, float row_pitch, int esize, bool own, const FpCall &c) {
+    int all = 0, in[2][10] = {};  // in[l][k]: layout l, in the first k classes
+    for (int l = 0; l < 2; ++l)
+        for (int b = 0; b < 9; ++b) in[l][b + 1] = in[l][b] + c.views[l][b], all += c.views[l][b];
+    // a call along an axis: every view within 25 degrees of it, three in four in the first `classes`
+    const auto close = [&](int l, int classes) { return in[l][5] == all && 4 * in[l][classes] >= 3 * all; };
+    const bool few = c.rays <= FP_SPLIT_RAYS;  // the split form, if from a texture
+    // (the copy's launch alone)
+    const bool tiny = !own && voxels < (1LL << 19) && c.rays >= 20000 && c.rays < 100000 && close(0, 2);
+    if (esize == 2) {
+        const bool slow_copy = voxels > (1LL << 24) && close(0, 4) && c.rays * 150 < voxels && !few;
+        const bool coarse = close(0, 2) && row_pitch > 2.0f && c.rays >= 80000 && c.rays < 200000;
+        return !own && (slow_copy || coarse || tiny) ? FpFrom::OwnTexture : FpFrom::Texture;
+    }
+    const bool past_l2 = voxels * 4 > 96000000;
+    // (loads of odd rows do better off the axis than those of rows a power of two apart)
+    const int fine = voxels < (1LL << 19) ? 5 : 4;
+    const int classes = own ? (voxels < (1LL << 22) ? 2 : 3) : (row_pitch < 0.9f || row_pitch > 2.5f ? fine : 3);
+    const bool many = c.rays >= 80000 && (!own || (voxels >= (1LL << 17) && (all >= 6 || c.rays >= 500000)));
+    if (many && close(0, classes) && (!past_l2 || row_pitch > 2.5f)) return FpFrom::Loads;
+    if (past_l2) return close(0, 1) && row_pitch > 3.5f ? FpFrom::OwnTexture : FpFrom::Texture;
+    // (along x loads make the z-fastest copy)
+    if (voxels >= (1LL << 18) && c.rays >= 700000 && c.rays * 10 >= voxels && close(1, 3)) return FpFrom::Loads;
+    if (own) return FpFrom::Texture;
+    if (close(0, 3)) return few && voxels <= (1LL << 23) && !tiny ? FpFrom::Texture : FpFrom::OwnTexture;
+    const bool slow_copy = voxels > (1LL << 23) && c.rays * 20 < voxels && !few;
+    return slow_copy && close(0, row_pitch < 2.0f ? 5 : 4) ? FpFrom::OwnTexture : FpFrom::Texture;
+}
+
 namespace {
 template <typename T>
 cudaError_t fp_any(const GeomDev &g, const ViewRec *views, const T *vol, const T *vol_t, int view0, int nviews,

@@ -353,21 +353,33 @@ struct FpSource {
     }
 };
 
+// The call's views for fp_from, added one by one.
+static void add_view(const stt_ctx *ctx, int view, stt::FpCall &c) {
+    ++c.views[ctx->views_h[view].layout][stt::off_axis_bin(ctx->off_axis_deg[view])];
+    c.rays += (long long)ctx->g.W * ctx->g.H;
+}
+
 template <typename T>
-static stt_status fp_source(stt_ctx *ctx, const T *vol, cudaStream_t s, FpSource<T> &src) {
-    if ((src.tex = stt::ctx_fp_tex(ctx, vol, s))) return STT_OK;
-    if (!(src.tex = stt::ctx_mirror_tex(ctx, s, &src.mirror))) return STT_OK;
+static stt::FpFrom from_of(const stt_ctx *ctx, const T *vol, const stt::FpCall &c) {
+    return stt::fp_from(nvox(ctx), ctx->g.row_pitch, (int)sizeof(T), stt::fp_tex_fits(ctx->g, vol, (int)sizeof(T)), c);
+}
+
+template <typename T>
+static stt_status fp_source(stt_ctx *ctx, const T *vol, stt::FpFrom from, cudaStream_t s, FpSource<T> &src) {
+    if (from == stt::FpFrom::Loads || (src.tex = stt::ctx_fp_tex(ctx, vol, s))) return STT_OK;
+    if (from == stt::FpFrom::OwnTexture || !(src.tex = stt::ctx_mirror_tex(ctx, s, &src.mirror))) return STT_OK;
     STT_CUDA(ctx, stt::launch_mirror(ctx->g, vol, src.mirror, s), "k_mirror launch");
     return STT_OK;
 }
 
-// Projections of [view0, view0 + nviews): corners from a texture where one
-// binds (no z-fastest copy), else by loads.
+// Projections of [view0, view0 + nviews), their corners fetched as fp_from says.
 template <typename T>
 static stt_status project(stt_ctx *ctx, const T *vol, float *proj, float *raylen, float *weight, int view0, int nviews,
                           cudaStream_t s) {
     FpSource<T> src(ctx, s);
-    stt_status st = fp_source(ctx, vol, s, src);
+    stt::FpCall call;
+    for (int v = view0; v < view0 + nviews; ++v) add_view(ctx, v, call);
+    stt_status st = fp_source(ctx, vol, from_of(ctx, vol, call), s, src);
     if (st) return st;
     const T *volt = nullptr;
     if (!src.tex && (st = transposed_if_needed(ctx, vol, view0, nviews, s, &volt))) return st;
@@ -376,11 +388,13 @@ static stt_status project(stt_ctx *ctx, const T *vol, float *proj, float *raylen
     return STT_OK;
 }
 
-// What project_corr fetches from: a texture only if the context's choice of
-// form is one.
+// What project_corr fetches from: a texture only if the context's choice of form is
+// one; by default of a mirror only where `pays` says so.
 template <typename T>
-static stt_status corr_source(stt_ctx *ctx, const T *vol, cudaStream_t s, FpSource<T> &src) {
-    return stt::fp_choice(ctx, vol, true).tex ? fp_source(ctx, vol, s, src) : STT_OK;
+static stt_status corr_source(stt_ctx *ctx, const T *vol, bool pays, cudaStream_t s, FpSource<T> &src) {
+    if (!stt::fp_choice(ctx, vol, true).tex) return STT_OK;
+    const bool chosen = !(sizeof(T) == 2 ? ctx->fp16_default : ctx->fp_default);
+    return fp_source(ctx, vol, pays || chosen ? stt::FpFrom::Texture : stt::FpFrom::OwnTexture, s, src);
 }
 
 // The fused forward projection and correction of one view: the gather form of
@@ -390,11 +404,12 @@ static stt_status project_corr(stt_ctx *ctx, const T *vol, const FpSource<T> &sr
                                const T *stack, float *raylen, float *corr, cudaStream_t s) {
     const stt::FpChoice c = stt::fp_choice(ctx, vol, src.tex != nullptr);
     const stt::ViewRec &v = ctx->views_h[sel.view];
+    const bool staged = (sizeof(T) == 2 ? v.staged16 : v.staged) != 0;
     const T *volt = nullptr;
-    if (stt::fp_needs_copy(c, v, (sizeof(T) == 2 ? v.staged16 : v.staged) != 0))
+    if (stt::fp_needs_copy(c, v, staged))
         if (stt_status st = make_copy(ctx, vol, s, &volt)) return st;
-    stt::FpSlabMaps maps{};  // ok = 0: every view gathers, one launch
-    if (c.stage[v.layout]) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
+    stt::FpSlabMaps maps{};  // ok = 0: the view gathers, one launch
+    if (c.stage[v.layout] && staged) stt::make_fp_slab_maps(ctx->g, vol, volt, maps, ctx->tuning.slab);
     STT_CUDA(ctx, stt::launch_fp_corr(ctx->g, ctx->views_d, vol, volt, sel, stack, raylen, corr, s, &maps, ctx->status,
                                       c.variant, c.tex ? src.tex : nullptr),
              "k_fp_corr launch");
@@ -431,7 +446,10 @@ stt_status stt_fp_correction(stt_ctx *ctx, const float *vol, const float *b, flo
     if ((st = check_views(ctx, view, 1))) return st;
     if ((st = set_device(ctx))) return st;
     FpSource<float> src(ctx, S(stream));
-    if ((st = corr_source(ctx, vol, S(stream), src))) return st;
+    stt::FpCall call;
+    add_view(ctx, view, call);
+    const bool pays = from_of(ctx, vol, call) == stt::FpFrom::Texture;
+    if ((st = corr_source(ctx, vol, pays, S(stream), src))) return st;
     return project_corr(ctx, vol, src, stt::ViewSel{view, nullptr, 0, view}, b, raylen_state, corr, S(stream));
 }
 
@@ -621,8 +639,23 @@ static stt_status sart_sweep_t(stt_ctx *ctx, T *vol, const T *proj_stack, const 
     const size_t npix = (size_t)ctx->g.W * ctx->g.H;
     if ((st = ensure(ctx, ctx->corr, ctx->corr_n, npix, "correction image"))) return st;
     if (bp_mode == 1 && (st = ensure_acc(ctx, s))) return st;
+    // A voxel-based sweep copies the volume once for all its views: that pays but for a
+    // single one along z of an FP32 volume (255^3 512^2 224 us against 190 by loads, 301^3
+    // 256^2 204 against 176; 203^3 256^2 80 against 89).  A ray-based one copies it for
+    // every view.
+    bool pays = true;
+    if (nperm > 0 && bp_mode == 1) {
+        stt::FpCall call;
+        for (int i = 0; i < nperm; ++i) add_view(ctx, view_offset + perm[i], call);
+        call.rays = (long long)npix;
+        pays = from_of(ctx, static_cast<const T *>(vol), call) == stt::FpFrom::Texture;
+    } else if (nperm == 1) {
+        const int v = view_offset + perm[0];
+        pays = sizeof(T) == 2 || ctx->views_h[v].layout == 1 || ctx->off_axis_deg[v] >= 25.0f ||
+               (long long)npix <= stt::FP_SPLIT_RAYS || nvox(ctx) <= (1LL << 23);
+    }
     FpSource<T> src(ctx, s);
-    if (nperm > 0 && (st = corr_source(ctx, static_cast<const T *>(vol), s, src))) return st;
+    if (nperm > 0 && (st = corr_source(ctx, static_cast<const T *>(vol), pays, s, src))) return st;
     for (int i = 0; i < nperm; ++i) {
         const stt::ViewSel sel{view_offset + perm[i], nullptr, 0, view_offset};
         // ray-based mode: TypicalRayProducer::Initial zeroes the ray lengths
@@ -844,6 +877,15 @@ stt_status stt_warp_vjp(const int *dim, const float *vel, const float *src, int 
     STT_CUDA(nullptr, stt::launch_warp_vjp(dim, vel, src, nc, dt, out_bar, src_bar, vel_bar, S(stream)),
              "k_warp_vjp launch");
     return STT_OK;
+}
+
+// The rule of fp_from as numbers (tests): views[l*9 + b]; 0 loads, 1 the volume's own
+// texture, 2 any texture.
+int stt_internal_fp_from(long long voxels, float row_pitch, int esize, int own, const int *views, long long rays) {
+    stt::FpCall c;
+    for (int k = 0; k < 18; ++k) c.views[k / 9][k % 9] = views[k];
+    c.rays = rays;
+    return (int)stt::fp_from(voxels, row_pitch, esize, own != 0, c);
 }
 
 }  // extern "C"

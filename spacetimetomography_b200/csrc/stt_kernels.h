@@ -157,6 +157,27 @@ inline long long fp_split_rays(int chains) {
     const long long share = FP_SPLIT_SHARED_RAYS / (chains > 1 ? chains : 1);
     return share < FP_SPLIT_RAYS ? share : FP_SPLIT_RAYS;
 }
+// Where a call's projections fetch their corners: by loads; from the volume's own
+// texture or, where none binds, by loads; or from a texture, of a mirror if need be.
+// views[l][b]: the call's views of ViewRec::layout l in off-axis class b (5 degrees
+// each); rays: of all of them; own: the volume's own texture binds.
+//
+// Textures are the faster by far for oblique views (the loads' lanes fall on more
+// lines) and for few rays (the split form), and BF16 ones almost always.  But a copy
+// of the volume costs some 0.45 us a megabyte, and along an axis loads are as fast or
+// faster where FP32 volumes stay in the L2.  Loads / own texture, us, at 0 degrees,
+// views x detector: 128^3 8 x 128^2 40 / 47, 24 x 64^2 37 / 48, 192^3 8 x 512^2
+// 520 / 623, 256^3 8 x 512^2 730 / 852, 24 x 64^2 75 / 117 (at 20 degrees 113 / 117, at
+// 45 218 / 120); but 256^3 1 x 256^2 56 / 40, 320^3 8 x 512^2 1211 / 1090.  Loads /
+// mirror, one view: 255^3 512^2 at 0 degrees 106 / 144, at 20 125 / 147, at 30 163 /
+// 147, 128^2 48 / 50; 187^3 128^2 37 / 27, 256^2 37 / 41; 301^3 256^2 112 / 98; a BF16
+// 301^3 256^2 60 / 74, 128^2 64 / 53.
+enum class FpFrom { Loads, OwnTexture, Texture };
+struct FpCall {
+    int views[2][9] = {};
+    long long rays = 0;
+};
+FpFrom fp_from(long long voxels, float row_pitch, int esize, bool own, const FpCall &c);
 cudaError_t launch_fp_split(const GeomDev &g, const ViewRec *views, int view0, int nviews, float *proj, float *raylen,
                             float *weight, cudaStream_t s, const FpTex &tex);
 cudaError_t launch_fp_corr_split(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *b_stack,
