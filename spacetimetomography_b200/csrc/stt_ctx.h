@@ -50,15 +50,16 @@ struct stt_ctx {
     bool tuned = false;
     stt_tuning report{};
     // Texture objects of the tld4 gather forms for the arrays the entry points
-    // were given, keyed by the array and the dimensions (at most kFpTexCache;
-    // past that the load-based forms run).  Kept until stt_destroy, so a stream
-    // capture of an entry point that bound one stays valid.
+    // were given, keyed by the array and the dimensions: at most kFpTexCache, past
+    // which the older half goes (cached_tex), but those that a stream capture bound,
+    // which stay valid until stt_destroy.
     struct FpTexEntry {
         const void *vol;
         int nx, ny, nz, esize;
         stt::FpTex tex;
+        bool captured;
     };
-    static constexpr int kFpTexCache = 32;
+    static constexpr int kFpTexCache = 256;
     std::vector<FpTexEntry> fp_tex;
     // The mirror of a volume no texture binds (launch_mirror), by storage:
     // [0] FP32, [1] BF16.  Written anew by every call that projects from it, on
@@ -86,8 +87,9 @@ inline int off_axis_bin(float deg) {
 // Applies ctx->staged_bins and staged_bins16 to every view (host and device tables).
 stt_status apply_staged_bins(stt_ctx *ctx);
 // The texture of `vol` (created on first use, cached in the context), whatever
-// the tuned variant; nullptr where it does not bind, the cache is full, or it
-// would have to be created while `s` is being captured.
+// the tuned variant; nullptr where it does not bind, it would have to be created
+// while `s` is being captured, or captures hold the whole cache.  Valid until the
+// next call.
 const FpTex *ctx_fp_tex(stt_ctx *ctx, const float *vol, cudaStream_t s);
 const FpTex *ctx_fp_tex(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s);
 // The texture of the context's mirror for volumes of this storage, and the

@@ -136,14 +136,33 @@ const FpTex *cached_tex(stt_ctx *ctx, const T *vol, cudaStream_t s) {
     const GeomDev &g = ctx->g;
     const int es = (int)sizeof(T);
     if (!fp_tex_fits(g, vol, es)) return nullptr;
-    for (const auto &e : ctx->fp_tex)
-        if (e.vol == vol && e.nx == g.nx && e.ny == g.ny && e.nz == g.nz && e.esize == es)
+    auto &cache = ctx->fp_tex;
+    const bool cap = capturing(s);
+    for (auto &e : cache)
+        if (e.vol == vol && e.nx == g.nx && e.ny == g.ny && e.nz == g.nz && e.esize == es) {
+            e.captured |= cap;
             return e.tex.ok ? &e.tex : nullptr;
-    if ((int)ctx->fp_tex.size() >= stt_ctx::kFpTexCache || capturing(s)) return nullptr;
-    stt_ctx::FpTexEntry e{vol, g.nx, g.ny, g.nz, es, FpTex{}};
+        }
+    if (cap) return nullptr;
+    if ((int)cache.size() >= stt_ctx::kFpTexCache) {
+        // launches enqueued earlier (on any stream) may still gather from the older
+        // half (by creation), so the device drains before it goes: once in as many arrays
+        if (cudaDeviceSynchronize() != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        std::vector<stt_ctx::FpTexEntry> kept;
+        for (size_t k = 0; k < cache.size(); ++k) {
+            if (cache[k].captured || k >= cache.size() / 2) kept.push_back(cache[k]);
+            else destroy_fp_tex(cache[k].tex);
+        }
+        cache.swap(kept);
+        if ((int)cache.size() >= stt_ctx::kFpTexCache) return nullptr;
+    }
+    stt_ctx::FpTexEntry e{vol, g.nx, g.ny, g.nz, es, FpTex{}, false};
     make_fp_tex(g, vol, e.tex);  // where it fails, tex.ok = 0 is cached too: the loads run
-    ctx->fp_tex.push_back(e);
-    return ctx->fp_tex.back().tex.ok ? &ctx->fp_tex.back().tex : nullptr;
+    cache.push_back(e);
+    return cache.back().tex.ok ? &cache.back().tex : nullptr;
 }
 
 template <typename T>
