@@ -225,21 +225,49 @@ __device__ __forceinline__ void scatter_column(const GeomDev &g, const ViewRec &
     }
 }
 
+// The most rays a thread that the distance of the rows pays for.
+int most_rays(const GeomDev &g) {
+    if (!((long long)g.nx * g.nz < (1LL << 31))) return 1;  // (32-bit cell keys)
+    return g.row_pitch < CLOSE_ROWS ? 4 : g.row_pitch < 1.05f ? 2 : 1;
+}
+
 // Rays a thread: enough to merge where rows lie close, as long as the launch
 // still fills the GPU.  Backprojection of one view with 1 / 2 / 4, us, mean of six
 // views: rows 0.6 voxels apart 65,536 rays 130/129/193, 102,400 226/208/256,
 // 147,456 363/289/308, 200,704 575/439/417; 0.9 apart 65,536 205/203/287, 90,000
-// 319/304/381; 1.2 apart (128^2 at 128^3) 52/99.  The adjoint of dense residuals the same:
-// one view of 65,536 rays 0.9 apart 172/176/235, four 515/410/430; of residuals with
-// empty surroundings, whose zeros a ray a thread skips: one view 72/123/209, twelve
-// 283/300/334 (402/392 where the volume is not in the L2), four 0.6 apart
-// 625/538/478.
+// 319/304/381; 1.2 apart (128^2 at 128^3) 52/99.
 int merged_rays(const GeomDev &g, int nviews) {
     const long long rays = (long long)g.W * g.H * nviews;
-    if (!((long long)g.nx * g.nz < (1LL << 31))) return 1;  // (32-bit cell keys)
-    if (g.row_pitch < CLOSE_ROWS && rays >= 180000) return 4;
-    if (g.row_pitch < 1.05f && rays >= 90000) return 2;
-    return 1;
+    const int most = most_rays(g);
+    if (most == 4 && rays >= 180000) return 4;
+    return most > 1 && rays >= 90000 ? 2 : 1;
+}
+
+// The adjoint of a residual that is nowhere zero the same, for all views of the launch.
+// But its rays of zero residual are skipped, and what fills the GPU is the
+// others: some 20 % where an object's shadow is surrounded by nothing.  So a launch
+// needs several times as many.  Its time with 1 / 2 / 4, us, residuals dense / live in
+// one ellipse of 20 % / in spots of 9 x 9 on 16 %, volume cold in the L2 (hot the same
+// within 5 %):
+//   rows 0.6 apart  128^3 4 x 256^2   342/254/244  188/135/186   96/106/160
+//                   256^3 1 x 512^2   453/356/338  211/168/283  161/197/287
+//                         2 x 512^2   922/680/557  338/281/344  254/283/363
+//                         4 x 512^2  2446/1624/1350  782/639/610  465/432/557
+//                        12 x 512^2  6822/4498/3397 2082/1491/1298 1223/1071/1302
+//   rows 0.9 apart  192x176x160 2 x 256x240  174/139/190   63/109/180   74/107/174
+//                   4              408/350/389  234/190/207  115/141/203
+//                  12            1006/801/797   444/424/449  217/256/338
+//                  24           1864/1416/1234  732/619/696  377/410/508
+//                   256^3 1 x 341^2   229/195/293   92/154/272  106/174/274
+//                        12 x 341^2  3092/2315/1987 1026/905/909 580/588/771
+// (twelve views of an object's shadow, 192x176x160 and 256x240: 407/399).  The lines lie
+// where ellipse and shadow gain; of the spots, which no scan leaves, the worst case past
+// them loses 18 % (the twelve views), the other launches timed at most 9 %.
+int merged_rays_adjoint(const GeomDev &g, int nviews) {
+    const long long rays = (long long)g.W * g.H * nviews;
+    const int most = most_rays(g);
+    if (most == 1 || rays < 700000) return 1;
+    return most == 4 && rays >= 3000000 ? 4 : 2;
 }
 
 // BP-mode march (SingleScalarVolume.core.h:128-143, UpdateContributionSum
@@ -388,6 +416,10 @@ cudaError_t bp_ray_any(const GeomDev &g, const ViewRec *views, const ViewSel &se
 
 }  // namespace
 
+int adjoint_rays(const GeomDev &g, int nviews, bool dense) {
+    return dense ? merged_rays(g, nviews) : merged_rays_adjoint(g, nviews);
+}
+
 const char *ray_variant_name(int v) {
     static const char *names[kRayVariants] = {"global vector atomics, neighbouring rows merged",
                                               "shared-memory box per slab"};
@@ -423,8 +455,8 @@ cudaError_t launch_bp_ray_scatter(const GeomDev &g, const ViewRec *views, const 
 }
 
 cudaError_t launch_fp_adjoint(const GeomDev &g, const ViewRec *views, int view0, int nviews,
-                              const float *proj_bar, float *vol_bar, cudaStream_t s) {
-    const int rays = merged_rays(g, nviews);
+                              const float *proj_bar, float *vol_bar, cudaStream_t s, bool dense) {
+    const int rays = adjoint_rays(g, nviews, dense);
     const dim3 grid = column_grid(g, rays, nviews);
     if (rays == 4) k_fp_adjoint<4><<<grid, THREADS, 0, s>>>(g, views, view0, proj_bar, vol_bar);
     else if (rays == 2) k_fp_adjoint<2><<<grid, THREADS, 0, s>>>(g, views, view0, proj_bar, vol_bar);

@@ -715,7 +715,7 @@ stt_status stt_opnorm_power_iter(stt_ctx *ctx, int n_iter, unsigned long long se
         for (int v0 = 0; v0 < nv; v0 += chunk) {
             const int k = nv - v0 < chunk ? nv - v0 : chunk;
             if ((st = stt_fp(ctx, x, y, nullptr, nullptr, v0, k, stream))) return st;
-            if ((st = stt_fp_vjp(ctx, y, ax, v0, k, stream))) return st;
+            STT_CUDA(ctx, stt::launch_fp_adjoint(ctx->g, ctx->views_d, v0, k, y, ax, s, true), "k_fp_adjoint launch");
         }
         STT_CUDA(ctx, stt::launch_dot_f64(n, x, ax, sums + 1, s), "k_dot_f64");
         STT_CUDA(ctx, stt::launch_dot_f64(n, ax, ax, sums + 2, s), "k_dot_f64");
@@ -877,6 +877,13 @@ stt_status stt_warp_vjp(const int *dim, const float *vel, const float *src, int 
     STT_CUDA(nullptr, stt::launch_warp_vjp(dim, vel, src, nc, dt, out_bar, src_bar, vel_bar, S(stream)),
              "k_warp_vjp launch");
     return STT_OK;
+}
+
+// The rays a thread of the adjoint (tests).
+int stt_internal_adjoint_rays(int W, int H, int nx, int nz, float row_pitch, int nviews, int dense) {
+    stt::GeomDev g{};
+    g.W = W, g.H = H, g.nx = nx, g.nz = nz, g.row_pitch = row_pitch;
+    return stt::adjoint_rays(g, nviews, dense != 0);
 }
 
 // The rule of fp_from as numbers (tests): views[l*9 + b]; 0 loads, 1 the volume's own

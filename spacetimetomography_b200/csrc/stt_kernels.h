@@ -260,8 +260,11 @@ cudaError_t launch_bp_ray_scatter_slab(const GeomDev &g, const ViewRec *views, c
                                        float2 *acc, cudaStream_t s);
 cudaError_t launch_bp_ray_scatter(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
                                   float2 *acc, float *contrib, float *wsum, cudaStream_t s, int ray_variant = -1);
+// dense: the residual is nowhere zero.  adjoint_rays: the rays a thread it then
+// marches (k_scatter.cu has the measurements).
 cudaError_t launch_fp_adjoint(const GeomDev &g, const ViewRec *views, int view0, int nviews,
-                              const float *proj_bar, float *vol_bar, cudaStream_t s);
+                              const float *proj_bar, float *vol_bar, cudaStream_t s, bool dense = false);
+int adjoint_rays(const GeomDev &g, int nviews, bool dense);
 // The gather ceiling (k_project.cu): one view's rays sampled at the
 // projector's step with its gathers and interpolation and none of its march
 // control; `host_view` is the view's record (its layout picks vol_t).  With
