@@ -314,6 +314,7 @@ cudaError_t bp_voxel_any(const GeomDev &g, const ViewRec *views, const ViewSel &
     case 4: return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
     default: break;
     }
+    if (g.bp_len == 4) return bp_cols<4, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
     if (g.bp_len == 8) return bp_cols<8, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
     if (g.bp_len == 12) return bp_cols<12, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
     return bp_cols<16, 8>(g, views, sel, corr, vol, alpha, gmax, s, mirror);
@@ -350,16 +351,20 @@ cudaError_t pd_extrapolate_any(const int *d, const int *cut, const T *vol, const
 }
 }  // namespace
 
-int bp_default_len(double rows) {
+int bp_default_len(double rows, long long voxels) {
     // (K - 1) steps of `rows` between the first and the last voxel, their
     // windows' 4 rows, and one for where the run starts within a row
-    for (int k : {16, 12})
+    for (int k : {16, 12, 8})
         if ((k - 1) * rows + 5.0 <= BP_ROWS) return k;
-    return 8;
+    // Past that some columns of 8 walk, which takes a larger volume to hide.  Columns of
+    // 8 / 4, us, views at 0 / 30 / 90 degrees: 64^3 at 12 rows a voxel 10/12/13 -> 9/9/9,
+    // 96^3 at 6 10/19/13 -> 11/15/15, 128^3 at 8 18/25/25 -> 19/22/19, 160^3 at 5.4
+    // 38/49/41 -> 36/45/41, 256^3 at 6 122/149/129 -> 127/154/139.
+    return voxels < (1LL << 23) && 3 * rows + 5.0 <= BP_ROWS ? 4 : 8;
 }
 
 const char *bp_variant_name(int v) {
-    static const char *names[kBpVariants] = {"columns of 16, 12 or 8 voxels by the magnification, 8 blocks per SM",
+    static const char *names[kBpVariants] = {"columns of 16, 12, 8 or 4 voxels by the magnification, 8 blocks per SM",
                                              "columns of 8 voxels, 8 blocks per SM",
                                              "columns of 20 voxels, 8 blocks per SM",
                                              "columns of 16 voxels, 6 blocks per SM",

@@ -286,7 +286,8 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g) {
     d.sdd_ds = (float)(g->sdd / g->ds);
     d.row_pitch = (float)(g->ds * g->sid / g->sdd / g->sy);
     // detector rows per voxel where the volume comes nearest to the source (sid exceeds the reach, checked above)
-    d.bp_len = stt::bp_default_len(g->sdd / g->ds * g->sy / (g->sid - std::sqrt(hx * hx + hz * hz) - off));
+    d.bp_len = stt::bp_default_len(g->sdd / g->ds * g->sy / (g->sid - std::sqrt(hx * hx + hz * hz) - off),
+                                   (long long)g->nx * g->ny * g->nz);
     ctx->sp[0] = g->sx;
     ctx->sp[1] = g->sy;
     ctx->sp[2] = g->sz;
@@ -878,6 +879,9 @@ stt_status stt_warp_vjp(const int *dim, const float *vel, const float *src, int 
              "k_warp_vjp launch");
     return STT_OK;
 }
+
+// The column length of the voxel backprojection (tests).
+int stt_internal_bp_len(double rows, long long voxels) { return stt::bp_default_len(rows, voxels); }
 
 // The rays a thread of the adjoint (tests).
 int stt_internal_adjoint_rays(int W, int H, int nx, int nz, float row_pitch, int nviews, int dense) {

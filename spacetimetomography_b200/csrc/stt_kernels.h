@@ -302,8 +302,9 @@ cudaError_t launch_iter_persistent(const SweepJob *jobs_d, int njobs, int nblock
 // Voxel-driven backprojection, bp variant `bp_variant` (0: columns of g.bp_len
 // voxels); every voxel it writes goes to `mirror` too, if given.
 // bp_default_len: the longest column whose detector rows fit in the kernel's
-// table at `rows` detector rows per voxel (the geometry's largest).
-int bp_default_len(double rows);
+// table at `rows` detector rows per voxel (the geometry's largest); 8 where only
+// a shorter one would and the volume is large.
+int bp_default_len(double rows, long long voxels);
 cudaError_t launch_bp_voxel(const GeomDev &g, const ViewRec *views, const ViewSel &sel, const float *corr,
                             float *vol, float alpha, float gmax, cudaStream_t s, int bp_variant = 0,
                             float *mirror = nullptr);
