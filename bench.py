@@ -16,8 +16,9 @@ metric: projector GUPS over the 4D primal-dual iteration
         = frames * N^3 * views_per_frame / seconds_per_iteration / 1e9
         (each voxel-view update is one forward projection + one backprojection).
 
-`python bench.py [--gpus N --steps K --warmup W]`; for N > 1 launch with
-torch.distributed.run: each rank solves its own 10 frames (weak scaling) and
+`python bench.py [--gpus N --steps K --warmup W]` prints one JSON line on stdout and
+the longer legs (the single-frame workloads, the batch, the flow, the tuner's
+report) as another object on stderr; for N > 1 launch with torch.distributed.run: each rank solves its own 10 frames (weak scaling) and
 exchanges the neighbouring frames' boundary volumes with NCCL.
 `--impl reference` times the reference's CPU implementation of the same step
 (the reference's own projector and warp compiled from its sources, the SART and
@@ -1368,13 +1369,33 @@ def run_stt(args):
                 "flow": flow,
                 "configs": configs,
                 "batch": batch}
-        print(json.dumps(line), flush=True)
+        head, legs = split_line(line)
+        print(json.dumps(legs), file=sys.stderr, flush=True)
+        print(json.dumps(head), flush=True)
     solver.close()
     ctx.close()
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
     return 0
+
+
+# The legs of the default run that are longer than a figure: their own JSON object on
+# stderr, so that the line on stdout stays a few kilobytes whatever they hold.
+LEGS = ("persistent", "fp_samples", "tuning", "fp64_check", "fp64_pd_iteration", "flow", "configs", "batch")
+
+
+def split_line(line: dict) -> tuple[dict, dict]:
+    """The headline line and its legs."""
+    legs = {k: line[k] for k in LEGS if k in line}
+    head = {k: v for k, v in line.items() if k not in legs}
+    at = lambda leg, key: (legs.get(leg) or {}).get(key)  # noqa: E731
+    head["legs"] = {"on": "stderr", "persistent_s_per_iter": at("persistent", "s_per_iter"),
+                    "fp_gsamples_per_s": at("fp_samples", "fp_gsamples_per_s"),
+                    "flow_ms_per_iteration": at("flow", "ms_per_iteration"),
+                    "batch_ms_per_iter": at("batch", "ms_per_step"),
+                    "sart_rel_l2_vs_fp64": at("fp64_check", "sart_rel_l2_vs_fp64")}
+    return head, legs
 
 
 def run_iter_probe(args) -> int:
@@ -1555,7 +1576,7 @@ def batch_leg(args, steps, warmup) -> dict:
     t0 = time.perf_counter()
     choices = [d["ctx"].autotune(stream) for d in inst]  # every instance's own geometry
     for d in inst:
-        d["autotune"] = True  # the batch then also chooses its projector split as a whole (stt_batch_staging)
+        d["autotune"] = True  # the batch then also times its choices as a whole and keeps the fastest
     t_tune = time.perf_counter() - t0
     t_batch = batched_time()
     f32_result = [d["vol"].clone() for d in inst]
@@ -1599,11 +1620,12 @@ def batch_leg(args, steps, warmup) -> dict:
     t_pers = e0.elapsed_time(e1) / 1000.0 / steps
     bpers.close()
     pers_diff = max(float((d["vol"] - r).abs().max()) for d, r in zip(inst, f32_result))
-    # the instances' own tuned choices again (the batches may have set their
-    # staged masks to 0), for the one-after-another forms below
+    # the instances' own tuned choices again (the batches may have kept others), for
+    # the one-after-another forms below
     for d, c in zip(inst, choices):
         d["ctx"].set_tuning(c["fp_variant"], c["slab_variant"], c["bp_variant"], staged_bins=c["staged_bins"],
-                            ray_variant=c["ray_variant"], staged_bins_bf16=c["staged_bins_bf16"])
+                            ray_variant=c["ray_variant"], staged_bins_bf16=c["staged_bins_bf16"],
+                            fp_variant_bf16=c["fp_variant_bf16"])
     # the same instances one after another (each its own graph-captured solver)
     solvers = []
     for d in inst:
