@@ -300,8 +300,10 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g) {
 
 }  // extern "C"
 
-// The context's z-fastest copy of `vol`, refreshed (FP32 and BF16 storage).
+// The context's z-fastest copy of `vol`, refreshed (FP32 and BF16 storage); none
+// where a capture would have to allocate it (every view then reads the volume).
 static stt_status make_copy(stt_ctx *ctx, const float *vol, cudaStream_t s, const float **volt) {
+    if (ctx->volt_n < (size_t)nvox(ctx) && stt::capturing(s)) return STT_OK;
     stt_status st = ensure(ctx, ctx->volt, ctx->volt_n, (size_t)nvox(ctx), "transposed volume");
     if (st) return st;
     STT_CUDA(ctx, stt::launch_transpose(ctx->g, vol, ctx->volt, s), "k_transpose launch");
@@ -310,6 +312,7 @@ static stt_status make_copy(stt_ctx *ctx, const float *vol, cudaStream_t s, cons
 }
 
 static stt_status make_copy(stt_ctx *ctx, const unsigned short *vol, cudaStream_t s, const unsigned short **volt) {
+    if (ctx->volt16_n < (size_t)nvox(ctx) && stt::capturing(s)) return STT_OK;
     stt_status st = ensure(ctx, ctx->volt16, ctx->volt16_n, (size_t)nvox(ctx), "transposed BF16 volume");
     if (st) return st;
     STT_CUDA(ctx, stt::launch_transpose_bf16(ctx->g, vol, ctx->volt16, s), "k_transpose launch");

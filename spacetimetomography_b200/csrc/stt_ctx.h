@@ -86,6 +86,9 @@ inline int off_axis_bin(float deg) {
 }
 // Applies ctx->staged_bins and staged_bins16 to every view (host and device tables).
 stt_status apply_staged_bins(stt_ctx *ctx);
+// Whether `s` is being captured: then nothing is allocated or created for it, and
+// the call takes the form that needs neither.
+bool capturing(cudaStream_t s);
 // The texture of `vol` (created on first use, cached in the context), whatever
 // the tuned variant; nullptr where it does not bind, it would have to be created
 // while `s` is being captured, or captures hold the whole cache.  Valid until the

@@ -119,9 +119,6 @@ stt_status apply_staged_bins(stt_ctx *ctx) {
     return STT_OK;
 }
 
-namespace {
-// While a stream is captured nothing is allocated or created for it: the call
-// takes the form that needs neither.
 bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
@@ -130,6 +127,8 @@ bool capturing(cudaStream_t s) {
     }
     return st != cudaStreamCaptureStatusNone;
 }
+
+namespace {
 
 template <typename T>
 const FpTex *cached_tex(stt_ctx *ctx, const T *vol, cudaStream_t s) {
