@@ -13,7 +13,7 @@
 //
 // Layout: the caller's fields are planar and x-fastest, idx = x + y*nx +
 // z*nx*ny, channel planes of n = nx*ny*nz floats (CImg's layout; dual field y: 10
-// planes Y1|Y2|Y3|Y4).  The iterations work on vectors per voxel (FlowVec below),
+// planes Y1|Y2|Y3|Y4).  The iterations work on vectors per voxel (Dual below),
 // packed when a level starts.  Between residual checks one kernel runs the dual
 // step of an iteration and the primal step of the next (k_flow_step).
 #include <algorithm>
@@ -780,7 +780,7 @@ cudaError_t launch_flow_step(const int *d, const FlowRoi &roi, const float *y_in
                              const float *k4prev, float *kty, float sigma1, float hf, float lambda, int huber,
                              int flags, const int *done, cudaStream_t s) {
     const int gx = (d[0] + 30) / 31, gy = (d[1] + STEP_Y - 1) / STEP_Y;
-    // Runs along z: the count whose rounds of resident blocks (two per SM) walk
+    // Runs along z: the count whose rounds of resident blocks (four per SM) walk
     // the fewest planes, each run with about one and a half on top (the duals
     // formed again below it, and its first loads).
     const int resident = 4 * sm_count();

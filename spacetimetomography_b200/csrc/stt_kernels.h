@@ -360,7 +360,7 @@ struct ResizeAxis {
 
 cudaError_t launch_warp_box(const int *dim, const float *box, const float *vel, const float *src, int nc,
                             float dt, float *out, cudaStream_t s);
-// The iterations' fields (float4 per voxel: v, u, steps; y packed): see FlowVec in
+// The iterations' fields (float4 per voxel: v, u, steps; y packed): see Dual in
 // k_flow.cu.  Y and V are the caller's planes.
 cudaError_t launch_flow_pack(long long n, const float *Y, const float *V, float *y, float4 *v0, float4 *v1, float4 *v2,
                              cudaStream_t s);
