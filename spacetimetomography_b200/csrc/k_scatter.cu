@@ -17,6 +17,8 @@
 // meeting costs less than the sectors); z-fastest accumulators for the views along
 // x (the scatter 576 -> 370 us at 90 degrees, but emptying 200 MB of them across the
 // volume's order takes 820 us, in order 70).
+#include <algorithm>
+
 #include "stt_internal.cuh"
 #include "stt_kernels.h"
 
@@ -260,13 +262,15 @@ int merged_rays(const GeomDev &g, int nviews) {
 //                  24           1864/1416/1234  732/619/696  377/410/508
 //                   256^3 1 x 341^2   229/195/293   92/154/272  106/174/274
 //                        12 x 341^2  3092/2315/1987 1026/905/909 580/588/771
-// (twelve views of an object's shadow, 192x176x160 and 256x240: 407/399).  The lines lie
-// where ellipse and shadow gain; of the spots, which no scan leaves, the worst case past
-// them loses 18 % (the twelve views), the other launches timed at most 9 %.
+// and of objects' shadows (16 to 20 % live): 80^3 11 x 132x106 101/95, 100^3 1 x 121x153
+// 47/77, 160^3 2 x 256^2 64/105, 4 x 256^2 187/163, 176^3 6 x 184x187 136/185,
+// 192x176x160 12 x 256x240 407/399.  A longer ray takes more other rays to hide, so two
+// rays a thread take 1500 of them per voxel of the largest extent and 150,000 at least;
+// past that line the spots, which no scan leaves, lose 18 % at most, the others gain.
 int merged_rays_adjoint(const GeomDev &g, int nviews) {
     const long long rays = (long long)g.W * g.H * nviews;
-    const int most = most_rays(g);
-    if (most == 1 || rays < 700000) return 1;
+    const int most = most_rays(g), extent = std::max(g.nx, std::max(g.ny, g.nz));
+    if (most == 1 || rays < std::max(150000LL, 1500LL * extent)) return 1;
     return most == 4 && rays >= 3000000 ? 4 : 2;
 }
 

@@ -887,9 +887,9 @@ stt_status stt_warp_vjp(const int *dim, const float *vel, const float *src, int 
 int stt_internal_bp_len(double rows, long long voxels) { return stt::bp_default_len(rows, voxels); }
 
 // The rays a thread of the adjoint (tests).
-int stt_internal_adjoint_rays(int W, int H, int nx, int nz, float row_pitch, int nviews, int dense) {
+int stt_internal_adjoint_rays(int W, int H, int n, float row_pitch, int nviews, int dense) {
     stt::GeomDev g{};
-    g.W = W, g.H = H, g.nx = nx, g.nz = nz, g.row_pitch = row_pitch;
+    g.W = W, g.H = H, g.nx = g.ny = g.nz = n, g.row_pitch = row_pitch;
     return stt::adjoint_rays(g, nviews, dense != 0);
 }
 
