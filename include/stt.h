@@ -124,10 +124,11 @@ stt_status stt_set_geometry(stt_ctx *ctx, const stt_geometry *g);
  *   fp_variant   the gather projector's detector tile and samples in flight;
  *                variants 10 and 11 fetch a sample's 8 corners as two tld4
  *                gathers of the FP32 volume bound as a pitch-linear 2D texture
- *                (the context keeps one texture object per array it is given,
- *                until stt_destroy; where the device's texture limits do not
- *                admit the array, the load-based variant of the same shape runs;
- *                views of few rays share each ray between a block's warps);
+ *                (the context keeps the texture objects of the arrays it was
+ *                given last, and those that a stream capture used until
+ *                stt_destroy; where the device's texture limits do not admit the
+ *                array, the load-based variant of the same shape runs; views of
+ *                few rays share each ray between a block's warps);
  *   slab_variant the box the slab-staged projector stages with TMA;
  *   bp_variant   the column length of the voxel backprojection (0: by the
  *                geometry's magnification) and the blocks per SM;
@@ -186,7 +187,9 @@ stt_status stt_fp_texture_ok_typed(stt_ctx *ctx, const void *vol, int dtype, int
 const char *stt_tuning_variant_name(int kernel, int variant);
 
 /* ---- forward projector (TypicalRayProducer.core.h:123-268) ---------------
- * Projects views [view0, view0+nviews) of `vol`.
+ * Projects views [view0, view0+nviews) of `vol`, by loads or through a texture
+ * of the volume or of its mirror, whichever is the faster for the call's views and
+ * sizes: the same bits.
  *   proj   : nviews*W*H line integrals (sum of f*sd, entry sample counted twice)
  *   raylen : optional W*H*nviews ray lengths (tfar - tnear, mm); written only
  *            where the ray hits the volume, as the reference does
