@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 7) k_iter_persistent(const Swee
         const int i = (int)(t % gx) * SWEEP_THREADS + threadIdx.x, j = (int)((t / gx) % d.y);
         const int k = (int)(t / ((long long)gx * d.y));
         if (i < d.x) {
-            warpdev::Cell s;
+            warpdev::Cell<I> s;
             warpdev::trace_cell(d, J.flow, -1.0f, i, j, k, s);
             float bw[1];
             warpdev::sample_cell<1, false, T>(xbar1, 0, s, bw);
@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 7) k_iter_persistent(const Swee
         if (i < d.x) {
             float fw = 0.0f;
             if (!J.first) {
-                warpdev::Cell s;
+                warpdev::Cell<I> s;
                 warpdev::trace_cell(d, J.flow_prev, 1.0f, i, j, k, s);
                 float v[1];
                 warpdev::sample_cell<1, false, float, true>(J.ybc_prev, 0, s, v);
@@ -318,6 +318,8 @@ const void *pick(bool bf16, bool wide, bool whole = false) {
 }
 
 }  // namespace
+
+bool sweep_wide(const GeomDev &g) { return warpdev::needs_general(warpdev::Dim3i{g.nx, g.ny, g.nz}); }
 
 int sweep_max_blocks(bool bf16, bool wide) {
     // (the smaller of the two kernels' resident blocks: one plan serves both)

@@ -29,21 +29,21 @@ using namespace warpdev;
 constexpr int WARP_BX = 32, WARP_BY = 4;
 
 // T: the source's storage (float, or BF16 bits widened exactly to FP32).
-template <typename T>
+template <typename T, typename I>
 __global__ void __launch_bounds__(WARP_BX *WARP_BY) k_warp(const Dim3i d, const float *__restrict__ vel,
                                                            const T *__restrict__ src, int nc, float dt,
                                                            float *__restrict__ out) {
     const int i = blockIdx.x * WARP_BX + threadIdx.x;
     const int j = blockIdx.y * WARP_BY + threadIdx.y, k = blockIdx.z;
     if (i >= d.x || j >= d.y) return;
-    const int n = d.x * d.y * d.z;
-    Cell s;
+    const size_t n = (size_t)d.x * d.y * d.z;
+    Cell<I> s;
     trace_cell(d, vel, dt, i, j, k, s);
-    const int o = i + j * d.x + k * d.x * d.y;
+    const I o = i + (I)j * d.x + (I)k * d.x * d.y;
     for (int ch = 0; ch < nc; ++ch) {
         float v[1];
-        sample_cell<1>(src + (size_t)ch * n, 0, s, v);
-        out[o + (size_t)ch * n] = v[0];
+        sample_cell<1>(src + ch * n, 0, s, v);
+        out[o + ch * n] = v[0];
     }
 }
 
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(WARP_BX *WARP_BY) k_warp_staged(const Dim3i d,
     const int i = blockIdx.x * WARP_BX + threadIdx.x;
     const int j = blockIdx.y * WARP_BY + threadIdx.y, k = blockIdx.z;
     const bool live = i < d.x && j < d.y;
-    const int n = d.x * d.y * d.z;
+    const size_t n = (size_t)d.x * d.y * d.z;
     const float h = -dt;
     const float p[3] = {(float)i + 0.5f, (float)j + 0.5f, (float)k + 0.5f};
     float p2[3] = {0.0f, 0.0f, 0.0f}, g2[3] = {1.0f, 1.0f, 1.0f};
@@ -132,12 +132,12 @@ __global__ void __launch_bounds__(WARP_BX *WARP_BY) k_warp_staged(const Dim3i d,
         }
     }
     if (!live) return;
-    Cell s2;
+    Cell<int> s2;
     cell_setup(d, g2, s2);
     float v2[3];
     const unsigned lx = (unsigned)(b0[0] - ox), ly = (unsigned)(b0[1] - oy), lz = (unsigned)(b0[2] - oz);
     if (staged && lx <= VX - 4 && ly <= VY - 4 && lz <= VZ - 4) {
-        Cell sl = s2;  // the same weights and edge flags, box-local offsets
+        Cell<int> sl = s2;  // the same weights and edge flags, box-local offsets
         sl.sy = VX;
         sl.sz = VX * VY;
         sl.x.lo = (int)lx;
@@ -154,13 +154,13 @@ __global__ void __launch_bounds__(WARP_BX *WARP_BY) k_warp_staged(const Dim3i d,
         q[a] = __fadd_rn(p2[a], __fmul_rn(0.5f, __fsub_rn(p[a], p0)));
     }
     const float gq[3] = {to_grid(q[0], d.x, nullptr), to_grid(q[1], d.y, nullptr), to_grid(q[2], d.z, nullptr)};
-    Cell s;
+    Cell<int> s;
     cell_setup(d, gq, s);
     const int o = i + j * d.x + k * d.x * d.y;
     for (int ch = 0; ch < nc; ++ch) {
         float v[1];
-        sample_cell<1>(src + (size_t)ch * n, 0, s, v);
-        out[o + (size_t)ch * n] = v[0];
+        sample_cell<1>(src + ch * n, 0, s, v);
+        out[o + ch * n] = v[0];
     }
 }
 
@@ -410,10 +410,12 @@ cudaError_t warp_any(const int *dim, const float *vel, const T *src, int nc, flo
     const dim3 grid((d.x + WARP_BX - 1) / WARP_BX, (d.y + WARP_BY - 1) / WARP_BY, d.z), block(WARP_BX, WARP_BY);
     CUtensorMap vmap;
     const unsigned box[4] = {VX, VY, VZ, 3};
-    if (encode_planes_map(&vmap, vel, d.x, d.y, d.z, 3, box))
+    if (needs_general(d))
+        k_warp<T, long long><<<grid, block, 0, s>>>(d, vel, src, nc, dt, out);
+    else if (encode_planes_map(&vmap, vel, d.x, d.y, d.z, 3, box))
         k_warp_staged<T><<<grid, block, 0, s>>>(d, vmap, vel, src, nc, dt, out, status);
     else
-        k_warp<T><<<grid, block, 0, s>>>(d, vel, src, nc, dt, out);
+        k_warp<T, int><<<grid, block, 0, s>>>(d, vel, src, nc, dt, out);
     return cudaGetLastError();
 }
 }  // namespace

@@ -137,8 +137,7 @@ stt_status build_sweep(stt_batch *b) {
     for (int i = 0; i < n; ++i) {
         if (stt_internal_solver_jobs(b->inst[i].solver, &jobs[i]) != 1)
             return bfail(b, STT_ERR_INVALID, "instance " + std::to_string(i) + ": sweep job");
-        const stt::GeomDev &g = jobs[i].g;
-        b->wide |= (long long)g.nx * g.ny * g.nz >= (1LL << 31);
+        b->wide |= stt::sweep_wide(jobs[i].g);
     }
     b->sweep_blocks = stt::sweep_max_blocks(b->bf16, b->wide);
     if (b->sweep_blocks < 1) return bfail(b, STT_ERR_CUDA, "occupancy of the persistent sweep");

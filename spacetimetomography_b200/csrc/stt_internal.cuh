@@ -597,13 +597,14 @@ struct MarchGen {
 };
 
 // Catmull-Rom weights for taps (-1, 0, +1, +2) at fraction d (the cubic of
-// ST_Tomography.cpp:183-186 and CImg's _cubic_atX, written in weight form).
+// ST_Tomography.cpp:183-186 and CImg's _cubic_atX, written in weight form), contracted
+// as written, so that every kernel gets the same bits.
 __device__ __forceinline__ void cr_weights(float d, float w[4]) {
-    float d2 = d * d, d3 = d2 * d;
-    w[0] = 0.5f * (-d + 2.0f * d2 - d3);
-    w[1] = 1.0f + 0.5f * (-5.0f * d2 + 3.0f * d3);
-    w[2] = 0.5f * (d + 4.0f * d2 - 3.0f * d3);
-    w[3] = 0.5f * (-d2 + d3);
+    const float d2 = __fmul_rn(d, d), d3 = __fmul_rn(d2, d), t3 = __fmul_rn(3.0f, d3);
+    w[0] = __fmul_rn(0.5f, __fsub_rn(__fmaf_rn(2.0f, d2, -d), d3));
+    w[1] = __fmaf_rn(0.5f, __fmaf_rn(-5.0f, d2, t3), 1.0f);
+    w[2] = __fmul_rn(0.5f, __fsub_rn(__fmaf_rn(4.0f, d2, d), t3));
+    w[3] = __fmul_rn(0.5f, __fsub_rn(d3, d2));
 }
 
 // The ray sum of one forward-projector ray (hit rays only): the Kahan sum of

@@ -280,8 +280,10 @@ cudaError_t launch_fill_seeded(long long n, unsigned long long seed, float *x, c
 // The persistent sweep (k_persist.cu): the SART calls of all jobs (frames or
 // batch instances, SweepJob in stt_internal.cuh) in one cooperative launch of
 // `nblocks` blocks, jobs_d a device array sorted by block0.  bf16: the jobs'
-// storage; wide: some job's volume has 2^31 voxels or more.
+// storage; wide: some job's volume takes 64-bit offsets (sweep_wide: 2^31 voxels or
+// more, or an extent of two, whose warps only that form samples).
 struct SweepJob;
+bool sweep_wide(const GeomDev &g);
 // Blocks of the launch that can be resident at once on the current device (0
 // on error): the most a launch may have.
 int sweep_max_blocks(bool bf16, bool wide);

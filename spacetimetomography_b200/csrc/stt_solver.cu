@@ -644,7 +644,7 @@ stt_status stt_solver_create(stt_ctx *ctx, const stt_solve_cfg *cfg, const stt_p
         }
     }
     if (cfg->mode == STT_SOLVE_PERSISTENT) {
-        s->sweep_wide = (long long)g->nx * g->ny * g->nz >= (1LL << 31);  // 64-bit gather offsets
+        s->sweep_wide = stt::sweep_wide(*g);
         s->sweep_blocks = stt::sweep_max_blocks(cfg->storage == STT_DTYPE_BF16, s->sweep_wide);
         std::vector<stt::SweepJob> jobs(F);
         fill_jobs(s, jobs.data());
